@@ -284,6 +284,7 @@ struct anacor_plan {
     int field8_state = 0;
     uint8_t *d_field8b = nullptr;  // the same in 4^3 bricks, built on first use by variants 13..16
     int field8b_state = 0;
+    int *d_walls = nullptr;        // [6] room between the non-vacuum labels and the walls, built with a field
 };
 
 namespace {
@@ -306,6 +307,7 @@ void plan_release(anacor_plan *p)
     dev_free(p->d_field, st);
     dev_free(p->d_field8, st);
     dev_free(p->d_field8b, st);
+    dev_free(p->d_walls, st);
     dev_free(p->d_order, st);
     if (p->h_refl && !p->h_refl_borrowed)
         cudaFreeHost(p->h_refl);
@@ -676,7 +678,8 @@ int plan_ensure_field(anacor_plan *p, int kind = 1)
     int bad = 0;
     cudaError_t e;
     if ((e = dev_alloc(&field, nvol * copies, st)) || (e = dev_alloc(&tmp, nvol * tmp_copies, st)) ||
-        (e = dev_alloc(&d_bad, 1, st)) ||
+        (e = dev_alloc(&d_bad, 1, st)) || (!p->d_walls && (e = dev_alloc(&p->d_walls, 6, st))) ||
+        (e = launch_wall_room(p->d_vol, p->dims, p->d_walls, st)) ||
         (e = kind == 2 ? launch_octant_fields(p->d_vol, p->dims, field, tmp, d_bad, st)
                        : launch_distance_field(p->d_vol, p->dims, field, tmp, d_bad, st)) ||
         (e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
@@ -748,6 +751,7 @@ SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1)
     d.qtab = p->d_qtab;
     d.work_begin = work_begin;
     d.order = p->n_refl > 0 ? p->d_order : nullptr;
+    d.walls = p->d_walls;
     if (fk < 0)
         fk = field_kind(p->variant);
     if (fk == 0) {
@@ -1074,11 +1078,12 @@ int plan_default_config(anacor_plan *p)
             variant = 12;
         succeed();   // labels outside 0..7: the cooperative march, no error
     }
-    // the largest tile that still gives every warp slot four items
-    const long long warps = (long long)p->dev->sms * 32;
+    // the largest tile that still gives every warp slot four items (the
+    // cooperative march, 32 warps a SM) or sixteen (the field march, 40)
+    const long long warps = (long long)p->dev->sms * (variant ? 160 : 32);
     int tile = kMinTile;
     for (int t : {2048, 1024, 512, 256})
-        if (p->n_refl * (((long long)p->n_vox + t - 1) / t) >= 4 * warps) {
+        if ((!variant || t <= 1024) && p->n_refl * (((long long)p->n_vox + t - 1) / t) >= 4 * warps) {
             tile = t;
             break;
         }

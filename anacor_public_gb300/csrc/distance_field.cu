@@ -395,6 +395,81 @@ cudaError_t launch_distance_field(const int8_t *d_vol, const int *dims, uint8_t 
     return cudaGetLastError();
 }
 
+namespace {
+
+// Room between the non-vacuum labels and the six walls: one read of the
+// volume (16 bytes a load; HBM-bound), per-thread minima, one atomic per wall
+// and block.
+__global__ void __launch_bounds__(256) wall_room_kernel(const int8_t *__restrict__ vol, int dz, int dy, int dx,
+                                                        int nvol, int *__restrict__ room)
+{
+    int m[6];
+#pragma unroll
+    for (int a = 0; a < 6; a++)
+        m[a] = INT_MAX;
+    auto see = [&](int z, int y, int x) {
+        m[0] = min(m[0], z);
+        m[1] = min(m[1], y);
+        m[2] = min(m[2], x);
+        m[3] = min(m[3], dz - 1 - z);
+        m[4] = min(m[4], dy - 1 - y);
+        m[5] = min(m[5], dx - 1 - x);
+    };
+    const int chunks = (int)(((long long)nvol + 15) / 16);
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < chunks; q += gridDim.x * blockDim.x) {
+        const int v0 = 16 * q, n = min(16, nvol - v0);
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+        if (n == 16 && ((uintptr_t)vol & 15u) == 0) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4 *>(vol) + q);
+            w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+        } else {
+            for (int k = 0; k < n; k++)
+                w[k >> 2] |= (uint32_t)(uint8_t)__ldg(vol + v0 + k) << (8 * (k & 3));
+        }
+        if (!(w[0] | w[1] | w[2] | w[3]))
+            continue;
+        int row = v0 / dx, x = v0 - row * dx;
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            if ((w[k >> 2] >> (8 * (k & 3))) & 0xffu) {
+                const int z = row / dy;
+                see(z, row - z * dy, x);
+            }
+            if (++x == dx) {
+                x = 0;
+                row++;
+            }
+        }
+    }
+    __shared__ int least[6];
+    if (threadIdx.x < 6)
+        least[threadIdx.x] = INT_MAX;
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 6; a++) {
+        const int r = __reduce_min_sync(0xffffffffu, m[a]);
+        if ((threadIdx.x & 31) == 0)
+            atomicMin(&least[a], r);
+    }
+    __syncthreads();
+    if (threadIdx.x < 6)
+        atomicMin(room + threadIdx.x, least[threadIdx.x]);
+}
+
+}  // namespace
+
+cudaError_t launch_wall_room(const int8_t *d_vol, const int *dims, int *d_room, cudaStream_t st)
+{
+    const long long nvol = (long long)dims[0] * dims[1] * dims[2];
+    cudaError_t e = cudaMemsetAsync(d_room, 0x7f, 6 * sizeof(int), st);
+    if (e != cudaSuccess || nvol == 0)
+        return e;
+    const long long blocks = (nvol / 16 + 255) / 256 + 1;
+    wall_room_kernel<<<(unsigned)std::min<long long>(blocks, 152 * 8), 256, 0, st>>>(d_vol, dims[0], dims[1], dims[2],
+                                                                                   (int)nvol, d_room);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_octant_fields(const int8_t *d_vol, const int *dims, uint8_t *d_out, uint8_t *d_tmp, int *d_bad,
                                  cudaStream_t st)
 {

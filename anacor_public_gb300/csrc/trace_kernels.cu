@@ -1039,6 +1039,404 @@ __device__ __forceinline__ void trace_leg(const LegHead &h, const FaceRule *rule
     leg_finish<kDetail, kF32>(rules, cz, cy, cx, v, full, voxel, sq, sq_stride, qtab, seg, S, out, voxelf);
 }
 
+// ---- field march ----------------------------------------------------------
+//
+// The A_h kernel's march on the packed fields: one lane walks one leg as a
+// chain of dependent byte loads (about 12, 16 for the slowest lane of a warp),
+// each an L2 access of some 450 cycles, so a warp alone needs 12,500 cycles a
+// leg and what counts is how many warps an SM holds and how many instructions
+// and L1 misses a step costs.  Hence:
+//  * what a step needs is prepared once per work item (32 voxels x tile / 32 x
+//    2 legs share it) in shared memory, one rule per leg and exit axis; a
+//    leg's own set-up is the exit face and a few shared loads;
+//  * a leg whose non-vacuum labels keep room from the walls ahead of it needs
+//    no step count and no wall limit: it meets vacuum first;
+//  * the inner loop holds no call (what lives across one is kept in local
+//    memory: 92 local loads a warp and leg before, 9 now), and the kernel fits
+//    48 registers, five CTAs an SM (six, at 40 registers: 3 % slower);
+//  * everything rare (close exit-face calls, ratios beyond fixed point,
+//    full_iteration, legs that reach the wall limit, more than kMaxSegments
+//    class changes) is out of line in leg_slow, which reads the full rule
+//    from global memory.
+// 512x512x400, 13,266 voxels, 20,000 reflections: 30.0 -> 20.6 ms (1,430 ->
+// 915 warp instructions per 32 legs; L1 misses at 70 %, L2 at 59 % of their
+// peak rates, issue slots at 56 %).
+
+// One leg's rule for one exit axis.  q: the 32.32 ratios of the two other
+// axes a and b (lo, hi words).  off: their initial low words -- the rounding
+// offset plus kFieldMargin, so that a fraction near a rounding boundary reads
+// below twice the margin (adding it changes the integer
+// part only there, where the exact expression is used).  A whole-numbered
+// ratio gets 2^31: its fraction stays one half, which is never ambiguous and
+// rounds to the exact integer in both modes.
+struct alignas(16) HotRule {
+    uint32_t qa_lo, qa_hi, qb_lo, qb_hi;
+    uint32_t off_a, off_b;
+    int dS, Sa;              // linear fields: signed stride of the step axis, stride of a
+    int Sb;
+    int rq;                  // skip multiplier (FaceRule::skip_rq)
+    uint32_t flags;
+    int face;
+    const uint8_t *fld;      // the field of the leg's octant
+    int ds;                  // +1 / -1 on the step axis
+    int pad;
+};
+static_assert(sizeof(HotRule) == 64, "HotRule layout");
+constexpr uint32_t kHotSimple = 1u;   // fixed point, no error status, no full_iteration
+constexpr uint32_t kHotFree = 2u;     // a leg stops at vacuum before any increment can clamp at a wall
+
+struct alignas(16) WarpTab {
+    HotRule rule[2][3];      // [leg][exit axis]
+    float inv[2][3];         // 1 / |e_a|; +inf for a zero component
+    float sgn[2][3];         // exit distance on axis a is n_a inv_a with n_a = org_a + sgn_a c_a (exact)
+    float org[2][3];
+    uint32_t exact_face[2];  // the FP64 quotients decide for every lane
+    float voxel[3];
+    float mu[4];
+    int dy, dx, is_exp, count_steps;
+    const ReflTable *refl;
+    const SampleDesc *desc;
+};
+
+// Half-width of the ambiguous zone around a rounding boundary, in 2^-32
+// units, for increments of a field march: i * Q differs from i * q * 2^32 by
+// at most i / 2 <= 4096 units (Q is rounded, kMaxDim bounds i), and the
+// reference's two FP64 roundings of values inside the volume (below 2^14) by
+// less than one.
+constexpr uint32_t kFieldMargin = 4096u + 16u;
+
+// Fills a warp's table for reflection table T: lanes 0..5 a rule each (leg,
+// axis), lanes 8..13 the exit-face operands, lanes 16..23 the sample's constants.
+__device__ __forceinline__ void fill_warp_tab(WarpTab &w, const ReflTable *__restrict__ T, const SampleDesc &D,
+                                              int lane)
+{
+    const int part = lane >> 3, k = lane & 7;
+    if (part < 2 && k < 6) {
+        const int leg = k / 3, a = k - 3 * leg;
+        const uint32_t sb = __ldg(&T->head[leg].sign_bits);
+        const bool pos = (sb >> a) & 1u, zero = !((sb >> a) & 9u);
+        if (part == 1) {
+            const int dim = a == 0 ? D.dim[0] : (a == 1 ? D.dim[1] : D.dim[2]);
+            w.inv[leg][a] = __ldg(&T->head[leg].inv[a]);
+            w.sgn[leg][a] = zero ? 0.0f : (pos ? -1.0f : 1.0f);
+            w.org[leg][a] = zero ? 1.0f : (pos ? (float)dim : 0.0f);
+            if (a == 0)
+                w.exact_face[leg] = sb & 64u;
+            return;
+        }
+        const int face = a == 2 ? (pos ? 1 : 6) : (a == 1 ? (pos ? 5 : 4) : (pos ? 3 : 2));
+        const FaceRule &R = T->rule[leg][face - 1];
+        HotRule h;
+        const int ia = a == 0 ? 1 : 0, ib = a == 2 ? 1 : 2;
+        const long long Qa = R.Q[ia], Qb = R.Q[ib];
+        h.qa_lo = (uint32_t)Qa;
+        h.qa_hi = (uint32_t)(Qa >> 32);
+        h.qb_lo = (uint32_t)Qb;
+        h.qb_hi = (uint32_t)(Qb >> 32);
+        const uint32_t off = (R.use_round ? 0x80000000u : 0u) + kFieldMargin;
+        h.off_a = (R.exact_mask >> ia) & 1 ? 0x80000000u : off;
+        h.off_b = (R.exact_mask >> ib) & 1 ? 0x80000000u : off;
+        h.ds = R.Q[a] > 0 ? 1 : -1;
+        const int sz = D.dim[1] * D.dim[2], sy = D.dim[2];
+        h.dS = h.ds * pick3(a, sz, sy, 1);
+        h.Sa = pick3(ia, sz, sy, 1);
+        h.Sb = pick3(ib, sz, sy, 1);
+        h.rq = (int)R.skip_rq;   // at most 2^22, times 31
+        h.pad = 0;
+        h.fld = D.field + R.octant * D.field_stride;
+        h.face = face;
+        uint32_t f = 0u;
+        if (R.fast && !R.status && !D.full_iteration && !zero) {
+            f |= kHotSimple;
+            // The examined increment after a non-vacuum one lies at most
+            // ceil(|q|) voxels further on each axis: when the non-vacuum
+            // labels keep that distance (and one more) from the walls the leg
+            // moves toward, it meets vacuum before a clamped increment, and
+            // before the last one of its face.
+            if (D.walls) {
+                const long long qm = max(Qa < 0 ? -Qa : Qa, Qb < 0 ? -Qb : Qb);
+                const int need = (int)(qm >> 32) + 2;
+                bool free_leg = true;
+#pragma unroll
+                for (int x = 0; x < 3; x++) {
+                    const bool back = (R.octant >> (2 - x)) & 1;   // toward coordinate 0
+                    free_leg = free_leg && __ldg(D.walls + (back ? x : 3 + x)) >= need;
+                }
+                if (free_leg)
+                    f |= kHotFree;
+            }
+        }
+        h.flags = f;
+        w.rule[leg][a] = h;
+    } else if (part == 2) {
+        if (k < 3)
+            w.voxel[k] = D.voxelf[k];
+        else if (k < 7)
+            w.mu[k - 3] = D.muf[k - 3];
+        else {
+            w.dy = D.dim[1];
+            w.dx = D.dim[2];
+            w.is_exp = D.is_exp;
+            w.count_steps = D.steps != nullptr;
+            w.refl = T;
+            w.desc = &D;
+        }
+    }
+}
+
+// integer part (the return value) and fraction of off + i * Q
+__device__ __forceinline__ int fixed_at(int i, uint32_t q_lo, uint32_t q_hi, unsigned long long off, uint32_t &frac)
+{
+    const unsigned long long p = (unsigned long long)(uint32_t)i * q_lo + off;
+    frac = (uint32_t)p;
+    return (int)((uint32_t)(p >> 32) + (uint32_t)i * q_hi);
+}
+
+// The increment examined after i, whose field byte holds the distance d (>= 1)
+// above its label: the ones the field proves to keep i's label, min(d - 1, floor((d - 2) / qmax))
+// and never a negative number of them, are passed over.
+__device__ __forceinline__ int next_increment(int i, uint32_t byte, int rq)
+{
+    const int d = (int)(byte >> 3);
+    return i + max(min((((d - 2) * rq) >> 16) + 1, d), 1);
+}
+
+// Byte of increment i of a field whose displacement on the two non-step axes
+// is (da, db): linear fields from the leg's start byte, bricked ones from the
+// absolute coordinates.
+template <bool kBrick>
+__device__ __forceinline__ uint32_t field_byte(const uint8_t *start, const HotRule &R, const SampleDesc *D, int axis,
+                                               int cz, int cy, int cx, int i, int da, int db, int dS, int Sa, int Sb)
+{
+    if (!kBrick)
+        return __ldg(start + (i * dS + da * Sa + db * Sb));
+    const Vol v{nullptr, D->dim[0], D->dim[1], D->dim[2], nullptr, 0, D->brick_sy, D->brick_sz};
+    const int s = i * R.ds;
+    const int pz = cz + (axis == 0 ? s : da);
+    const int py = cy + (axis == 1 ? s : (axis == 0 ? da : db));
+    const int px = cx + (axis == 2 ? s : db);
+    return __ldg(R.fld + brick_offset(pz, py, px, v));
+}
+
+// Class changes go to rows 1.. of the lane's list in shared memory; a list
+// that would be longer than kMaxSegments parks in the row after the last.
+constexpr int kSegRows = kMaxSegments + 1;
+
+struct SlowLeg {
+    float4 L;
+    int len;
+};
+
+// What leg_slow continues from: 0 the start; 1 the wall limit (increments
+// 0..lim-1 accepted); 2 the stop at increment i (only the lengths are left).
+enum SlowFrom { kFromStart = 0, kFromLimit = 1, kFromStop = 2 };
+
+// The rest of a leg that the field march does not finish by itself.
+__device__ __noinline__ SlowLeg leg_slow(const WarpTab &W, int leg, int axis, const short4 *voxel, uint16_t *seg,
+                                         int from, int i, int nseg, int prev, int lim)
+{
+    const short4 cv = __ldg(voxel);
+    const int cz = cv.x, cy = cv.y, cx = cv.z;
+    const SampleDesc &D = *W.desc;
+    const ReflTable *T = W.refl;
+    const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
+    LegResult out;
+    out.Lf[0] = out.Lf[1] = out.Lf[2] = out.Lf[3] = 0.0f;
+    out.len = 1;
+    out.status = kOk;
+    const FaceRule *rules = T->rule[leg];
+    const int face = from == kFromStart ? exit_face(T->head[leg], cz, cy, cx, v) : W.rule[leg][axis].face;
+    if (face == 0)
+        out.status = kErrNoFace;
+    else if (rules[face - 1].status)
+        out.status = rules[face - 1].status;
+    if (out.status == kOk) {
+        LegState S;
+        S.m.last_i = (from == kFromStop ? i : lim) - 1;
+        S.m.nseg = nseg;
+        S.m.prev = prev;
+        S.m.vac = 0;
+        S.face = face;
+        S.lim = lim;
+        S.base = 0;
+        S.need = true;
+        S.coop = from != kFromStart;
+        S.stopped = from == kFromStop;
+        S.live = false;
+        S.b0 = 0;
+        S.dlast = -1;
+        leg_finish<false, true>(rules, cz, cy, cx, v, D.full_iteration, D.voxel, D.sq, D.sq_stride, D.qtab, seg, S,
+                                out, D.voxelf);
+    } else {
+        atomicOr(D.status, 1 << out.status);
+    }
+    SlowLeg r;
+    r.L = make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
+    r.len = out.len;
+    return r;
+}
+
+// Displacement of increment i on the two non-step axes from the reference's
+// FP64 expression (a position near a rounding boundary, inside the volume).
+__device__ __forceinline__ void exact_displacement(const WarpTab &W, int leg, const HotRule &R, int axis,
+                                                   const short4 *voxel, int i, int &da, int &db)
+{
+    const short4 cv = __ldg(voxel);
+    const FaceRule &F = W.refl->rule[leg][R.face - 1];
+    const int a = axis == 0 ? 1 : 0, b = axis == 2 ? 1 : 2;
+    const int ca = axis == 0 ? cv.y : cv.x, cb = axis == 2 ? cv.y : cv.z;
+    const double va = __dadd_rn((double)ca, __dmul_rn((double)i, F.q[a]));
+    const double vb = __dadd_rn((double)cb, __dmul_rn((double)i, F.q[b]));
+    const bool rnd = F.use_round;
+    da = (int)(rnd ? round(va) : floor(va)) - ca;
+    db = (int)(rnd ? round(vb) : floor(vb)) - cb;
+}
+
+// The number of leading increments of a leg that cannot clamp at a wall (the
+// last one excluded where its face clamps it), or 0 when the leg is left to
+// the per-lane march: the path is monotone on every axis, so its first and
+// last points decide; where the far wall is within reach of the whole leg,
+// the part ends at the last increment that stays clear of it.
+__device__ __noinline__ int leg_limit(const FaceRule *R, int cz, int cy, int cx, int dz, int dy, int dx)
+{
+    Vol v{nullptr, dz, dy, dx};
+    LegGeom g;
+    leg_geom(*R, cz, cy, cx, v, g);
+    const int cc = pick3(R->count_axis, cz, cy, cx);
+    const int dd = pick3(R->count_axis, dz, dy, dx);
+    const int steps = R->count_kind == 0 ? cc + 1 : (R->count_kind == 1 ? dd - cc : dd - cc + 1);
+    const int steps_eff = R->count_kind == 2 ? steps - 1 : steps;
+    if (steps_eff <= 1)
+        return 0;
+    int kend = steps_eff - 1;
+    for (int pass = 0; pass < 2; pass++) {
+        const long long ena = g.off + (long long)kend * g.Qa;
+        const long long enb = g.off + (long long)kend * g.Qb;
+        const int a1 = g.ca + (int)((g.off + g.Qa) >> 32), an = g.ca + (int)(ena >> 32);
+        const int b1 = g.cb + (int)((g.off + g.Qb) >> 32), bn = g.cb + (int)(enb >> 32);
+        if (min(a1, an) >= 1 && max(a1, an) <= g.ha - 1 && min(b1, bn) >= 1 && max(b1, bn) <= g.hb - 1)
+            return kend + 1;
+        kend = min(kend, min(wall_increments(R->q[g.ia], g.ca, g.ha), wall_increments(R->q[g.ib], g.cb, g.hb)));
+        if (kend < 1)
+            break;
+    }
+    return 0;
+}
+
+// One leg of one voxel (not warp-synchronous): exit face, march, FP32 lengths
+// (liquor, loop, crystal, bubble).
+//
+// The inner loop is kept to one load, one exit branch and predicated
+// bookkeeping (about 30 instructions) and holds no call: what lives across
+// one would be kept in local memory.  A position near a rounding boundary is
+// off by at most one voxel in the inner loop, still inside the volume (free
+// legs keep a voxel of room, the others their wall limit); the outer loop
+// takes that increment with the exact position.
+template <bool kBrick>
+__device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int &len)
+{
+    // the coordinates are loaded per leg (and again where they are rarely
+    // needed) rather than kept across the march
+    const short4 cv = __ldg(voxel);
+    const int cz = cv.x, cy = cv.y, cx = cv.z;
+    len = 1;
+    // ---- exit face: the smallest of the three distances n_a / |e_a| (n_a
+    // exact, the estimates within 2^-22), when the next one is clearly larger
+    // and the voxel is not on a min plane (a zero distance wins there)
+    const float tx = __fmaf_rn(W.sgn[leg][2], (float)cx, W.org[leg][2]) * W.inv[leg][2];
+    const float ty = __fmaf_rn(W.sgn[leg][1], (float)cy, W.org[leg][1]) * W.inv[leg][1];
+    const float tz = __fmaf_rn(W.sgn[leg][0], (float)cz, W.org[leg][0]) * W.inv[leg][0];
+    const float lo = fminf(tx, ty);
+    const float t1 = fminf(lo, tz), t2 = fmaxf(lo, fminf(fmaxf(tx, ty), tz));
+    const int axis = tx == t1 ? 2 : (ty == t1 ? 1 : 0);
+    const HotRule &R = W.rule[leg][axis];
+    const uint32_t flags = R.flags;
+    int from = kFromStart, i = 0, nseg = 1, prev = 0, lim = 0x7fffffff;
+    bool go = t2 > t1 * (1.0f + 0x1p-20f) && !W.exact_face[leg] && min(cx, min(cy, cz)) > 0 && (flags & kHotSimple);
+    if (go && !(flags & kHotFree)) {
+        lim = leg_limit(&W.refl->rule[leg][R.face - 1], cz, cy, cx, W.desc->dim[0], W.dy, W.dx);
+        go = lim > 1;
+    }
+    if (go) {
+        const uint8_t *start =
+            R.fld + (kBrick ? brick_offset(cz, cy, cx, Vol{nullptr, W.desc->dim[0], W.dy, W.dx, nullptr, 0,
+                                                           W.desc->brick_sy, W.desc->brick_sz})
+                            : (cz * W.dy + cy) * W.dx + cx);
+        uint32_t b = __ldg(start);
+        if ((b & 7u) == 0u)
+            return make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // starts in vacuum
+        const uint32_t qa_lo = R.qa_lo, qa_hi = R.qa_hi, qb_lo = R.qb_lo, qb_hi = R.qb_hi;
+        const unsigned long long off_a = R.off_a, off_b = R.off_b;
+        const int dS = R.dS, Sa = R.Sa, Sb = R.Sb, rq = R.rq;
+        prev = (int)(b & 7u);
+        i = next_increment(0, b, rq);
+        auto take = [&](int lab) {   // class-change bookkeeping and the step
+            if (lab != prev && lab <= 4) {
+                seg[min(nseg, kMaxSegments) * kBlock] = (uint16_t)((lab << 13) | i);
+                nseg++;
+            }
+            prev = lab;
+            i = next_increment(i, b, rq);
+        };
+        from = kFromLimit;
+        while (i < lim) {
+            bool near;
+            for (;;) {
+                uint32_t fa, fb;
+                const int da = fixed_at(i, qa_lo, qa_hi, off_a, fa);
+                const int db = fixed_at(i, qb_lo, qb_hi, off_b, fb);
+                b = field_byte<kBrick>(start, R, W.desc, axis, cz, cy, cx, i, da, db, dS, Sa, Sb);
+                near = min(fa, fb) < 2u * kFieldMargin;
+                const int lab = (int)(b & 7u);
+                if (near | (lab == 0))
+                    break;
+                take(lab);
+                if (i >= lim)
+                    break;
+            }
+            if (i >= lim)
+                break;
+            if (near) {
+                int da, db;
+                exact_displacement(W, leg, R, axis, voxel, i, da, db);
+                b = field_byte<kBrick>(start, R, W.desc, axis, cz, cy, cx, i, da, db, dS, Sa, Sb);
+                if (b & 7u) {
+                    take((int)(b & 7u));
+                    continue;
+                }
+            }
+            from = kFromStop;
+            break;
+        }
+        if (from == kFromStop) {
+            len = i;
+            if (i == 1)
+                return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (nseg <= kMaxSegments) {
+                // the last point's displacement: last_i on the step axis
+                const int last_i = i - 1;
+                uint32_t fa, fb;
+                int da = fixed_at(last_i, qa_lo, qa_hi, off_a, fa);
+                int db = fixed_at(last_i, qb_lo, qb_hi, off_b, fb);
+                if (min(fa, fb) < 2u * kFieldMargin)
+                    exact_displacement(W, leg, R, axis, voxel, last_i, da, db);
+                const int d0 = axis == 0 ? last_i : abs(da);
+                const int d1 = axis == 1 ? last_i : (axis == 0 ? abs(da) : abs(db));
+                const int d2 = axis == 2 ? last_i : abs(db);
+                LegResult out;
+                out.Lf[0] = out.Lf[1] = out.Lf[2] = out.Lf[3] = 0.0f;
+                seg[0] = (uint16_t)(3 << 13);
+                lengths_f32(d0, d1, d2, len, nseg, seg, nullptr, W.voxel, out);
+                return make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
+            }
+        }
+    }
+    seg[0] = (uint16_t)(3 << 13);
+    const SlowLeg r = leg_slow(W, leg, axis, voxel, seg, from, i, nseg, prev, lim);
+    len = r.len;
+    return r.L;
+}
+
 __device__ __forceinline__ int find_sample(const SampleDesc *d, int n, long long item)
 {
     int s = 0;
@@ -1100,7 +1498,44 @@ __device__ __forceinline__ void finish_item(float s, float c, const SampleDesc &
     }
 }
 
-template <int kMinBlocks, bool kField, bool kBrick = false>
+// The end of an absorption work item: the warp's compensated sum, the item's
+// FP64 partial and, for the last tile of the reflection to arrive, the
+// fixed-order combination of the partials into A_h.
+__device__ __forceinline__ void finish_warp_item(float s, float c, const SampleDesc &D, long long r, int t, int lane)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float so = __shfl_down_sync(kAll, s, o);
+        const float co = __shfl_down_sync(kAll, c, o);
+        float ns, e;
+        two_sum(s, so, ns, e);
+        s = ns;
+        c = c + co + e;
+    }
+    int last = 0;
+    if (lane == 0) {
+        D.partial[r * D.tiles + t] = (double)s + (double)c;
+        __threadfence();
+        last = atomicAdd(D.arrive + r, 1u) == (unsigned)(D.tiles - 1);
+    }
+    if (__shfl_sync(kAll, last, 0)) {
+        __threadfence();
+        const volatile double *pp = D.partial + r * D.tiles;
+        double acc = 0.0;
+        for (int k = lane; k < D.tiles; k += 32)
+            acc += pp[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            acc += __shfl_down_sync(kAll, acc, o);
+        if (lane == 0) {
+            D.out[r] = acc / (double)D.n_vox;
+            D.arrive[r] = 0u;   // ready for the next launch
+        }
+    }
+}
+
+// The A_h kernel with the warp-cooperative march.
+template <int kMinBlocks>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const SampleDesc *__restrict__ descs,
                                                                         int n_desc, long long total_items,
                                                                         unsigned long long *__restrict__ work_counter)
@@ -1122,13 +1557,6 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
             break;
         const int si = find_sample(descs, n_desc, item);
         const SampleDesc &D = descs[si];
-        if (kField && (!D.field || (D.brick_sz != 0) != kBrick)) {
-            // a field variant launched over a sample without its field (or
-            // with the other layout): an error status, no reads
-            if (lane == 0)
-                atomicOr(D.status, 1 << kErrArgs);
-            continue;
-        }
         const long long local = item - D.work_begin;
         const long long k = local / D.tiles;
         const long long r = D.order ? (long long)__ldg(D.order + k) : k;
@@ -1142,7 +1570,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
         }
         __syncwarp();
 
-        const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2], D.field, D.field_stride, D.brick_sy, D.brick_sz};
+        const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
         float s = 0.0f, c = 0.0f;
         int bad = kOk;
         unsigned nsteps = 0;
@@ -1156,7 +1584,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
 #pragma unroll 1
             for (int leg = 0; leg < 2; leg++) {
                 LegResult a;
-                trace_leg<false, true, kField, kBrick>(tab.head[leg], tab.rule[leg], cv.x, cv.y, cv.z, valid, v,
+                trace_leg<false, true>(tab.head[leg], tab.rule[leg], cv.x, cv.y, cv.z, valid, v,
                                        D.full_iteration, D.voxel, D.sq, D.sq_stride, D.qtab, seg + tid, a,
                                        D.voxelf);
                 bad |= a.status;
@@ -1189,37 +1617,85 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
             if (lane == 0)
                 atomicAdd(D.steps, w);
         }
-        // warp TwoSum reduction, the item's partial, and the fixed-order
-        // combination of the reflection's partials by the last item to arrive
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float so = __shfl_down_sync(kAll, s, o);
-            const float co = __shfl_down_sync(kAll, c, o);
+        finish_warp_item(s, c, D, r, t, lane);
+    }
+}
+
+// The A_h kernel on packed fields (centred, octant or bricked octant).
+template <int kMinBlocks, bool kBrick>
+__global__ void __launch_bounds__(kBlock, kMinBlocks + 1) field_kernel(const SampleDesc *__restrict__ descs, int n_desc,
+                                                                   long long total_items,
+                                                                   unsigned long long *__restrict__ work_counter)
+{
+    __shared__ WarpTab tabs[kWarps];
+    __shared__ uint16_t seg[kSegRows * kBlock];
+    __shared__ float4 incident[kBlock];
+    __shared__ float2 total[kBlock];   // compensated sums; in shared memory to leave the march its registers
+
+    if (!block_shape_ok(n_desc > 0 ? descs[0].status : nullptr))
+        return;
+    const int tid = threadIdx.x, lane = tid & 31;
+    WarpTab &W = tabs[tid >> 5];
+    for (;;) {
+        unsigned long long it = 0;
+        if (lane == 0)
+            it = atomicAdd(work_counter, 1ull);
+        const long long item = (long long)__shfl_sync(kAll, it, 0);
+        if (item >= total_items)
+            break;
+        const SampleDesc &D = descs[find_sample(descs, n_desc, item)];
+        if (!D.field || (D.brick_sz != 0) != kBrick) {
+            // launched over a sample without its field (or with the other
+            // layout): an error status, no reads
+            if (lane == 0)
+                atomicOr(D.status, 1 << kErrArgs);
+            continue;
+        }
+        const long long local = item - D.work_begin;
+        const long long k = local / D.tiles;
+        const long long r = D.order ? (long long)__ldg(D.order + k) : k;
+        const int t = (int)(local - k * D.tiles);
+        __syncwarp();   // the previous item's reads of the table are done
+        fill_warp_tab(W, D.refl + r, D, lane);
+        __syncwarp();
+
+        total[tid] = make_float2(0.0f, 0.0f);
+        unsigned nsteps = 0;
+        const int n = min(D.tile, D.n_vox - t * D.tile);
+        const short4 *coords = D.coords + (long long)t * D.tile;
+        for (int vi = lane; vi < n; vi += 32) {
+            float4 L;
+#pragma unroll 1
+            for (int leg = 0; leg < 2; leg++) {
+                int len;
+                L = field_leg<kBrick>(W, leg, coords + vi, seg + tid, len);
+                if (W.count_steps)
+                    nsteps += (unsigned)len;
+                // the incident leg's lengths wait in shared memory
+                if (leg == 0)
+                    incident[tid] = L;
+            }
+            // L_incident + L_diffracted per class and cal_rate's exponent
+            // (AnACor/src/ray_tracing_basic.c:1573-1576), in FP32
+            const float4 I = incident[tid];
+            const float ex = W.mu[0] * (I.x + L.x) + W.mu[1] * (I.y + L.y) + W.mu[2] * (I.z + L.z) +
+                             W.mu[3] * (I.w + L.w);
+            const float term = W.is_exp ? expf(-ex) : ex;
+            const float2 sc = total[tid];
             float ns, e;
-            two_sum(s, so, ns, e);
-            s = ns;
-            c = c + co + e;
+            two_sum(sc.x, term, ns, e);
+            total[tid] = make_float2(ns, sc.y + e);
         }
-        int last = 0;
-        if (lane == 0) {
-            D.partial[r * D.tiles + t] = (double)s + (double)c;
-            __threadfence();
-            last = atomicAdd(D.arrive + r, 1u) == (unsigned)(D.tiles - 1);
-        }
-        if (__shfl_sync(kAll, last, 0)) {
-            __threadfence();
-            const volatile double *pp = D.partial + r * D.tiles;
-            double acc = 0.0;
-            for (int k = lane; k < D.tiles; k += 32)
-                acc += pp[k];
+        __syncwarp();
+        if (D.steps) {
+            unsigned long long w = nsteps;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
-                acc += __shfl_down_sync(kAll, acc, o);
-            if (lane == 0) {
-                D.out[r] = acc / (double)D.n_vox;
-                D.arrive[r] = 0u;   // ready for the next launch
-            }
+                w += __shfl_down_sync(kAll, w, o);
+            if (lane == 0)
+                atomicAdd(D.steps, w);
         }
+        finish_warp_item(total[tid].x, total[tid].y, D, r, t, lane);
     }
 }
 
@@ -1678,23 +2154,24 @@ cudaError_t launch_absorption(const SampleDesc *d_descs, int n_desc, long long t
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess)
         return e;
-#define ANACOR_LAUNCH(B, F, K) \
-    absorption_kernel<B, F, K><<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter)
+#define ANACOR_COOP(B) absorption_kernel<B><<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter)
+#define ANACOR_FIELD(B, K) field_kernel<B, K><<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter)
     switch (variant > 0 ? variant : absorption_variant()) {
-    case 1: ANACOR_LAUNCH(1, false, false); break;
-    case 3: ANACOR_LAUNCH(3, false, false); break;
-    case 4: ANACOR_LAUNCH(4, false, false); break;
-    case 5: ANACOR_LAUNCH(1, true, false); break;
-    case 6: ANACOR_LAUNCH(2, true, false); break;
-    case 7: ANACOR_LAUNCH(3, true, false); break;
-    case 8: ANACOR_LAUNCH(4, true, false); break;
-    case 9: ANACOR_LAUNCH(1, true, true); break;
-    case 10: ANACOR_LAUNCH(2, true, true); break;
-    case 11: ANACOR_LAUNCH(3, true, true); break;
-    case 12: ANACOR_LAUNCH(4, true, true); break;
-    default: ANACOR_LAUNCH(2, false, false); break;
+    case 1: ANACOR_COOP(1); break;
+    case 3: ANACOR_COOP(3); break;
+    case 4: ANACOR_COOP(4); break;
+    case 5: ANACOR_FIELD(1, false); break;
+    case 6: ANACOR_FIELD(2, false); break;
+    case 7: ANACOR_FIELD(3, false); break;
+    case 8: ANACOR_FIELD(4, false); break;
+    case 9: ANACOR_FIELD(1, true); break;
+    case 10: ANACOR_FIELD(2, true); break;
+    case 11: ANACOR_FIELD(3, true); break;
+    case 12: ANACOR_FIELD(4, true); break;
+    default: ANACOR_COOP(2); break;
     }
-#undef ANACOR_LAUNCH
+#undef ANACOR_COOP
+#undef ANACOR_FIELD
     return cudaGetLastError();
 }
 
@@ -1788,7 +2265,7 @@ int block_guard_selftest(int threads, int *status_out)
         cudaMemset(counter, 0, sizeof(unsigned long long)) == cudaSuccess) {
         h.status = status;
         if (cudaMemcpy(d, &h, sizeof(h), cudaMemcpyHostToDevice) == cudaSuccess) {
-            absorption_kernel<2, false><<<2, threads>>>(d, 1, 0, counter);
+            absorption_kernel<2><<<2, threads>>>(d, 1, 0, counter);
             if (cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess &&
                 cudaMemcpy(status_out, status, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess)
                 rc = kOk;
@@ -1805,11 +2282,15 @@ int block_guard_selftest(int threads, int *status_out)
 int absorption_set_carveout(int pct)
 {
     cudaError_t e = cudaSuccess;
-#define ANACOR_CARVE(B, F) \
+#define ANACOR_CARVE(K) \
     if (e == cudaSuccess) \
-        e = cudaFuncSetAttribute(absorption_kernel<B, F>, cudaFuncAttributePreferredSharedMemoryCarveout, pct)
-    ANACOR_CARVE(1, false); ANACOR_CARVE(2, false); ANACOR_CARVE(3, false); ANACOR_CARVE(4, false);
-    ANACOR_CARVE(1, true); ANACOR_CARVE(2, true); ANACOR_CARVE(3, true); ANACOR_CARVE(4, true);
+        e = cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, pct)
+    ANACOR_CARVE(absorption_kernel<1>); ANACOR_CARVE(absorption_kernel<2>);
+    ANACOR_CARVE(absorption_kernel<3>); ANACOR_CARVE(absorption_kernel<4>);
+#define ANACOR_CARVE2(B) \
+    ANACOR_CARVE((field_kernel<B, false>)); ANACOR_CARVE((field_kernel<B, true>))
+    ANACOR_CARVE2(1); ANACOR_CARVE2(2); ANACOR_CARVE2(3); ANACOR_CARVE2(4);
+#undef ANACOR_CARVE2
 #undef ANACOR_CARVE
     return e == cudaSuccess ? kOk : kErrCuda;
 }
@@ -1817,21 +2298,20 @@ int absorption_set_carveout(int pct)
 int absorption_occupancy(int *blocks_per_sm, int variant)
 {
     cudaError_t e;
-#define ANACOR_OCC(B, F, K) \
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, absorption_kernel<B, F, K>, kBlock, 0)
+#define ANACOR_OCC(K) cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, K, kBlock, 0)
     switch (variant > 0 ? variant : absorption_variant()) {
-    case 1: e = ANACOR_OCC(1, false, false); break;
-    case 3: e = ANACOR_OCC(3, false, false); break;
-    case 4: e = ANACOR_OCC(4, false, false); break;
-    case 5: e = ANACOR_OCC(1, true, false); break;
-    case 6: e = ANACOR_OCC(2, true, false); break;
-    case 7: e = ANACOR_OCC(3, true, false); break;
-    case 8: e = ANACOR_OCC(4, true, false); break;
-    case 9: e = ANACOR_OCC(1, true, true); break;
-    case 10: e = ANACOR_OCC(2, true, true); break;
-    case 11: e = ANACOR_OCC(3, true, true); break;
-    case 12: e = ANACOR_OCC(4, true, true); break;
-    default: e = ANACOR_OCC(2, false, false); break;
+    case 1: e = ANACOR_OCC(absorption_kernel<1>); break;
+    case 3: e = ANACOR_OCC(absorption_kernel<3>); break;
+    case 4: e = ANACOR_OCC(absorption_kernel<4>); break;
+    case 5: e = ANACOR_OCC((field_kernel<1, false>)); break;
+    case 6: e = ANACOR_OCC((field_kernel<2, false>)); break;
+    case 7: e = ANACOR_OCC((field_kernel<3, false>)); break;
+    case 8: e = ANACOR_OCC((field_kernel<4, false>)); break;
+    case 9: e = ANACOR_OCC((field_kernel<1, true>)); break;
+    case 10: e = ANACOR_OCC((field_kernel<2, true>)); break;
+    case 11: e = ANACOR_OCC((field_kernel<3, true>)); break;
+    case 12: e = ANACOR_OCC((field_kernel<4, true>)); break;
+    default: e = ANACOR_OCC(absorption_kernel<2>); break;
     }
 #undef ANACOR_OCC
     return e == cudaSuccess ? kOk : kErrCuda;

@@ -48,6 +48,8 @@ struct SampleDesc {
     long long field_stride; // 0: one centred field; else 8 octant fields this far apart (launch_octant_fields)
     int brick_sy, brick_sz; // 0: linear fields; else 4^3-bricked (launch_brick_fields), byte strides of a
                             // brick step in y and z; required by variants 9..12
+    const int *walls;       // optional [6]: voxels between the non-vacuum labels and the volume's walls
+                            // (launch_wall_room), for the field march
     const int *order;       // optional [n_refl]: the k-th reflection processed (octant-sorted), else k
 };
 
@@ -153,6 +155,10 @@ cudaError_t launch_distance_field(const int8_t *d_vol, const int *dims, uint8_t 
 // d_out holds 8 volumes, d_tmp 6.
 cudaError_t launch_octant_fields(const int8_t *d_vol, const int *dims, uint8_t *d_out, uint8_t *d_tmp, int *d_bad,
                                  cudaStream_t st);
+// d_room[a] = the smallest coordinate on axis a (z, y, x) of a voxel that is
+// not vacuum, d_room[3 + a] = the smallest dims[a] - 1 - coordinate (large
+// values when every voxel is vacuum).
+cudaError_t launch_wall_room(const int8_t *d_vol, const int *dims, int *d_room, cudaStream_t st);
 // Bricked copies of `n_fields` linear fields (each dims[0]*dims[1]*dims[2]
 // bytes, consecutive): 4x4x4 bricks of 64 bytes in (z, y, x) brick order,
 // bytes (z, y, x) inside a brick, padding bytes 0.  Each copy holds
