@@ -274,7 +274,8 @@ struct anacor_plan {
     int64_t n_refl = 0, refl_cap = 0;
     size_t partial_cap = 0;        // entries of d_partial (refl_cap * tiles)
     int tiles = 0;
-    int tile = kTile;              // voxels per work item
+    int tile = kTile;              // most voxels of a work item (the configured tile)
+    int work_tile = kTile;         // voxels per work item (plan_split)
     int variant = 0;               // register-budget variant (0: process default)
     int order = 1;                 // voxel order of the packed list (0 the caller's, 1 Morton, 2.. blocked)
     long long *d_c64 = nullptr;    // the caller's int64 voxel list (for re-packing)
@@ -445,6 +446,8 @@ private:
     pid_t pid_ = 0;
 };
 
+constexpr int kItemsPerWarp = 4;
+
 // the tile actually used: at least `tile`, and large enough that a reflection
 // has at most kMaxTilesPerRefl tiles (a multiple of 32 voxels)
 int effective_tile(int n_vox, int tile)
@@ -453,6 +456,28 @@ int effective_tile(int n_vox, int tile)
     if (need > tile)
         tile = (int)((need + 31) / 32 * 32);
     return tile;
+}
+
+// Work items of the plan's reflections: the configured tile, halved (down to
+// one voxel per lane) while there are fewer than four items for each of the
+// forty warps an SM runs, so that the last wave is short and a handful of
+// reflections still fills the device (3,001 reflections of 1,150 voxels: 926
+// us at one item a warp, 810 at four, 840 at nine; six samples in one batch,
+// whose items are many already: 3.98 ms, 4.01, 4.26).  The per-voxel terms are
+// summed with compensation, so the split changes A_h by less than 1e-12.
+int plan_ensure_partial(anacor_plan *p);
+long long wanted_items(const anacor_plan *p) { return (long long)p->dev->sms * 40 * kItemsPerWarp; }
+int plan_split(anacor_plan *p)
+{
+    const long long want = wanted_items(p);
+    const int least = effective_tile(p->n_vox, 32);
+    int t = p->tile;
+    auto tiles = [&](int x) { return ((long long)p->n_vox + x - 1) / x; };
+    while (t > least && p->n_refl * tiles(t) < want)
+        t = std::max(least, (t / 2 + 31) / 32 * 32);
+    p->work_tile = t;
+    p->tiles = (int)tiles(t);
+    return plan_ensure_partial(p);
 }
 
 // Volume, tables and sizes of a plan (the voxel list comes next).
@@ -517,7 +542,8 @@ int plan_set_voxels(anacor_plan *p, const int64_t *coords, int64_t n, bool on_de
     dev_free(p->d_c64, st);
     p->n_vox = (int)n;
     p->tile = effective_tile(p->n_vox, p->tile);
-    p->tiles = (int)((n + p->tile - 1) / p->tile);
+    if (int s = plan_split(p))
+        return s;
     cudaError_t e;
     if ((e = dev_alloc(&p->d_coords, (size_t)n, st)) || (e = dev_alloc(&p->d_c64, (size_t)n * 3, st)))
         return cuda_fail(e, "device allocation");
@@ -592,9 +618,14 @@ int sample_voxels_device(anacor_plan *p, int code, int method, int64_t sampling_
 }
 
 // tile partial sums: one per (reflection, tile) for the reserved reflections
+// at the configured tile, and at least the most items plan_split makes (fewer
+// reflections later are split further without a new allocation)
 int plan_ensure_partial(anacor_plan *p)
 {
-    const size_t need = (size_t)p->refl_cap * (size_t)std::max(1, p->tiles);
+    if (p->refl_cap == 0)
+        return kOk;
+    const size_t tiles = ((size_t)p->n_vox + p->tile - 1) / p->tile;
+    const size_t need = std::max((size_t)p->refl_cap * std::max<size_t>(1, tiles), (size_t)(2 * wanted_items(p)));
     if (need <= p->partial_cap)
         return kOk;
     cudaStream_t st = p->stream;
@@ -633,7 +664,7 @@ int plan_reserve_refl(anacor_plan *p, int64_t n_refl)
         p->refl_cap = n_refl;
     }
     p->n_refl = n_refl;
-    return plan_ensure_partial(p);
+    return plan_split(p);
 }
 
 // The packed distance field of the plan's volume (variants 5..8), built once.
@@ -739,7 +770,7 @@ SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1)
     d.refl = p->d_refl;
     d.n_refl = p->n_refl;
     d.tiles = p->tiles;
-    d.tile = p->tile;
+    d.tile = p->work_tile;
     d.full_iteration = p->full;
     d.is_exp = p->is_exp;
     d.out = p->d_out;
@@ -863,11 +894,12 @@ int plan_launch_bisection(anacor_plan *p, cudaStream_t st, int num_cls)
     const long long items = (long long)p->n_refl * p->tiles;
     if (items == 0)
         return kOk;
-    static int bps = 0;
-    if (!bps && (bisection_occupancy(&bps) != kOk || bps <= 0))
+    const bool fixed = std::max(p->dims[0], std::max(p->dims[1], p->dims[2])) <= kBisectFixedDim;
+    int bps = 0;
+    if (bisection_occupancy(&bps, fixed) != kOk || bps <= 0)
         bps = 1;
     const int grid = (int)std::max(1ll, std::min(items, (long long)p->dev->sms * bps));
-    cudaError_t e = launch_bisection(p->d_desc, 1, items, p->d_counter, grid, num_cls, st);
+    cudaError_t e = launch_bisection(p->d_desc, 1, items, p->d_counter, grid, num_cls, fixed, st);
     if (e != cudaSuccess)
         return cuda_fail(e, "kernel launch");
     return kOk;
@@ -971,8 +1003,7 @@ int plan_configure(anacor_plan *p, int variant, int tile, int order)
         p->order = order;
     if (tile) {
         p->tile = effective_tile(p->n_vox, tile);
-        p->tiles = (int)(((long long)p->n_vox + p->tile - 1) / p->tile);
-        if (int st = plan_ensure_partial(p))
+        if (int st = plan_split(p))
             return st;
     }
     p->variant = variant;
@@ -1062,8 +1093,7 @@ bool tune_lookup(const anacor_plan *p, TuneVal &v)
 // the distance-field march for volumes with an axis of 256 voxels or more
 // (long legs: it steps over most increments; 25-50 % faster there, while the
 // cooperative march is as fast on a 96^3 volume) and the cooperative march
-// below that, with the largest tile up to 1024 voxels that still gives every
-// warp four work items.
+// below that.
 int plan_default_config(anacor_plan *p)
 {
     TuneVal v{0, 0, 1, 0.0f};
@@ -1078,16 +1108,8 @@ int plan_default_config(anacor_plan *p)
             variant = 12;
         succeed();   // labels outside 0..7: the cooperative march, no error
     }
-    // the largest tile that still gives every warp slot four items (the
-    // cooperative march, 32 warps a SM) or sixteen (the field march, 40)
-    const long long warps = (long long)p->dev->sms * (variant ? 160 : 32);
-    int tile = kMinTile;
-    for (int t : {2048, 1024, 512, 256})
-        if ((!variant || t <= 1024) && p->n_refl * (((long long)p->n_vox + t - 1) / t) >= 4 * warps) {
-            tile = t;
-            break;
-        }
-    return plan_configure(p, variant, tile, -1);
+    // plan_split makes the items smaller where there are few
+    return plan_configure(p, variant, variant ? 1024 : 2048, -1);
 }
 
 }  // namespace

@@ -29,4 +29,80 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
     e = (a - (s - bp)) + (b - bp);
 }
 
+// ---- pairs of floats (h + l, |l| <= ulp(h) / 2) ----------------------------
+//
+// About 46 significant bits from FP32 instructions (Dekker, "A floating-point
+// technique for extending the available precision", Numer. Math. 18, 1971),
+// where GB300's FP64 pipe would bind a kernel: an FP64 instruction takes a
+// warp 16 cycles there, an FP32 one a quarter of a cycle.
+
+struct FloatPair {
+    float h, l;
+};
+
+__device__ __forceinline__ FloatPair pair_of(double x)
+{
+    const float h = (float)x;
+    return {h, (float)(x - (double)h)};
+}
+
+// h + l with |l| <= |h| renormalised (Fast2Sum)
+__device__ __forceinline__ FloatPair pair_norm(float h, float l)
+{
+    const float s = __fadd_rn(h, l);
+    return {s, __fadd_rn(l, -__fadd_rn(s, -h))};
+}
+
+__device__ __forceinline__ FloatPair pair_add(FloatPair a, FloatPair b)
+{
+    const float s = __fadd_rn(a.h, b.h);
+    const float t = __fadd_rn(s, -a.h);
+    const float e = __fadd_rn(__fadd_rn(a.h, -__fadd_rn(s, -t)), __fadd_rn(b.h, -t));
+    return pair_norm(s, __fadd_rn(e, __fadd_rn(a.l, b.l)));
+}
+
+__device__ __forceinline__ FloatPair pair_neg(FloatPair a) { return {-a.h, -a.l}; }
+
+// a * b for a float b
+__device__ __forceinline__ FloatPair pair_mul(FloatPair a, float b)
+{
+    const float p = __fmul_rn(a.h, b);
+    return pair_norm(p, __fmaf_rn(a.l, b, __fmaf_rn(a.h, b, -p)));
+}
+
+__device__ __forceinline__ FloatPair pair_mul(FloatPair a, FloatPair b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    return pair_norm(p, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.h, -p))));
+}
+
+// square root: one Newton step on the FP32 root
+__device__ __forceinline__ FloatPair pair_sqrt(FloatPair a)
+{
+    if (!(a.h > 0.0f))
+        return {0.0f, 0.0f};
+    const float s = __fsqrt_rn(a.h);
+    const float r = __fadd_rn(__fmaf_rn(-s, s, a.h), a.l);   // a - s^2 (exact but for a.l's place)
+    return pair_norm(s, __fdividef(r, __fadd_rn(s, s)));
+}
+
+// exp(-x) as exp_neg, from a pair: the same k and the same FP32 r but where
+// r's rounding is a near tie.  ln 2 as the sum of three floats, each the
+// rounding of what the ones before leave, the first cut to 12 bits so that
+// its product with k is exact.
+__device__ __forceinline__ float exp_neg(FloatPair x)
+{
+    const float k = rintf(__fmul_rn(x.h, 1.44269504f));
+    const float c1 = 2839.0f / 4096.0f;
+    const float c2 = 0x1.0bfbe80000000p-15f;
+    const float c3 = 0x1.cf79ac0000000p-40f;
+    const float t = __fmaf_rn(-k, c1, x.h);   // exact
+    const float p = __fmul_rn(-k, c2);
+    const float pe = __fmaf_rn(-k, c2, -p);
+    const FloatPair r = pair_add({t, 0.0f}, pair_add({p, pe}, {x.l, -k * c3}));
+    const float e = expf(-__fadd_rn(r.h, r.l));
+    const int n = (int)fmaxf(fminf(k, 400.0f), -400.0f);
+    return ldexpf(e, -n);
+}
+
 }  // namespace anacor

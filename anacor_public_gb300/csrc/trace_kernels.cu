@@ -1951,6 +1951,282 @@ __global__ void __launch_bounds__(kBlock, 2) bisection_kernel(const SampleDesc *
     }
 }
 
+// ---- bisection in fixed point ----------------------------------------------
+//
+// The same searches for volumes with axes of at most kBisectFixedDim voxels.
+// Every value a search halves is a dyadic number there: the first one starts
+// from [0, n] with n < 2^10 and halves at most 10 times, each later one starts
+// from earlier results and adds at most 10 bits, the deepest chain (sample
+// boundary, crystal boundary, loop or bubble inner, outer boundary) ends on
+// multiples of 2^-40.  The reference's FP64 halvings are exact on such values
+// (at most 50 bits), so 24.40 integers take the same decisions.
+//
+// Probe points floor(c + mid q): on the step axis c +- mid exactly; on the
+// others mid cut to 11.21 times the rule's 32.32 ratio, T = floor(product) in
+// 2^-21 units (32-bit: the exit face is the nearest, so displacements stay
+// below 2^10).  It is off by at most |q| + 1.25 units (mid's and T's cuts, Q's
+// rounding); a fraction within `margin` >= |q| + 2 units of an integer is
+// recomputed with the reference's FP64 expression.  Lengths and the exponent
+// run on pairs of floats.
+//
+// What is left is a chain of about 45 dependent label loads per ray, one ray
+// a lane, so the kernel is bound by load latency and the warps an SM holds.
+// 288x240x257, 6,800 voxels, 701 reflections: a call 8.9 ms (FP64 searches,
+// FP64 pipe) -> 1.27 ms, A_h bit for bit the same.  Longer axes keep the FP64
+// searches: their halvings would need more than 40 fractional bits.
+
+constexpr long long kBisectOne = 1ll << 40;
+
+struct BisectRay {
+    const int8_t *start;     // the voxel's label
+    uint32_t qa_lo, qa_hi, qb_lo, qb_hi;
+    uint32_t margin;         // in 2^-21 units
+    int ds, Ss, Sa, Sb;      // step direction; element strides
+    int cs, ca, cb;          // start coordinates
+    int ns, na, nb;          // dimensions
+};
+
+// the reference's FP64 probe point of axis a (0 z, 1 y, 2 x)
+__device__ __noinline__ int bisect_exact(const WarpTab &W, int leg, int face, int axis, int c, double mid)
+{
+    const double x = floor(__dadd_rn((double)c, __dmul_rn(mid, W.refl->rule[leg][face - 1].q[axis])));
+    return x >= -1.0 && x <= 8192.0 ? (int)x : -1;
+}
+
+// One boundary search: longest moves in on a label equal to cls (boundary 0),
+// or shortest moves out on one (boundary 1).  False when a probe leaves the
+// volume.
+__device__ __forceinline__ bool bisect_fixed(const BisectRay &r, const WarpTab &W, int leg, int axis,
+                                             long long longest, long long shortest, bool boundary, int cls,
+                                             long long &mid)
+{
+    mid = (longest + shortest) >> 1;
+    while (longest - shortest > kBisectOne) {
+        mid = (longest + shortest) >> 1;
+        const uint32_t m = (uint32_t)(mid >> 19);
+        const int ta = (int)(__umulhi(m, r.qa_lo) + m * r.qa_hi);
+        const int tb = (int)(__umulhi(m, r.qb_lo) + m * r.qb_hi);
+        const int whole = (int)(mid >> 40);
+        const int sd = r.ds > 0 ? whole : -whole - ((mid & (kBisectOne - 1)) != 0);
+        int da = ta >> 21, db = tb >> 21;
+        constexpr uint32_t kFrac = (1u << 21) - 1u;
+        if (min(((uint32_t)ta + r.margin) & kFrac, ((uint32_t)tb + r.margin) & kFrac) < 2u * r.margin) {
+            const double md = (double)mid * 0x1p-40;
+            const int face = W.rule[leg][axis].face;
+            da = bisect_exact(W, leg, face, axis == 0 ? 1 : 0, r.ca, md) - r.ca;
+            db = bisect_exact(W, leg, face, axis == 2 ? 1 : 2, r.cb, md) - r.cb;
+        }
+        if ((unsigned)(r.cs + sd) >= (unsigned)r.ns || (unsigned)(r.ca + da) >= (unsigned)r.na ||
+            (unsigned)(r.cb + db) >= (unsigned)r.nb)
+            return false;
+        const int lab = __ldg(r.start + (sd * r.Ss + da * r.Sa + db * r.Sb));
+        if ((lab == cls) != boundary)
+            longest = mid;
+        else
+            shortest = mid;
+    }
+    return true;
+}
+
+// the search's point floor(c + floor(mid) q) as its displacement on (step
+// axis, a, b)
+struct BisectPoint {
+    int s, a, b;
+};
+
+__device__ __forceinline__ BisectPoint bisect_point(const BisectRay &r, const WarpTab &W, int leg, int axis,
+                                                    long long mid)
+{
+    const int i = (int)(mid >> 40);
+    uint32_t fa, fb;
+    BisectPoint p;
+    p.s = r.ds * i;
+    p.a = fixed_at(i, r.qa_lo, r.qa_hi, kFieldMargin, fa);
+    p.b = fixed_at(i, r.qb_lo, r.qb_hi, kFieldMargin, fb);
+    if (min(fa, fb) < 2u * kFieldMargin) {
+        const int face = W.rule[leg][axis].face;
+        p.a = bisect_exact(W, leg, face, axis == 0 ? 1 : 0, r.ca, (double)i) - r.ca;
+        p.b = bisect_exact(W, leg, face, axis == 2 ? 1 : 2, r.cb, (double)i) - r.cb;
+    }
+    return p;
+}
+
+__device__ __forceinline__ BisectPoint operator-(const BisectPoint &x, const BisectPoint &y)
+{
+    return {x.s - y.s, x.a - y.a, x.b - y.b};
+}
+
+__device__ __forceinline__ int abs_sum(const BisectPoint &d) { return abs(d.s) + abs(d.a) + abs(d.b); }
+
+// length of a displacement; v2: the squared voxel edges of (step axis, a, b)
+__device__ __forceinline__ FloatPair pair_length(const BisectPoint &d, const FloatPair *v2)
+{
+    const FloatPair s = pair_add(pair_add(pair_mul(v2[0], (float)(d.s * d.s)), pair_mul(v2[1], (float)(d.a * d.a))),
+                                 pair_mul(v2[2], (float)(d.b * d.b)));
+    return pair_sqrt(s);
+}
+
+// iterative_bisection and cal_path_bisection (AnACor/src/bisection.c:272-463)
+// for one leg; adds mu_m L_m to `sum`.  Returns a status.
+__device__ __forceinline__ int bisect_leg_fixed(const BisectRay &r, const WarpTab &W, int leg, int axis, int reach,
+                                                int num_cls, const FloatPair *v2, const FloatPair *mu, FloatPair *L)
+{
+    long long m_air, m_cr, m_in, m_out;
+    if (!bisect_fixed(r, W, leg, axis, (long long)reach << 40, 0, false, 0, m_air) ||
+        !bisect_fixed(r, W, leg, axis, m_air, 0, true, 3, m_cr))
+        return kErrArgs;
+    const BisectPoint air = bisect_point(r, W, leg, axis, m_air);
+    FloatPair pair_l = {0.0f, 0.0f};   // the last pair of points found
+    int pairs = 0;
+    bool more = true;
+    if (!bisect_fixed(r, W, leg, axis, m_air, m_cr, false, 2, m_in))
+        return kErrArgs;
+    BisectPoint in = bisect_point(r, W, leg, axis, m_in);
+    if (abs_sum(in - air) > 3) {
+        if (!bisect_fixed(r, W, leg, axis, m_air, m_in, true, 2, m_out))
+            return kErrArgs;
+        const BisectPoint d = in - bisect_point(r, W, leg, axis, m_out);
+        if (abs_sum(d) <= 6) {
+            more = false;
+        } else {
+            pair_l = pair_length(d, v2);
+            pairs = 1;
+        }
+    }
+    if (more && num_cls > 3) {
+        if (!bisect_fixed(r, W, leg, axis, m_air, m_cr, false, 4, m_in))
+            return kErrArgs;
+        in = bisect_point(r, W, leg, axis, m_in);
+        if (abs_sum(in - air) > 1) {
+            if (!bisect_fixed(r, W, leg, axis, m_air, m_in, true, 4, m_out))
+                return kErrArgs;
+            const BisectPoint d = in - bisect_point(r, W, leg, axis, m_out);
+            if (abs_sum(d) > 6) {
+                pair_l = pair_length(d, v2);
+                pairs++;
+            }
+        }
+    }
+    // read from the path by its length: one pair is counted as loop, of two
+    // the second as bubble
+    const FloatPair cr = pair_length(bisect_point(r, W, leg, axis, m_cr), v2);
+    L[0] = pair_add(pair_add(pair_length(air, v2), pair_neg(pair_l)), pair_neg(cr));
+    L[1] = pairs == 1 ? pair_l : FloatPair{0.0f, 0.0f};
+    L[2] = cr;
+    L[3] = pairs == 2 ? pair_l : FloatPair{0.0f, 0.0f};
+    return kOk;
+}
+
+__global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const SampleDesc *__restrict__ descs, int n_desc,
+                                                                    long long total_items,
+                                                                    unsigned long long *__restrict__ work_counter,
+                                                                    int num_cls)
+{
+    __shared__ WarpTab tabs[kWarps];
+    __shared__ FloatPair consts[kWarps][7];   // squared voxel edges (z, y, x), mu
+    if (!block_shape_ok(n_desc > 0 ? descs[0].status : nullptr))
+        return;
+    const int tid = threadIdx.x, lane = tid & 31;
+    WarpTab &W = tabs[tid >> 5];
+    FloatPair *K = consts[tid >> 5];
+    for (;;) {
+        unsigned long long it = 0;
+        if (lane == 0)
+            it = atomicAdd(work_counter, 1ull);
+        const long long item = (long long)__shfl_sync(kAll, it, 0);
+        if (item >= total_items)
+            break;
+        const SampleDesc &D = descs[find_sample(descs, n_desc, item)];
+        const long long local = item - D.work_begin;
+        const long long k = local / D.tiles;
+        const long long refl = D.order ? (long long)__ldg(D.order + k) : k;
+        const int t = (int)(local - k * D.tiles);
+        __syncwarp();   // the previous item's reads of the table are done
+        fill_warp_tab(W, D.refl + refl, D, lane);
+        if (lane < 3)
+            K[lane] = pair_of(__dmul_rn(D.voxel[lane], D.voxel[lane]));
+        else if (lane < 7)
+            K[lane] = pair_of(D.mu[lane - 3]);
+        __syncwarp();
+        float s = 0.0f, c = 0.0f;
+        const int n = min(D.tile, D.n_vox - t * D.tile);
+        const short4 *coords = D.coords + (long long)t * D.tile;
+        for (int vi = lane; vi < n; vi += 32) {
+            FloatPair L[2][4];
+            int bad = kOk;
+#pragma unroll 1
+            for (int leg = 0; leg < 2 && !bad; leg++) {
+                const short4 cv = __ldg(coords + vi);
+                const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
+                const int face = exit_face(D.refl[refl].head[leg], cv.x, cv.y, cv.z, v);
+                if (face == 0) {
+                    bad = kErrNoFace;
+                    break;
+                }
+                // the rule of the exit axis (of its own face: a start on a min
+                // plane may leave against the direction of travel)
+                const FaceRule &F = D.refl[refl].rule[leg][face - 1];
+                if (F.status) {
+                    bad = F.status;
+                    break;
+                }
+                const int axis = F.count_axis;
+                const HotRule &R = W.rule[leg][axis];
+                const int dz = D.dim[0], dy = D.dim[1], dx = D.dim[2];
+                int reach;
+                switch (face) {
+                case 4: reach = cv.y; break;
+                case 5: reach = dy - 1 - cv.y; break;
+                case 6: reach = cv.z; break;
+                case 1: reach = dx - 1 - cv.z; break;
+                case 2: reach = cv.x; break;
+                default: reach = dz - 1 - cv.x; break;
+                }
+                const long long qm = max(F.Q[axis == 0 ? 1 : 0] < 0 ? -F.Q[axis == 0 ? 1 : 0] : F.Q[axis == 0 ? 1 : 0],
+                                         F.Q[axis == 2 ? 1 : 2] < 0 ? -F.Q[axis == 2 ? 1 : 2] : F.Q[axis == 2 ? 1 : 2]);
+                if (!F.fast || R.face != face || qm >= 64ll << 32) {
+                    // ratios beyond the 32-bit products: the FP64 searches
+                    double Ld[4];
+                    bad = ib_leg(D.refl[refl].head[leg], D.refl[refl].rule[leg], cv.x, cv.y, cv.z, v, num_cls, D.voxel,
+                                 Ld);
+                    for (int m = 0; m < 4; m++)
+                        L[leg][m] = pair_of(Ld[m]);
+                    continue;
+                }
+                BisectRay r;
+                r.start = D.vol + ((long long)cv.x * dy + cv.y) * dx + cv.z;
+                r.qa_lo = R.qa_lo; r.qa_hi = R.qa_hi; r.qb_lo = R.qb_lo; r.qb_hi = R.qb_hi;
+                r.margin = (uint32_t)(qm >> 32) + 3u;
+                r.ds = R.ds;
+                r.Ss = R.dS * R.ds; r.Sa = R.Sa; r.Sb = R.Sb;
+                r.cs = pick3(axis, cv.x, cv.y, cv.z);
+                r.ca = axis == 0 ? cv.y : cv.x;
+                r.cb = axis == 2 ? cv.y : cv.z;
+                r.ns = pick3(axis, dz, dy, dx);
+                r.na = axis == 0 ? dy : dz;
+                r.nb = axis == 2 ? dy : dx;
+                const FloatPair v2[3] = {K[axis], K[axis == 0 ? 1 : 0], K[axis == 2 ? 1 : 2]};
+                bad = bisect_leg_fixed(r, W, leg, axis, reach, num_cls, v2, K + 3, L[leg]);
+            }
+            if (bad) {
+                atomicOr(D.status, 1 << bad);
+                continue;
+            }
+            // cal_rate (AnACor/src/ray_tracing_basic.c:1573-1576)
+            FloatPair ex = {0.0f, 0.0f};
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+                ex = pair_add(ex, pair_mul(pair_add(L[0][m], L[1][m]), K[3 + m]));
+            float ns, e;
+            two_sum(s, exp_neg(ex), ns, e);
+            s = ns;
+            c += e;
+        }
+        __syncwarp();
+        finish_warp_item(s, c, D, refl, t, lane);
+    }
+}
+
 // Absorption map: work item = (grid direction, tile of voxels); the
 // diffracted leg of every voxel, one output per (direction, voxel).
 template <bool kField>
@@ -2189,14 +2465,17 @@ cudaError_t launch_leg_detail(const ReflTable *d_tab, const int8_t *d_vol, const
 }
 
 cudaError_t launch_bisection(const SampleDesc *d_descs, int n_desc, long long total_items,
-                             unsigned long long *d_counter, int grid, int num_cls, cudaStream_t st)
+                             unsigned long long *d_counter, int grid, int num_cls, bool fixed, cudaStream_t st)
 {
     if (total_items <= 0)
         return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess)
         return e;
-    bisection_kernel<<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter, num_cls);
+    if (fixed)
+        bisection_fixed_kernel<<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter, num_cls);
+    else
+        bisection_kernel<<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter, num_cls);
     return cudaGetLastError();
 }
 
@@ -2212,11 +2491,12 @@ cudaError_t launch_ib_direction(const ReflTable *d_dir, const int8_t *d_vol, con
     return cudaGetLastError();
 }
 
-int bisection_occupancy(int *blocks_per_sm)
+int bisection_occupancy(int *blocks_per_sm, bool fixed)
 {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, bisection_kernel, kBlock, 0) == cudaSuccess
-               ? kOk
-               : kErrCuda;
+    const cudaError_t e =
+        fixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, bisection_fixed_kernel, kBlock, 0)
+              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, bisection_kernel, kBlock, 0);
+    return e == cudaSuccess ? kOk : kErrCuda;
 }
 
 cudaError_t launch_gridding_map(const MapDesc *d_desc, long long total_items, unsigned long long *d_counter, int grid,

@@ -177,9 +177,12 @@ cudaError_t launch_leg_detail(const ReflTable *d_tab, const int8_t *d_vol, const
                               int *status, cudaStream_t st);
 // The reference's iterative-bisection variant (ib_test) over the same work
 // items as launch_absorption; num_cls > 3 also searches bubble boundaries.
+// `fixed`: the fixed-point searches, for volumes with axes of at most
+// kBisectFixedDim voxels; else the FP64 ones.
+constexpr int kBisectFixedDim = 1023;
 cudaError_t launch_bisection(const SampleDesc *d_descs, int n_desc, long long total_items,
-                             unsigned long long *d_counter, int grid, int num_cls, cudaStream_t st);
-int bisection_occupancy(int *blocks_per_sm);
+                             unsigned long long *d_counter, int grid, int num_cls, bool fixed, cudaStream_t st);
+int bisection_occupancy(int *blocks_per_sm, bool fixed);
 // ib_single_gridding for n voxels of one direction (leg 1 of d_dir):
 // d_out[k] = sum_m mu_m (0 + L_m) with the bisection lengths (exp is left to
 // the caller), d_status[k] its status; d_vox_mu = voxel[3], mu[4].
