@@ -1256,6 +1256,7 @@ int plan_view_field(anacor_plan *p, PlanView *v)
     if (plan_ensure_field(p, 2) == kOk) {
         v->field = p->d_field8;
         v->field_stride = (long long)p->dims[0] * p->dims[1] * p->dims[2];
+        v->walls = p->d_walls;
     } else {
         succeed();   // labels outside 0..7: the cooperative march
     }

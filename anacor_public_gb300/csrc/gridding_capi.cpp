@@ -197,6 +197,7 @@ struct anacor_gridding {
     int *d_status = nullptr;
     unsigned long long *d_counter = nullptr;
     MapDesc *d_desc = nullptr;
+    SampleDesc *d_sample = nullptr;
     bool built = false;
     InterpRow *d_rows = nullptr;
     double *d_out = nullptr;
@@ -292,24 +293,65 @@ int run_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int i
     d.sq = pv.sq;
     d.sq_stride = pv.sq_stride;
     d.qtab = pv.qtab;
-    d.field = pv.field;
-    d.field_stride = pv.field_stride;
     cudaError_t e;
     if ((e = cudaMemsetAsync(d_status, 0, sizeof(int), st)) ||
         (e = cudaMemcpyAsync(d_desc, &d, sizeof(d), cudaMemcpyHostToDevice, st)))
         return cuda_err(e);
     const long long items = n_dirs * d.tiles;
-    if ((e = launch_gridding_map(d_desc, items, d_counter, (int)std::max(1ll, std::min<long long>(items, grid)), st,
-                                 pv.field != nullptr)))
+    if ((e = launch_gridding_map(d_desc, items, d_counter, (int)std::max(1ll, std::min<long long>(items, grid)), st)))
         return cuda_err(e);
     // the descriptor is on the stack
     return check_map_status(d_status, st);
 }
 
-int map_grid_size(int sms)
+// The same on the view's octant fields.  Items of 512 voxels: a direction is
+// a few of them, tens of thousands of directions fill the device.
+int run_field_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int is_exp, float *out, long long ld,
+                  SampleDesc *d_sample, unsigned long long *d_counter, int *d_status, int grid, cudaStream_t st)
+{
+    SampleDesc d;
+    std::memset(&d, 0, sizeof(d));
+    d.vol = pv.vol;
+    for (int a = 0; a < 3; a++) {
+        d.dim[a] = pv.dims[a];
+        d.voxel[a] = pv.voxel[a];
+        d.voxelf[a] = (float)pv.voxel[a];
+    }
+    for (int a = 0; a < 4; a++) {
+        d.mu[a] = pv.mu[a];
+        d.muf[a] = (float)pv.mu[a];
+    }
+    d.n_vox = pv.n_vox;
+    d.coords = pv.coords;
+    d.refl = d_dirs;
+    d.n_refl = n_dirs;
+    d.tile = 512;
+    d.tiles = (pv.n_vox + d.tile - 1) / d.tile;
+    d.full_iteration = pv.full_iteration;
+    d.is_exp = is_exp;
+    d.status = d_status;
+    d.sq = pv.sq;
+    d.sq_stride = pv.sq_stride;
+    d.qtab = pv.qtab;
+    d.field = pv.field;
+    d.field_stride = pv.field_stride;
+    d.walls = pv.walls;
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(d_status, 0, sizeof(int), st)) ||
+        (e = cudaMemcpyAsync(d_sample, &d, sizeof(d), cudaMemcpyHostToDevice, st)))
+        return cuda_err(e);
+    const long long items = n_dirs * d.tiles;
+    if ((e = launch_field_map(d_sample, items, d_counter, (int)std::max(1ll, std::min<long long>((items + 7) / 8, grid)),
+                              out, ld, nullptr, st)))
+        return cuda_err(e);
+    // the descriptor is on the stack
+    return check_map_status(d_status, st);
+}
+
+int map_grid_size(int sms, bool field)
 {
     int b = 0;
-    if (gridding_map_occupancy(&b) != kOk || b <= 0)
+    if ((field ? field_map_occupancy(&b) : gridding_map_occupancy(&b)) != kOk || b <= 0)
         b = 1;
     return std::max(1, sms) * b;
 }
@@ -352,11 +394,11 @@ anacor_gridding *anacor_gridding_create(anacor_plan *plan, int n_theta, int n_ph
     g->ta.make(n_theta, 180.0);
     g->pa.make(n_phi, 90.0);
     g->ld = ((long long)g->pv.n_vox + 31) / 32 * 32;
-    g->map_grid = map_grid_size(g->pv.sms);
+    g->map_grid = map_grid_size(g->pv.sms, g->pv.field != nullptr);
     cudaError_t e;
     cudaStream_t st = g->pv.stream;
     if ((e = dalloc(&g->d_map, (size_t)(g->G * std::max(1ll, g->ld)))) || (e = dalloc(&g->d_status, 1)) ||
-        (e = dalloc(&g->d_counter, 1)) || (e = dalloc(&g->d_desc, 1))) {
+        (e = dalloc(&g->d_counter, 1)) || (e = dalloc(&g->d_desc, 1)) || (e = dalloc(&g->d_sample, 1))) {
         cuda_err(e);
         anacor_gridding_destroy(g);
         return nullptr;
@@ -391,6 +433,7 @@ void anacor_gridding_destroy(anacor_gridding *g)
     dfree(g->d_status);
     dfree(g->d_counter);
     dfree(g->d_desc);
+    dfree(g->d_sample);
     dfree(g->d_rows);
     dfree(g->d_out);
     delete g;
@@ -434,8 +477,10 @@ int anacor_gridding_build(anacor_gridding *g, const double *rotated_s1, const do
         dfree(d_dirs);
         return cuda_err(e);
     }
-    const int r = run_map(g->pv, d_dirs, G, g->method == 1, g->pv.mu, g->d_map, nullptr, g->ld, nullptr, g->d_desc,
-                          g->d_counter, g->d_status, g->map_grid, st);
+    const int r = g->pv.field ? run_field_map(g->pv, d_dirs, G, g->method == 1, g->d_map, g->ld, g->d_sample,
+                                              g->d_counter, g->d_status, g->map_grid, st)
+                              : run_map(g->pv, d_dirs, G, g->method == 1, g->pv.mu, g->d_map, nullptr, g->ld, nullptr,
+                                        g->d_desc, g->d_counter, g->d_status, g->map_grid, st);
     dfree(d_dirs);
     if (r)
         return r;

@@ -406,141 +406,6 @@ __device__ __forceinline__ int wall_increments(double q, int c, int h)
     return (int)fminf(floorf(k * 0.9999f), 1.0e9f);
 }
 
-// Distance-field march of one lane over increments 1 .. lim-1 (all clear of
-// the volume's walls, as for the cooperative march).  The field byte of the
-// current increment i gives the label and D, the chessboard distance to the
-// nearest voxel with another label.  Increment i + n lies n voxels away on
-// the step axis and at most ceil(n qmax) + 1 on the other two (two roundings
-// of c + n q), so every increment up to i + nmax(D) with
-//     nmax(D) = min(D - 1, floor((D - 2) / qmax))
-// carries increment i's label: it is accepted without a load, and the march
-// goes on at i + nmax + 1.  Labels, stops, class changes and len_path_2 are
-// therefore exactly those of the per-increment march.
-// One lane's field march over one leg, as a chain of dependent loads.  With
-// a bricked field (kBrick) the chain holds absolute coordinates instead of
-// linear strides (the members of the other layout are never set).
-struct FieldChain {
-    const FaceRule *R;
-    const uint8_t *fld;       // the field this leg marches on (its octant's)
-    const uint8_t *pk;        // linear: fld + the leg's start voxel
-    long long off, Qa, Qb;    // bricked: off of axis a, offb of axis b, with the start coordinates
-    long long offb;
-    uint32_t Ma, Mb, rq;
-    int dS, Sa, Sb;           // linear: strides of the step axis (signed) and the two others
-    int cs, ds;               // bricked: start coordinate and direction on the step axis
-    int k_s, k_a, k_b;        // bricked: brick_term's K of the step axis and the two others
-    int is_s, is_a, is_b;     // bricked: their in-brick strides
-    int i, lim, last, prev, nseg;
-    bool on;
-};
-
-__device__ __forceinline__ int field_nmax(uint32_t d, uint32_t rq)
-{
-    return d < 2u ? 0 : min((int)d - 1, (int)(((d - 2u) * rq) >> 16));
-}
-
-template <bool kBrick>
-__device__ __forceinline__ void chain_init(FieldChain &c, const FaceRule &R, const LegGeom &g, const uint8_t *fld,
-                                           int base, int lim, uint32_t b0, const March &m, const Vol &v)
-{
-    c.R = &R;
-    c.fld = fld;
-    c.Qa = g.Qa;
-    c.Qb = g.Qb;
-    c.Ma = g.Ma;
-    c.Mb = g.Mb;
-    c.rq = R.skip_rq;   // below 2^16 / qmax: the skip never exceeds nmax
-    if (kBrick) {
-        // adding c * 2^32 changes neither the fraction nor the ambiguity test
-        c.off = ((long long)g.ca << 32) + g.off;
-        c.offb = ((long long)g.cb << 32) + g.off;
-        c.cs = g.cs;
-        c.ds = g.ds;
-        const int s = R.count_axis;
-        c.k_s = brick_k(s, v);
-        c.k_a = brick_k(g.ia, v);
-        c.k_b = brick_k(g.ib, v);
-        c.is_s = brick_is(s);
-        c.is_a = brick_is(g.ia);
-        c.is_b = brick_is(g.ib);
-    } else {
-        c.pk = fld + base;
-        c.off = g.off;
-        c.dS = g.ds * g.Ss;
-        c.Sa = g.Sa;
-        c.Sb = g.Sb;
-    }
-    c.lim = lim;
-    c.prev = m.prev;
-    c.nseg = m.nseg;
-    c.i = 1 + field_nmax(b0 >> 3, c.rq);
-    c.last = min(c.i - 1, lim - 1);
-    c.on = c.i < lim;
-}
-
-// field byte of the chain's current increment
-template <bool kBrick>
-__device__ __forceinline__ uint32_t chain_load(const FieldChain &c, int cz, int cy, int cx, const Vol &v)
-{
-    const long long ea = c.off + (long long)c.i * c.Qa;
-    const long long eb = (kBrick ? c.offb : c.off) + (long long)c.i * c.Qb;
-    if (((uint32_t)ea + c.Ma < 2u * c.Ma) | ((uint32_t)eb + c.Mb < 2u * c.Mb))
-        return exact_byte(*c.R, cz, cy, cx, c.i, v, c.fld, kBrick);
-    if (kBrick)
-        return __ldg(c.fld + (brick_term(c.cs + c.i * c.ds, c.k_s, c.is_s) + brick_term((int)(ea >> 32), c.k_a, c.is_a) +
-                              brick_term((int)(eb >> 32), c.k_b, c.is_b)));
-    return __ldg(c.pk + (c.i * c.dS + (int)(ea >> 32) * c.Sa + (int)(eb >> 32) * c.Sb));
-}
-
-// the stop / class-change test of the current increment, then the skip
-__device__ __forceinline__ void chain_step(FieldChain &c, uint32_t b, uint16_t *seg, bool &stopped)
-{
-    const int lab = (int)(b & 7u);
-    if (lab == 0) {
-        stopped = true;
-        c.last = c.i - 1;
-        c.on = false;
-        return;
-    }
-    if (lab != c.prev) {
-        if (lab <= 4) {
-            if (c.nseg < kMaxSegments)
-                seg[c.nseg * kBlock] = (uint16_t)((lab << 13) | c.i);
-            c.nseg++;
-        }
-        c.prev = lab;
-    }
-    const int n = field_nmax(b >> 3, c.rq);
-    c.last = min(c.i + n, c.lim - 1);
-    c.i += n + 1;
-    c.on = c.i < c.lim;
-}
-
-__device__ __forceinline__ void chain_done(const FieldChain &c, March &m)
-{
-    m.last_i = c.last;
-    m.prev = c.prev;
-    m.nseg = c.nseg;
-}
-
-// The march of one lane on its field.  dlast: |displacement| of the last
-// accepted increment on the two non-step axes (a | b << 16), when its
-// fixed-point position is not near a rounding boundary; else -1.
-template <bool kBrick>
-__device__ __forceinline__ void field_march(const FaceRule &R, const LegGeom &g, int cz, int cy, int cx,
-                                            const Vol &v, const uint8_t *fld, int base, int lim, uint32_t b0,
-                                            March &m, bool &stopped, uint16_t *seg, int &dlast)
-{
-    FieldChain c;
-    chain_init<kBrick>(c, R, g, fld, base, lim, b0, m, v);
-    while (c.on)
-        chain_step(c, chain_load<kBrick>(c, cz, cy, cx, v), seg, stopped);
-    chain_done(c, m);
-    const long long ea = g.off + (long long)c.last * g.Qa, eb = g.off + (long long)c.last * g.Qb;
-    const bool amb = ((uint32_t)ea + c.Ma < 2u * c.Ma) | ((uint32_t)eb + c.Mb < 2u * c.Mb);
-    dlast = amb ? -1 : (abs((int)(ea >> 32)) | abs((int)(eb >> 32)) << 16);
-}
-
 // fl(fl(d * v_axis)^2), from the sample's table when it has one
 __device__ __forceinline__ double sq_len(const double *sq, int stride, int axis, int d, double vox)
 {
@@ -649,13 +514,12 @@ struct LegState {
     March m;
     int face, lim, base;
     bool need, coop, stopped, live;
-    uint32_t b0;   // field byte of increment 0 (field march)
-    int dlast;     // field march: the last point's displacement (see field_march), else -1
+    int dlast;     // stopped at vacuum: |displacement| of the last accepted increment on the two non-step
+                   // axes (a | b << 16) unless its position is near a rounding boundary, else -1
 };
 
-// cube_face and the march set-up of one leg (warp-synchronous).  With kField
-// the lane's field march runs here too.
-template <bool kDetail, bool kField, bool kBrick>
+// cube_face and the march set-up of one leg (warp-synchronous).
+template <bool kDetail>
 __device__ __forceinline__ void leg_setup(const LegHead &h, const FaceRule *rules, int cz, int cy, int cx, bool valid,
                                           const Vol &v, int full, uint16_t *seg, LegResult &out, LegState &S)
 {
@@ -684,8 +548,6 @@ __device__ __forceinline__ void leg_setup(const LegHead &h, const FaceRule *rule
     // few values cross the cooperative loop; the geometry is recomputed after.
     bool coop = false, stopped = false, live = false;
     int lim = 0, base = 0;
-    uint32_t b0 = 0;
-    int dlast = -1;
     if (need) {
         const FaceRule &R = rules[face - 1];
         LegGeom g;
@@ -722,26 +584,12 @@ __device__ __forceinline__ void leg_setup(const LegHead &h, const FaceRule *rule
         if (coop) {
             base = g.cs * g.Ss + g.ca * g.Sa + g.cb * g.Sb;
             seg[0] = (uint16_t)(3 << 13);
-            if (kField) {
-                // per lane, no warp synchronisation: the field march
-                const uint8_t *fld = v.field + R.octant * v.field_stride;
-                b0 = __ldg(fld + (kBrick ? brick_offset(cz, cy, cx, v) : base));
-                if ((b0 & 7u) == 0) {
-                    stopped = true;
-                } else {
-                    m.prev = (int)(b0 & 7u);
-                    live = lim > 1;
-                    if (live)
-                        field_march<kBrick>(R, g, cz, cy, cx, v, fld, base, lim, b0, m, stopped, seg, dlast);
-                }
+            const int lab0 = __ldg(v.p + base);
+            if (lab0 == 0) {
+                stopped = true;
             } else {
-                const int lab0 = __ldg(v.p + base);
-                if (lab0 == 0) {
-                    stopped = true;
-                } else {
-                    m.prev = lab0;
-                    live = lim > 1;
-                }
+                m.prev = lab0;
+                live = lim > 1;
             }
         }
     }
@@ -754,11 +602,10 @@ __device__ __forceinline__ void leg_setup(const LegHead &h, const FaceRule *rule
     S.coop = coop;
     S.stopped = stopped;
     S.live = live;
-    S.b0 = b0;
-    S.dlast = dlast;
+    S.dlast = -1;
 }
 
-// The warp-cooperative march of the legs set up by leg_setup<.., false>.
+// The warp-cooperative march of the legs set up by leg_setup.
 __device__ __forceinline__ void leg_coop(const FaceRule *rules, int cz, int cy, int cx, const Vol &v, uint16_t *seg,
                                          LegState &S)
 {
@@ -873,8 +720,7 @@ __device__ __forceinline__ void leg_coop(const FaceRule *rules, int cz, int cy, 
     S.m = m;
     S.stopped = stopped;
     if (coop && stopped) {
-        // the last point of a leg that stopped at vacuum, as the field march
-        // gives it (see field_march's dlast)
+        // the last point of a leg that stopped at vacuum (LegState::dlast)
         const FaceRule &R = rules[face - 1];
         const int s = R.count_axis, a = s == 0 ? 1 : 0, b = s == 2 ? 1 : 2;
         const long long off = R.use_round ? 0x80000000ll : 0ll;
@@ -901,7 +747,7 @@ __device__ __forceinline__ void leg_finish(const FaceRule *rules, int cz, int cy
         return;
 
     if (!kDetail && coop && stopped && S.dlast >= 0 && m.nseg <= kMaxSegments) {
-        // a field march that stopped at vacuum: the last point is known
+        // a leg that stopped at vacuum: the last point is known
         // (step axis: last_i increments; the others: dlast), so the lengths
         // need neither the geometry nor the point
         const int len = m.last_i + 1;
@@ -1026,16 +872,15 @@ __device__ __forceinline__ void leg_finish(const FaceRule *rules, int cz, int cy
 // kF32: the per-class lengths in FP32 (for A_h, which needs 1e-6; the march
 // itself, and hence the visited voxels, segments and len_path_2, is the same);
 // otherwise FP64 in the reference's order (bit-exact lengths).
-template <bool kDetail, bool kF32 = false, bool kField = false, bool kBrick = false>
+template <bool kDetail, bool kF32 = false>
 __device__ __forceinline__ void trace_leg(const LegHead &h, const FaceRule *rules, int cz, int cy, int cx,
                                           bool valid, const Vol &v, int full, const double *voxel,
                                           const double *sq, int sq_stride, const double *qtab, uint16_t *seg,
                                           LegResult &out, const float *voxelf = nullptr)
 {
     LegState S;
-    leg_setup<kDetail, kField, kBrick>(h, rules, cz, cy, cx, valid, v, full, seg, out, S);
-    if (!kField)
-        leg_coop(rules, cz, cy, cx, v, seg, S);
+    leg_setup<kDetail>(h, rules, cz, cy, cx, valid, v, full, seg, out, S);
+    leg_coop(rules, cz, cy, cx, v, seg, S);
     leg_finish<kDetail, kF32>(rules, cz, cy, cx, v, full, voxel, sq, sq_stride, qtab, seg, S, out, voxelf);
 }
 
@@ -1231,45 +1076,54 @@ struct SlowLeg {
 // 0..lim-1 accepted); 2 the stop at increment i (only the lengths are left).
 enum SlowFrom { kFromStart = 0, kFromLimit = 1, kFromStop = 2 };
 
-// The rest of a leg that the field march does not finish by itself.
-__device__ __noinline__ SlowLeg leg_slow(const WarpTab &W, int leg, int axis, const short4 *voxel, uint16_t *seg,
-                                         int from, int i, int nseg, int prev, int lim)
+// The rest of a leg that the field march does not finish by itself: FP32
+// lengths (out.Lf), or FP64 ones in the reference's order (out.L).
+template <bool kF32>
+__device__ __forceinline__ void leg_rest(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int from,
+                                         int axis, int i, int nseg, int prev, int lim, LegResult &out)
 {
     const short4 cv = __ldg(voxel);
-    const int cz = cv.x, cy = cv.y, cx = cv.z;
     const SampleDesc &D = *W.desc;
     const ReflTable *T = W.refl;
     const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
-    LegResult out;
-    out.Lf[0] = out.Lf[1] = out.Lf[2] = out.Lf[3] = 0.0f;
+    for (int k = 0; k < 4; k++) {
+        out.L[k] = 0.0;
+        out.Lf[k] = 0.0f;
+    }
     out.len = 1;
     out.status = kOk;
     const FaceRule *rules = T->rule[leg];
-    const int face = from == kFromStart ? exit_face(T->head[leg], cz, cy, cx, v) : W.rule[leg][axis].face;
+    const int face = from == kFromStart ? exit_face(T->head[leg], cv.x, cv.y, cv.z, v) : W.rule[leg][axis].face;
     if (face == 0)
         out.status = kErrNoFace;
     else if (rules[face - 1].status)
         out.status = rules[face - 1].status;
-    if (out.status == kOk) {
-        LegState S;
-        S.m.last_i = (from == kFromStop ? i : lim) - 1;
-        S.m.nseg = nseg;
-        S.m.prev = prev;
-        S.m.vac = 0;
-        S.face = face;
-        S.lim = lim;
-        S.base = 0;
-        S.need = true;
-        S.coop = from != kFromStart;
-        S.stopped = from == kFromStop;
-        S.live = false;
-        S.b0 = 0;
-        S.dlast = -1;
-        leg_finish<false, true>(rules, cz, cy, cx, v, D.full_iteration, D.voxel, D.sq, D.sq_stride, D.qtab, seg, S,
-                                out, D.voxelf);
-    } else {
-        atomicOr(D.status, 1 << out.status);
-    }
+    if (out.status)
+        return;
+    LegState S;
+    S.m.last_i = (from == kFromStop ? i : lim) - 1;
+    S.m.nseg = nseg;
+    S.m.prev = prev;
+    S.m.vac = 0;
+    S.face = face;
+    S.lim = lim;
+    S.base = 0;
+    S.need = true;
+    S.coop = from != kFromStart;
+    S.stopped = from == kFromStop;
+    S.live = false;
+    S.dlast = -1;
+    leg_finish<false, kF32>(rules, cv.x, cv.y, cv.z, v, D.full_iteration, D.voxel, D.sq, D.sq_stride, D.qtab, seg, S,
+                            out, D.voxelf);
+}
+
+__device__ __noinline__ SlowLeg leg_slow(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int from,
+                                         int axis, int i, int nseg, int prev, int lim)
+{
+    LegResult out;
+    leg_rest<true>(W, leg, voxel, seg, from, axis, i, nseg, prev, lim, out);
+    if (out.status)
+        atomicOr(W.desc->status, 1 << out.status);
     SlowLeg r;
     r.L = make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
     r.len = out.len;
@@ -1323,8 +1177,12 @@ __device__ __noinline__ int leg_limit(const FaceRule *R, int cz, int cy, int cx,
     return 0;
 }
 
-// One leg of one voxel (not warp-synchronous): exit face, march, FP32 lengths
-// (liquor, loop, crystal, bubble).
+// Exit face and march of one leg of one voxel (not warp-synchronous).
+// Returns `none()` for a leg without length (it starts in vacuum or stops at
+// increment 1), `done(i, nseg, d0, d1, d2)` for one that stopped at vacuum at
+// increment i with its class changes in the list and its last point's
+// |displacement| (z, y, x), and `slow(from, axis, i, nseg, prev, lim)` for one
+// that is left to the slow path.
 //
 // The inner loop is kept to one load, one exit branch and predicated
 // bookkeeping (about 30 instructions) and holds no call: what lives across
@@ -1332,14 +1190,14 @@ __device__ __noinline__ int leg_limit(const FaceRule *R, int cz, int cy, int cx,
 // off by at most one voxel in the inner loop, still inside the volume (free
 // legs keep a voxel of room, the others their wall limit); the outer loop
 // takes that increment with the exact position.
-template <bool kBrick>
-__device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int &len)
+template <bool kBrick, class None, class Done, class Slow>
+__device__ __forceinline__ auto field_march(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, None none,
+                                            Done done, Slow slow)
 {
     // the coordinates are loaded per leg (and again where they are rarely
     // needed) rather than kept across the march
     const short4 cv = __ldg(voxel);
     const int cz = cv.x, cy = cv.y, cx = cv.z;
-    len = 1;
     // ---- exit face: the smallest of the three distances n_a / |e_a| (n_a
     // exact, the estimates within 2^-22), when the next one is clearly larger
     // and the voxel is not on a min plane (a zero distance wins there)
@@ -1364,7 +1222,7 @@ __device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const sho
                             : (cz * W.dy + cy) * W.dx + cx);
         uint32_t b = __ldg(start);
         if ((b & 7u) == 0u)
-            return make_float4(0.0f, 0.0f, 0.0f, 0.0f);   // starts in vacuum
+            return none();   // starts in vacuum
         const uint32_t qa_lo = R.qa_lo, qa_hi = R.qa_hi, qb_lo = R.qb_lo, qb_hi = R.qb_hi;
         const unsigned long long off_a = R.off_a, off_b = R.off_b;
         const int dS = R.dS, Sa = R.Sa, Sb = R.Sb, rq = R.rq;
@@ -1408,33 +1266,73 @@ __device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const sho
             from = kFromStop;
             break;
         }
-        if (from == kFromStop) {
-            len = i;
-            if (i == 1)
-                return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (nseg <= kMaxSegments) {
-                // the last point's displacement: last_i on the step axis
-                const int last_i = i - 1;
-                uint32_t fa, fb;
-                int da = fixed_at(last_i, qa_lo, qa_hi, off_a, fa);
-                int db = fixed_at(last_i, qb_lo, qb_hi, off_b, fb);
-                if (min(fa, fb) < 2u * kFieldMargin)
-                    exact_displacement(W, leg, R, axis, voxel, last_i, da, db);
-                const int d0 = axis == 0 ? last_i : abs(da);
-                const int d1 = axis == 1 ? last_i : (axis == 0 ? abs(da) : abs(db));
-                const int d2 = axis == 2 ? last_i : abs(db);
-                LegResult out;
-                out.Lf[0] = out.Lf[1] = out.Lf[2] = out.Lf[3] = 0.0f;
-                seg[0] = (uint16_t)(3 << 13);
-                lengths_f32(d0, d1, d2, len, nseg, seg, nullptr, W.voxel, out);
-                return make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
-            }
+        if (from == kFromStop && i == 1)
+            return none();
+        if (from == kFromStop && nseg <= kMaxSegments) {
+            // the last point's displacement: last_i on the step axis
+            const int last_i = i - 1;
+            uint32_t fa, fb;
+            int da = fixed_at(last_i, qa_lo, qa_hi, off_a, fa);
+            int db = fixed_at(last_i, qb_lo, qb_hi, off_b, fb);
+            if (min(fa, fb) < 2u * kFieldMargin)
+                exact_displacement(W, leg, R, axis, voxel, last_i, da, db);
+            const int d0 = axis == 0 ? last_i : abs(da);
+            const int d1 = axis == 1 ? last_i : (axis == 0 ? abs(da) : abs(db));
+            const int d2 = axis == 2 ? last_i : abs(db);
+            seg[0] = (uint16_t)(3 << 13);
+            return done(i, nseg, d0, d1, d2);
         }
     }
     seg[0] = (uint16_t)(3 << 13);
-    const SlowLeg r = leg_slow(W, leg, axis, voxel, seg, from, i, nseg, prev, lim);
-    len = r.len;
-    return r.L;
+    return slow(from, axis, i, nseg, prev, lim);
+}
+
+// One leg of one voxel: FP32 lengths (liquor, loop, crystal, bubble).
+template <bool kBrick>
+__device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int &len)
+{
+    len = 1;
+    return field_march<kBrick>(
+        W, leg, voxel, seg, [] { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); },
+        [&](int i, int nseg, int d0, int d1, int d2) {
+            len = i;
+            LegResult out;
+            out.Lf[0] = out.Lf[1] = out.Lf[2] = out.Lf[3] = 0.0f;
+            lengths_f32(d0, d1, d2, i, nseg, seg, nullptr, W.voxel, out);
+            return make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
+        },
+        [&](int from, int axis, int i, int nseg, int prev, int lim) {
+            const SlowLeg r = leg_slow(W, leg, voxel, seg, from, axis, i, nseg, prev, lim);
+            len = r.len;
+            return r.L;
+        });
+}
+
+// A map value (cal_rate with a zero incident leg) of a leg
+// in the reference's FP64 operations: legs the march leaves, and values too
+// close to a rounding boundary of float.
+__device__ __noinline__ float map_slow(const WarpTab &W, const short4 *voxel, uint16_t *seg, int from, int axis, int i,
+                                       int nseg, int prev, int lim, int d0, int d1, int d2)
+{
+    const SampleDesc &D = *W.desc;
+    LegResult out;
+    if (d0 >= 0) {   // marched to its stop: the lengths alone
+        out.L[0] = out.L[1] = out.L[2] = out.L[3] = 0.0;
+        out.status = kOk;
+        lengths_f64(d0, d1, d2, i, nseg, seg, D.voxel, D.sq, D.sq_stride, D.qtab, out);
+    } else {
+        leg_rest<false>(W, 1, voxel, seg, from, axis, i, nseg, prev, lim, out);
+    }
+    if (out.status) {
+        atomicOr(D.status, 1 << out.status);
+        return __int_as_float(0x7fffffff);
+    }
+    const double t0 = __dmul_rn(D.mu[0], out.L[0]);
+    const double t1 = __dmul_rn(D.mu[1], out.L[1]);
+    const double t2 = __dmul_rn(D.mu[2], out.L[2]);
+    const double t3 = __dmul_rn(D.mu[3], out.L[3]);
+    const double ex = __dadd_rn(__dadd_rn(__dadd_rn(t0, t1), t2), t3);
+    return (float)(D.is_exp ? exp(-ex) : ex);
 }
 
 __device__ __forceinline__ int find_sample(const SampleDesc *d, int n, long long item)
@@ -2229,7 +2127,6 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
 
 // Absorption map: work item = (grid direction, tile of voxels); the
 // diffracted leg of every voxel, one output per (direction, voxel).
-template <bool kField>
 __global__ void __launch_bounds__(kBlock, 2) gridding_map_kernel(const MapDesc *__restrict__ dp, long long total_items,
                                                                  unsigned long long *__restrict__ work_counter)
 {
@@ -2240,7 +2137,7 @@ __global__ void __launch_bounds__(kBlock, 2) gridding_map_kernel(const MapDesc *
     if (!block_shape_ok(D.status))
         return;
     const int tid = threadIdx.x;
-    const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2], D.field, D.field_stride};
+    const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
     for (;;) {
         if (tid == 0)
             item_s = (long long)atomicAdd(work_counter, 1ull);
@@ -2266,7 +2163,7 @@ __global__ void __launch_bounds__(kBlock, 2) gridding_map_kernel(const MapDesc *
             const bool valid = vi < v1;
             const short4 cv = valid ? __ldg(D.coords + vi) : make_short4(0, 0, 0, 0);
             LegResult a;
-            trace_leg<false, false, kField>(tab.head[1], tab.rule[1], cv.x, cv.y, cv.z, valid, v, D.full_iteration,
+            trace_leg<false>(tab.head[1], tab.rule[1], cv.x, cv.y, cv.z, valid, v, D.full_iteration,
                                             D.voxel, D.sq, D.sq_stride, D.qtab, seg + tid, a);
             if (!valid)
                 continue;
@@ -2292,6 +2189,92 @@ __global__ void __launch_bounds__(kBlock, 2) gridding_map_kernel(const MapDesc *
         if (bad)
             atomicOr(D.status, 1 << bad);
         __syncthreads();   // the table and item_s are rewritten next
+    }
+}
+
+// The absorption map on the octant fields, bit for bit the FP64 values rounded
+// to float: the reference's sum mu_m L_m = total / (len - 1) * sum mu_m span_m
+// is formed on pairs of floats (within 2^-43 of it), and where that leaves the
+// rounding to float open (a few in 10^5) map_slow evaluates the FP64
+// expressions.  On GB300 those bound the kernel before (a square root, the
+// quotients and the sums of every leg on an FP64 pipe of two lanes a cycle).
+// 64,800 directions x 1,657 voxels of a 512x512x400 volume: 14.8 -> 5.5 ms.
+__global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *__restrict__ dp, long long total_items,
+                                                              unsigned long long *__restrict__ work_counter,
+                                                              float *__restrict__ out, long long ld,
+                                                              const int *__restrict__ col)
+{
+    __shared__ WarpTab tabs[kWarps];
+    __shared__ uint16_t seg[kSegRows * kBlock];
+    __shared__ FloatPair consts[7];   // squared voxel edges (z, y, x), mu
+    const SampleDesc &D = *dp;
+    if (!block_shape_ok(D.status))
+        return;
+    const int tid = threadIdx.x, lane = tid & 31;
+    WarpTab &W = tabs[tid >> 5];
+    if (tid < 3)
+        consts[tid] = pair_of(__dmul_rn(D.voxel[tid], D.voxel[tid]));
+    else if (tid < 7)
+        consts[tid] = pair_of(D.mu[tid - 3]);
+    __syncthreads();
+    // the error bound is relative to the sum: no cancellation between terms
+    const bool positive = D.mu[0] >= 0.0 && D.mu[1] >= 0.0 && D.mu[2] >= 0.0 && D.mu[3] >= 0.0;
+    for (;;) {
+        unsigned long long it = 0;
+        if (lane == 0)
+            it = atomicAdd(work_counter, 1ull);
+        const long long item = (long long)__shfl_sync(kAll, it, 0);
+        if (item >= total_items)
+            break;
+        const long long d = item / D.tiles;
+        const int t = (int)(item - d * D.tiles);
+        __syncwarp();   // the previous item's reads of the table are done
+        fill_warp_tab(W, D.refl + d, D, lane);
+        __syncwarp();
+        const int n = min(D.tile, D.n_vox - t * D.tile);
+        const short4 *coords = D.coords + (long long)t * D.tile;
+        for (int vi = lane; vi < n; vi += 32) {
+            const float val = field_march<false>(
+                W, 1, coords + vi, seg + tid, [&] { return W.is_exp ? 1.0f : 0.0f; },
+                [&](int i, int nseg, int d0, int d1, int d2) {
+                    const FloatPair tot = pair_sqrt(
+                        pair_add(pair_add(pair_mul(consts[0], (float)(d0 * d0)), pair_mul(consts[1], (float)(d1 * d1))),
+                                 pair_mul(consts[2], (float)(d2 * d2))));
+                    FloatPair sum = {0.0f, 0.0f};
+                    int cur = 3 << 13;
+                    for (int j = 1; j <= nseg; j++) {
+                        const int nxt = j < nseg ? (int)seg[j * kBlock + tid] : i;
+                        const int cls = cur >> 13, span = (nxt & 0x1fff) - (cur & 0x1fff);
+                        if (cls >= 1)
+                            sum = pair_add(sum, pair_mul(consts[2 + cls], (float)span));
+                        cur = nxt;
+                    }
+                    const FloatPair p = pair_mul(tot, sum);
+                    const float den = (float)(i - 1);
+                    const float q = __fdiv_rn(p.h, den);
+                    const FloatPair r = pair_norm(q, __fdividef(__fadd_rn(__fmaf_rn(-q, den, p.h), p.l), den));
+                    float v;
+                    bool sure;
+                    if (W.is_exp) {
+                        const double ex = (double)r.h + (double)r.l, y = exp(-ex);
+                        const double err = y * (fabs(ex) * 0x1p-40 + 0x1p-50);
+                        v = (float)y;
+                        sure = (float)(y + err) == v && (float)(y - err) == v;
+                    } else {
+                        // the float nearest to r, unless r is within 2^-40 of a tie
+                        const float err = fabsf(r.h) * 0x1p-40f;
+                        v = r.h;
+                        sure = __fadd_rn(r.h, r.l + err) == r.h && __fadd_rn(r.h, r.l - err) == r.h && r.h > 0x1p-80f;
+                    }
+                    return positive && sure ? v
+                                            : map_slow(W, coords + vi, seg + tid, kFromStop, 0, i, nseg, 0, 0, d0, d1, d2);
+                },
+                [&](int from, int axis, int i, int nseg, int prev, int lim) {
+                    return map_slow(W, coords + vi, seg + tid, from, axis, i, nseg, prev, lim, -1, 0, 0);
+                });
+            const int k = t * D.tile + vi;
+            out[d * ld + (col ? __ldg(col + k) : k)] = val;
+        }
     }
 }
 
@@ -2499,28 +2482,42 @@ int bisection_occupancy(int *blocks_per_sm, bool fixed)
     return e == cudaSuccess ? kOk : kErrCuda;
 }
 
-cudaError_t launch_gridding_map(const MapDesc *d_desc, long long total_items, unsigned long long *d_counter, int grid,
-                                cudaStream_t st, bool field)
+cudaError_t launch_field_map(const SampleDesc *d_desc, long long total_items, unsigned long long *d_counter, int grid,
+                             float *out, long long ld, const int *col, cudaStream_t st)
 {
     if (total_items <= 0)
         return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess)
         return e;
-    if (field)
-        gridding_map_kernel<true><<<grid, kBlock, 0, st>>>(d_desc, total_items, d_counter);
-    else
-        gridding_map_kernel<false><<<grid, kBlock, 0, st>>>(d_desc, total_items, d_counter);
+    field_map_kernel<<<grid, kBlock, 0, st>>>(d_desc, total_items, d_counter, out, ld, col);
     return cudaGetLastError();
 }
 
-int gridding_map_occupancy(int *blocks_per_sm, bool field)
+int field_map_occupancy(int *blocks_per_sm)
 {
-    const cudaError_t e = field ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, gridding_map_kernel<true>,
-                                                                                kBlock, 0)
-                                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, gridding_map_kernel<false>,
-                                                                                kBlock, 0);
-    return e == cudaSuccess ? kOk : kErrCuda;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, field_map_kernel, kBlock, 0) == cudaSuccess
+               ? kOk
+               : kErrCuda;
+}
+
+cudaError_t launch_gridding_map(const MapDesc *d_desc, long long total_items, unsigned long long *d_counter, int grid,
+                                cudaStream_t st)
+{
+    if (total_items <= 0)
+        return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess)
+        return e;
+    gridding_map_kernel<<<grid, kBlock, 0, st>>>(d_desc, total_items, d_counter);
+    return cudaGetLastError();
+}
+
+int gridding_map_occupancy(int *blocks_per_sm)
+{
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, gridding_map_kernel, kBlock, 0) == cudaSuccess
+               ? kOk
+               : kErrCuda;
 }
 
 int absorption_block_threads() { return kBlock; }

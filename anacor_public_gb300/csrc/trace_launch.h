@@ -77,8 +77,6 @@ struct MapDesc {
     const double *sq;
     int sq_stride;
     const double *qtab;
-    const uint8_t *field;   // optional: octant fields (launch_octant_fields) for the field march
-    long long field_stride;
 };
 
 // Device-resident sample of a plan, for the other entry points that march it.
@@ -98,6 +96,7 @@ struct PlanView {
     int sms;
     const uint8_t *field;     // the plan's octant fields, when built (plan_view_field)
     long long field_stride;
+    const int *walls;         // room between the labels and the walls, built with the fields
 };
 int plan_view(const anacor_plan *p, PlanView *out);
 // plan_view with the plan's octant fields, built if needed (left out, with
@@ -191,8 +190,14 @@ cudaError_t launch_ib_direction(const ReflTable *d_dir, const int8_t *d_vol, con
                                 cudaStream_t st);
 // Persistent launch over n_dirs * tiles work items of the map.
 cudaError_t launch_gridding_map(const MapDesc *d_desc, long long total_items, unsigned long long *d_counter, int grid,
-                                cudaStream_t st, bool field = false);
-int gridding_map_occupancy(int *blocks_per_sm, bool field = false);
+                                cudaStream_t st);
+int gridding_map_occupancy(int *blocks_per_sm);
+// The same map values as floats on the octant fields of one sample whose
+// reflection tables are the directions (leg 1): out[d * ld + k], or column
+// col[k].  One-sample work items as launch_absorption.
+cudaError_t launch_field_map(const SampleDesc *d_desc, long long total_items, unsigned long long *d_counter, int grid,
+                             float *out, long long ld, const int *col, cudaStream_t st);
+int field_map_occupancy(int *blocks_per_sm);
 // Lookup of one reflection in an absorption map: for each leg (0 incident,
 // 1 diffracted) the map rows (grid directions) and weights of the value, as
 // the reference's interpolation reads it
