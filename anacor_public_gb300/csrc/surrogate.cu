@@ -25,6 +25,7 @@
 
 #include "anacor_gb300.h"
 #include "anacor_internal.h"
+#include "gelu.cuh"
 #include "umma_gemm.cuh"
 
 namespace anacor {
@@ -76,18 +77,6 @@ struct GemmArgs {
     long long ldaux, sAux;
     int *err;
 };
-
-__device__ __forceinline__ float gelu(float x)
-{
-    return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
-}
-
-__device__ __forceinline__ float gelu_grad(float x)
-{
-    const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-    const float pdf = 0.3989422804014327f * expf(-0.5f * x * x);
-    return cdf + x * pdf;
-}
 
 // Stage one K-chunk of 64 of A (128 rows) and B (BN rows) into the canonical
 // no-swizzle K-major tile layout with 16-byte cp.async copies.
@@ -179,6 +168,7 @@ __global__ void __launch_bounds__(umma::kThreads, 1) gemm_kernel(GemmArgs g)
         const long long zo = ks > 1 ? z : e;
         for (int c0 = 0; c0 < BN; c0 += 16) {
             float v[16];
+            uint32_t t[8];   // 16 BF16
             umma::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
             const int n = n0 + c0;
             if (g.mode == kEpiStoreF32) {
@@ -199,29 +189,26 @@ __global__ void __launch_bounds__(umma::kThreads, 1) gemm_kernel(GemmArgs g)
                     for (int i = 0; i < 16; i += 4)
                         *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    v[i] = gelu(v[i]);
+                gelu::values_bf16<8>(v, t);
             } else {   // kEpiGeluBwd
                 const float *h = g.aux + e * g.sAux + (long long)row * g.ldaux + n;
 #pragma unroll
                 for (int i = 0; i < 16; i++)
-                    v[i] *= gelu_grad(h[i]);
+                    v[i] *= gelu::grad(h[i]);
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    t[i] = gelu::bf16x2(v[2 * i], v[2 * i + 1]);
             }
             if (g.ob) {
-                __align__(16) bf16 t[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    t[i] = __float2bfloat16_rn(v[i]);
                 bf16 *o = g.ob + e * g.sOb + (long long)row * g.ldob + n;
-                *reinterpret_cast<uint4 *>(o) = *reinterpret_cast<const uint4 *>(t);
-                *reinterpret_cast<uint4 *>(o + 8) = *reinterpret_cast<const uint4 *>(t + 8);
+                *reinterpret_cast<uint4 *>(o) = make_uint4(t[0], t[1], t[2], t[3]);
+                *reinterpret_cast<uint4 *>(o + 8) = make_uint4(t[4], t[5], t[6], t[7]);
             }
             if (g.ot) {
-                bf16 *o = g.ot + e * g.sOt + row;
+                uint16_t *o = reinterpret_cast<uint16_t *>(g.ot + e * g.sOt + row);
 #pragma unroll
                 for (int i = 0; i < 16; i++)
-                    o[(long long)(n + i) * g.ldot] = __float2bfloat16_rn(v[i]);
+                    o[(long long)(n + i) * g.ldot] = (uint16_t)(t[i >> 1] >> (16 * (i & 1)));
             }
         }
     }
@@ -428,7 +415,7 @@ __global__ void head_kernel(const bf16 *__restrict__ A4, const float *__restrict
     __align__(16) bf16 t[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) {
-        t[q] = __float2bfloat16_rn(g * P[kOffW5 + lane * 8 + q] * gelu_grad(h[q]));
+        t[q] = __float2bfloat16_rn(g * P[kOffW5 + lane * 8 + q] * gelu::grad(h[q]));
         dHT[((long long)e * kWidth + lane * 8 + q) * rows + r] = t[q];
     }
     reinterpret_cast<uint4 *>(dH + base * kWidth)[lane] = *reinterpret_cast<const uint4 *>(t);
@@ -982,26 +969,26 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
                                     v);
 #pragma unroll
                     for (int q = 0; q < 16; q++)
-                        v[q] = gelu(v[q] + bias[c0 + q]);
-                    __align__(16) __nv_bfloat162 t2[8];
-#pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        t2[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-                    const bf16 *t = reinterpret_cast<const bf16 *>(t2);
+                        v[q] += bias[c0 + q];
+                    uint32_t t2[8];
+                    gelu::values_bf16<8>(v, t2);
                     if (l < kDepth - 1) {
                         uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
                         const int k = c0 % umma::kBK;
-                        *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) = *reinterpret_cast<const uint4 *>(t);
+                        *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) =
+                            make_uint4(t2[0], t2[1], t2[2], t2[3]);
                         *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) =
-                            *reinterpret_cast<const uint4 *>(t + 8);
+                            make_uint4(t2[4], t2[5], t2[6], t2[7]);
                     } else {
                         // the head's per-8-column partial sums, as head_kernel's lanes form them
 #pragma unroll
                         for (int g = 0; g < 2; g++) {
                             float acc = 0.0f;
 #pragma unroll
-                            for (int q = 0; q < 8; q++)
-                                acc += __bfloat162float(t[8 * g + q]) * w5[c0 + 8 * g + q];
+                            for (int q = 0; q < 8; q++) {
+                                const uint32_t w = t2[4 * g + (q >> 1)];
+                                acc += __uint_as_float(q & 1 ? w & 0xffff0000u : w << 16) * w5[c0 + 8 * g + q];
+                            }
                             gs[rl * kGStride + (c0 + 8 * g) / 8] = acc;
                         }
                     }
@@ -1090,6 +1077,26 @@ __global__ void wait_guard_kernel(unsigned limit, int *err)
     __syncthreads();
     if (threadIdx.x < 32)
         umma::tmem_dealloc(tslot, 32);
+}
+
+// every float through the layers' BF16 GELU: counts[0] the values whose bits
+// differ from the reference evaluation's, counts[1] those the approximation
+// left to it
+__global__ void gelu_check_kernel(unsigned long long *counts)
+{
+    unsigned long long wrong = 0, open = 0;
+    for (unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; t < (1ull << 31);
+         t += (unsigned long long)gridDim.x * blockDim.x) {
+        const float v[2] = {__uint_as_float((uint32_t)(2 * t)), __uint_as_float((uint32_t)(2 * t + 1))};
+        uint32_t r, o;
+        gelu::values_bf16<1>(v, &r);
+        gelu::value_bf16x2(v[0], v[1], o);
+        const uint32_t d = r ^ gelu::bf16x2(gelu::value(v[0]), gelu::value(v[1]));
+        wrong += ((d & 0xffffu) != 0) + ((d >> 16) != 0);
+        open += ((o & 0xffffu) != 0) + ((o >> 16) != 0);
+    }
+    atomicAdd(&counts[0], wrong);
+    atomicAdd(&counts[1], open);
 }
 
 std::once_flag g_infer_once[64];
@@ -1881,6 +1888,25 @@ int anacor_wait_guard_check(unsigned iterations, int32_t *status)
     if (e)
         return cuda_fail(e);
     *status = h;
+    return report_status(kOk, "");
+}
+
+int anacor_gelu_check(uint64_t *wrong, uint64_t *open)
+{
+    if (!wrong || !open)
+        return report_status(kErrArgs, "bad arguments");
+    unsigned long long *d = nullptr, h[2] = {0, 0};
+    cudaError_t e;
+    if (!(e = dalloc(&d, 2)) && !(e = cudaMemset(d, 0, sizeof(h)))) {
+        gelu_check_kernel<<<1024, 256>>>(d);
+        if (!(e = cudaGetLastError()) && !(e = cudaDeviceSynchronize()))
+            e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+    }
+    dfree(d);
+    if (e)
+        return cuda_fail(e);
+    *wrong = h[0];
+    *open = h[1];
     return report_status(kOk, "");
 }
 

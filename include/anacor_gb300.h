@@ -406,6 +406,10 @@ int anacor_surrogate_load(anacor_surrogate *s, const char *path);
  * A [batch][M][K], B [batch][N][K] rounded to BF16, FP32 accumulation, the K
  * range split into ksplit slices whose partial products are summed in order */
 int anacor_tc_gemm_check(const float *A, const float *B, int M, int N, int K, int batch, int ksplit, float *C);
+/* The layers' BF16 GELU over all 2^32 floats: *wrong the values whose bits
+ * differ from the reference evaluation's, *open those the approximation leaves
+ * to it. */
+int anacor_gelu_check(uint64_t *wrong, uint64_t *open);
 /* The error path of the tensor-core kernels' bounded mbarrier waits: one CTA
  * allocates tensor memory, waits at most `iterations` polls for a phase that
  * nothing completes, records the error, releases the tensor memory and
