@@ -4,12 +4,15 @@
 // instructions a value, which bound the inference kernel: tensor pipe 12 %,
 // issue 59 %).  What the layers keep is the value rounded to BF16, so a
 // cheaper approximation whose error interval rounds to one BF16 number gives
-// the same bits; where the two ends differ (about one value in a thousand of
+// the same bits; where the two ends differ (about four values in 10,000 of
 // normally distributed ones) the reference decides.  The approximation is
-//   Phi(x) = 1/2 + s (1/2 - Q),  s = sign of x,  Q = erfc(|x| / sqrt 2) / 2,
-//   Q = 2^-P(|x|),  P a degree-8 polynomial with P(0) = 1 (a weighted minimax
-// fit of -log2 Q by Lawson's iteration, error of Q below 1e-8), evaluated two
-// values at a time with packed FP32 multiply-adds.
+//   Phi(x) = 1 / (1 + 2^-G(x)),  G(x) = log2(Phi(x) / Phi(-x)) = x W(x^2),
+// W a degree-6 polynomial (a minimax fit weighted by Phi's sensitivity, by
+// Lawson's iteration: Phi within 3e-8; its leading coefficient is positive, so
+// the ends need no clamp), evaluated two values at a time with packed FP32
+// multiply-adds.  (Phi from erfc(|x|) = 2^-P(|x|) with the sign put back took a
+// degree-8 polynomial and four bit operations a value more: 3.60 ms for a
+// million rows x 4 members.)
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -82,23 +85,28 @@ __device__ __forceinline__ uint32_t bf16x2(float a, float b)
     return r;
 }
 
+// 1 / x of a positive float, within one ulp
+__device__ __forceinline__ float rcp(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Phi(x) of two values
 __device__ __forceinline__ F2 phi(F2 x)
 {
-    const F2 a = x & 0x7fffffff7fffffffull;
-    F2 p = fma2(a, f2(-2.83490704e-06f, -2.83490704e-06f), f2(3.93776281e-05f, 3.93776281e-05f));
-    p = fma2(a, p, f2(-0.000186179954f, -0.000186179954f));
-    p = fma2(a, p, f2(-0.000136937015f, -0.000136937015f));
-    p = fma2(a, p, f2(0.00706342096f, 0.00706342096f));
-    p = fma2(a, p, f2(-0.0524961799f, -0.0524961799f));
-    p = fma2(a, p, f2(-0.45920819f, -0.45920819f));
-    p = fma2(a, p, f2(-1.15110517f, -1.15110517f));
-    p = fma2(a, p, f2(-1.0f, -1.0f));
+    const F2 y = mul2(x, x);
+    F2 p = fma2(y, f2(-5.06723685e-09f, -5.06723685e-09f), f2(3.8163131e-07f, 3.8163131e-07f));
+    p = fma2(y, p, f2(-1.14398335e-05f, -1.14398335e-05f));
+    p = fma2(y, p, f2(0.00015957994f, 0.00015957994f));
+    p = fma2(y, p, f2(9.40492246e-05f, 9.40492246e-05f));
+    p = fma2(y, p, f2(-0.104835123f, -0.104835123f));
+    p = fma2(y, p, f2(-2.30220938f, -2.30220938f));
     float p0, p1;
-    split(p, p0, p1);
-    const F2 h = add2(f2(0.5f, 0.5f), f2(-ex2(p0), -ex2(p1)));
-    const F2 s = (x & 0x8000000080000000ull) | 0x3f8000003f800000ull;
-    return fma2(s, h, f2(0.5f, 0.5f));
+    split(mul2(x, p), p0, p1);
+    split(add2(f2(ex2(p0), ex2(p1)), f2(1.0f, 1.0f)), p0, p1);
+    return f2(rcp(p0), rcp(p1));
 }
 
 // An interval around phi(x) that holds the reference's (1 + erff) / 2 and
@@ -113,19 +121,17 @@ __device__ __forceinline__ void widen(F2 u, F2 &lo, F2 &hi)
     hi = fma2(u, f2(kMore, kMore), f2(kAbs, kAbs));
 }
 
-// BF16 of gelu at two values (a in the lower half); `open` is nonzero in the
-// half whose rounding the approximation leaves open.
-__device__ __forceinline__ uint32_t value_bf16x2(float a, float b, uint32_t &open)
+// BF16 of gelu at two values (the first in the lower half) from the two ends
+// of the interval; they differ in a half whose rounding is left open
+__device__ __forceinline__ uint32_t value_bf16x2(F2 x, uint32_t &other)
 {
-    const F2 x = f2(a, b);
     F2 lo, hi;
     widen(phi(x), lo, hi);
     float l0, l1, h0, h1;
     split(mul2(x, lo), l0, l1);
     split(mul2(x, hi), h0, h1);
-    const uint32_t r = bf16x2(l0, l1);
-    open = r ^ bf16x2(h0, h1);
-    return r;
+    other = bf16x2(h0, h1);
+    return bf16x2(l0, l1);
 }
 
 // the halves left open, from the reference evaluation
@@ -138,21 +144,24 @@ __device__ __noinline__ uint32_t value_decide(float a, float b, uint32_t r, uint
     return r;
 }
 
-// BF16 of gelu at 2 * n values, bit for bit the reference's
+// BF16 of gelu at the 2 * n values v + bias, bit for bit the reference's
 template <int n>
-__device__ __forceinline__ void values_bf16(const float *v, uint32_t *r)
+__device__ __forceinline__ void values_bf16(float *v, const float *bias, uint32_t *r)
 {
-    uint32_t open[n], any = 0u;
+    uint32_t other[n], any = 0u;   // the roundings of the intervals' other ends
 #pragma unroll
     for (int j = 0; j < n; j++) {
-        r[j] = value_bf16x2(v[2 * j], v[2 * j + 1], open[j]);
-        any |= open[j];
+        const F2 x = bias ? add2(f2(v[2 * j], v[2 * j + 1]), f2(bias[2 * j], bias[2 * j + 1]))
+                          : f2(v[2 * j], v[2 * j + 1]);
+        split(x, v[2 * j], v[2 * j + 1]);
+        r[j] = value_bf16x2(x, other[j]);
+        any |= r[j] ^ other[j];
     }
     if (any) {
 #pragma unroll
         for (int j = 0; j < n; j++)
-            if (open[j])
-                r[j] = value_decide(v[2 * j], v[2 * j + 1], r[j], open[j]);
+            if (r[j] != other[j])
+                r[j] = value_decide(v[2 * j], v[2 * j + 1], r[j], r[j] ^ other[j]);
     }
 }
 

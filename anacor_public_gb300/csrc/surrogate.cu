@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(umma::kThreads, 1) gemm_kernel(GemmArgs g)
                     for (int i = 0; i < 16; i += 4)
                         *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
-                gelu::values_bf16<8>(v, t);
+                gelu::values_bf16<8>(v, nullptr, t);
             } else {   // kEpiGeluBwd
                 const float *h = g.aux + e * g.sAux + (long long)row * g.ldaux + n;
 #pragma unroll
@@ -602,44 +602,59 @@ __global__ void audit_kernel(const float *__restrict__ spread, long long n, uint
 // one persistent kernel: the tile's Fourier features and each layer's
 // activations stay in shared memory, the accumulators in tensor memory, and
 // only the weights stream in (from L2: 1.7 MB for four members), as 16 KiB
-// K-chunks copied by the bulk-copy engine (cp.async.bulk) into a 4-stage ring
-// kept three chunks ahead of the MMAs.
+// K-chunks copied by the bulk-copy engine (cp.async.bulk) into a 4-stage ring.
 //
 // Two members are in flight at a time, on two "streams" with their own
-// 256-column TMEM accumulator and 128 x 256 activation tile: while the twelve
-// epilogue warps apply bias and GELU to one member's layer (the expensive
-// part: an erf per element), the control warp issues the other member's MMAs
-// and weight copies.  The streams hand over through mbarriers: acc_full[s]
-// (the layer's MMAs are done), act_ready[s] (its epilogue has read the
-// accumulator and written the next operand), x0_ready (the tile's features).
+// 256-column TMEM accumulator and 128 x 256 activation tile: while the sixteen
+// epilogue warps apply bias and GELU to one member's layer, the MMA warp issues
+// the other member's MMAs (it never waits for one) and a copy warp keeps the
+// weight ring full.  The streams hand over through mbarriers: acc_full[s] (the
+// layer's MMAs are done), act_ready[s] (its epilogue has read the accumulator
+// and written the next operand), x0_ready (a tile's features, which are
+// computed while the tile before it is still in its last layers).  An epilogue
+// warp owns 32 rows x 64 columns of every layer and loads the next 16 columns
+// from tensor memory while it works on the last; warps meet only around the
+// head's sums, in groups of four.  (Eight warps for each stream instead: 10 %
+// slower, a stream's MMAs leave the other's eight too little to fill the SM.)
+//
+// What bounds it is the epilogue: alone it takes 2.9 of the 3.2 ms for a
+// million rows x 4 members (18 instructions a value, issue slots at 61 %, FMA
+// pipe at 52 %); the MMAs alone with their hand-overs take 1.7 ms, the weight
+// copies alone 1.3 ms (13.3 GB from L2).  Before the packed GELU, the copy
+// warp of its own and the features ahead of time it took 5.95 ms.
+//
 // The arithmetic is the layered path's: the same MMAs in the same K order,
-// the same epilogue expressions and the head's and ensemble's summation
-// orders, so the outputs are the same numbers without the per-layer round
-// trips through HBM.
+// the same epilogue values and the head's and ensemble's summation orders, so
+// the outputs are the same numbers without the per-layer round trips through
+// HBM.
+//
+// A call whose tiles leave more than half of the SMs idle runs each tile on a
+// cluster of two, four or eight CTAs that share its members; their outputs
+// meet in the first CTA's shared memory.
 
 constexpr int kWChunkK = 32;                                          // K per weight chunk
 constexpr int kChunkBytes = kWidth * kWChunkK * 2;                    // 256 rows x 32 BF16 = 16 KiB
 constexpr int kChunksPerMember = (kFeat + (kDepth - 1) * kWidth) / kWChunkK;   // 2 + 3 * 8 = 26
 constexpr int kInferStages = 4;
-constexpr int kEpiWarps = 12;                                         // three per TMEM lane quarter
+constexpr int kEpiWarps = 16;                                         // four per TMEM lane quarter
 constexpr int kEpiThreads = 32 * kEpiWarps;
-constexpr int kInferThreads = kEpiThreads + 32;                       // + the control warp
+constexpr int kInferThreads = kEpiThreads + 64;                       // + the MMA and the copy warp
 constexpr int kTileRows = umma::kBM;                                  // 128
 constexpr int kActChunk = kTileRows * umma::kBK * 2;                 // 128 rows x 64 BF16 = 16 KiB
 constexpr int kActBytes = (kWidth / umma::kBK) * kActChunk;          // 64 KiB
-constexpr int kMemberConsts = kDepth * kWidth + kWidth + 2;           // biases, w5, b5, pad
-constexpr int kConstBytes = ((kMemberConsts * 4 + 15) / 16) * 16;
-constexpr int kGStride = 33;                                          // head partials per row (32 + pad)
 constexpr int kInferMaxMembers = 8;
 constexpr int kOffInferAct = kInferStages * kChunkBytes;             // two activation tiles
 constexpr int kOffInferX0 = kOffInferAct + 2 * kActBytes;
-constexpr int kOffInferC = kOffInferX0 + kActChunk;                  // two members' constants
-constexpr int kOffInferY = kOffInferC + 2 * kConstBytes;
+constexpr int kOffInferY = kOffInferX0 + kActChunk;
 constexpr int kInferSmem = kOffInferY + kInferMaxMembers * kTileRows * 4;
-// the head's partial sums live in the stream's activation tile, which the
-// last layer's MMAs have finished reading when the head writes them
-static_assert(kTileRows * kGStride * 4 <= kActBytes, "head partials fit the activation tile");
+// The head's partial sums (32 per row) live in the stream's activation tile,
+// which the last layer's MMAs have finished reading when the head writes them:
+// each TMEM lane quarter's in the bytes of its own 32 rows of the first
+// K-chunk, so that the only warps that write there next are the quarter's.
+constexpr int kQuarterBytes = 32 * 32 * 4;
+static_assert(kQuarterBytes == 4 * 1024, "a quarter's rows of a K-chunk");
 static_assert(kInferSmem + 512 <= 227 * 1024, "fused inference shared memory");
+static_assert(kEpiWarps / 4 * 64 == kWidth, "an epilogue warp owns 64 columns");
 
 // byte offset of element (r, k) of a rows x 32 K-major weight chunk in the
 // canonical no-swizzle layout (8-row groups 512 bytes apart)
@@ -648,10 +663,10 @@ __host__ __device__ constexpr uint32_t wchunk_off(int r, int k)
     return (uint32_t)(((r >> 3) * (kWChunkK / 8) + (k >> 3)) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
-// The work of one tile as jobs (stream s, member e, layer l), in the order
-// both the control warp and the epilogue warps take them: members in pairs
-// (2p on stream 0, 2p + 1 on stream 1), layer by layer, alternating streams;
-// an odd last member alone on stream 0.
+// The work of one tile on E members as jobs (stream s, member e, layer l), in
+// the order that the copy, MMA and epilogue warps take them: members
+// in pairs (2p on stream 0, 2p + 1 on stream 1), layer by layer, alternating
+// streams; an odd last member alone on stream 0.
 __host__ __device__ inline void job_of(int j, int E, int &s, int &e, int &l)
 {
     const int pairs = E / 2;
@@ -667,32 +682,26 @@ __host__ __device__ inline void job_of(int j, int E, int &s, int &e, int &l)
     l = j - pairs * 2 * kDepth;
 }
 
+// the last job that reads the tile's features
+__host__ __device__ inline int last_feature_job(int E)
+{
+    return E % 2 ? E / 2 * 2 * kDepth : (E / 2 - 1) * 2 * kDepth + 1;
+}
+
 __host__ __device__ constexpr int job_chunks(int l) { return in_dim(l) / kWChunkK; }
 
-// Weight chunk c of the image (the control warp's consumption order):
-// member e, layer l, K-chunk kq
-__host__ __device__ inline void chunk_of(int c, int E, int &e, int &l, int &kq)
+// index of K-chunk kq of layer l of member e in the weight image
+__host__ __device__ constexpr int chunk_index(int e, int l, int kq)
 {
-    int j = 0;
-    int s = 0;
-    for (;; j++) {
-        job_of(j, E, s, e, l);
-        const int n = job_chunks(l);
-        if (c < n) {
-            kq = c;
-            return;
-        }
-        c -= n;
-    }
+    return e * kChunksPerMember + (l == 0 ? 0 : job_chunks(0) + (l - 1) * job_chunks(1)) + kq;
 }
 
 struct WeightPtrs {
     const bf16 *w[kDepth];
 };
 
-// The weight image: for every member its 26 K-chunks of W_l [256][K], each in
-// the canonical no-swizzle K-major layout of a 256 x 32 tile, in the order the
-// fused kernel consumes them.
+// The weight image: for every member its 26 K-chunks of W_l [256][K], layer by
+// layer, each in the canonical no-swizzle K-major layout of a 256 x 32 tile.
 __global__ void weight_image_kernel(WeightPtrs W, int E, uint8_t *__restrict__ img)
 {
     constexpr int kPieces = kChunkBytes / 16;   // 16-byte pieces (8 BF16 along K) per chunk
@@ -701,8 +710,9 @@ __global__ void weight_image_kernel(WeightPtrs W, int E, uint8_t *__restrict__ i
          t += (long long)gridDim.x * blockDim.x) {
         const int c = (int)(t / kPieces);
         const int p = (int)(t - (long long)c * kPieces);
-        int e, l, kq;
-        chunk_of(c, E, e, l, kq);
+        const int e = c / kChunksPerMember, m = c - e * kChunksPerMember;
+        const int l = m < job_chunks(0) ? 0 : 1 + (m - job_chunks(0)) / job_chunks(1);
+        const int kq = m - (l == 0 ? 0 : job_chunks(0) + (l - 1) * job_chunks(1));
         const int K = in_dim(l);
         const int r = p >> 2, kc = p & 3;
         const bf16 *src = W.w[l] + (long long)e * kWidth * K + (long long)r * K + kq * kWChunkK + kc * 8;
@@ -753,17 +763,10 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, vo
     return false;
 }
 
-// barrier over the epilogue warps (named barrier 1) that also ANDs a
-// predicate across them: every epilogue thread takes the same branch after it
-__device__ __forceinline__ bool epi_sync_and(bool ok)
+// barrier over the four epilogue warps of a TMEM lane quarter
+__device__ __forceinline__ void quarter_sync(int quarter)
 {
-    uint32_t r;
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
-        : "=r"(r)
-        : "r"((uint32_t)ok), "r"(kEpiThreads)
-        : "memory");
-    return r != 0;
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory");
 }
 
 struct InferArgs {
@@ -773,20 +776,47 @@ struct InferArgs {
     const uint8_t *wimg;
     const float *params;
     int E;
+    int share;   // CTAs of a cluster that share a tile's members (1: no cluster)
     float mu, sd;
     float *mean, *spread, *members;
     long long ldm;
     int *err;
 };
 
-// member constant i (biases of the four layers, w5, b5) from the FP32 masters
-__device__ __forceinline__ float member_const(const float *P, int i)
+// Fourier features of a tile (features_kernel's expressions), BF16 into the
+// layer-0 operand tile; rows past n are zeros.  Thread t: row t / 4, eight
+// frequencies.
+__device__ __forceinline__ void tile_features(const InferArgs &a, long long row0, int t, uint8_t *X0s)
 {
-    if (i < kDepth * kWidth)
-        return P[off_b(i / kWidth) + (i % kWidth)];
-    if (i < kDepth * kWidth + kWidth)
-        return P[kOffW5 + (i - kDepth * kWidth)];
-    return i == kDepth * kWidth + kWidth ? P[kOffB5] : 0.0f;
+    const int r = t >> 2, h = t & 3;
+    const long long i = row0 + r;
+    float sv[8], cv[8];
+#pragma unroll
+    for (int jj = 0; jj < 8; jj++) {
+        sv[jj] = 0.0f;
+        cv[jj] = 0.0f;
+    }
+    if (i < a.n) {
+        const float *x = a.x7 + 7 * i;
+#pragma unroll
+        for (int jj = 0; jj < 8; jj++) {
+            const int j = 8 * h + jj;
+            float p = 0.0f;
+#pragma unroll
+            for (int q = 0; q < kIn; q++)
+                p += __ldg(a.Bf + j * kIn + q) * __ldg(x + q);
+            sincospif(2.0f * p, &sv[jj], &cv[jj]);
+        }
+    }
+    uint32_t u[4], w[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        u[q] = gelu::bf16x2(sv[2 * q], sv[2 * q + 1]);
+        w[q] = gelu::bf16x2(cv[2 * q], cv[2 * q + 1]);
+    }
+    *reinterpret_cast<uint4 *>(X0s + umma::tile_off(r, 8 * h)) = make_uint4(u[0], u[1], u[2], u[3]);
+    *reinterpret_cast<uint4 *>(X0s + umma::tile_off(r, kFeat / 2 + 8 * h)) = make_uint4(w[0], w[1], w[2], w[3]);
+    umma::fence_async_smem();
 }
 
 __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
@@ -800,9 +830,12 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
     float *ys = reinterpret_cast<float *>(smem + kOffInferY);
     volatile int *abort = &s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = a.share > 1 ? (int)(blockIdx.x % a.share) : 0;
+    const long long first = blockIdx.x / a.share, step = gridDim.x / a.share;   // tiles of this CTA (cluster)
     const long long tiles = (a.n + kTileRows - 1) / kTileRows;
-    const long long my_tiles = tiles > (long long)blockIdx.x ? (tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    const int jobs = kDepth * a.E;
+    const long long my_tiles = tiles > first ? (tiles - 1 - first) / step + 1 : 0;
+    const int e0 = rank * a.E / a.share, E = (rank + 1) * a.E / a.share - e0;    // this CTA's members
+    const int jobs = kDepth * E;
 
     if (tid == 0) {
         for (int s = 0; s < kInferStages; s++) {
@@ -811,9 +844,9 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
         }
         for (int s = 0; s < 2; s++) {
             umma::mbar_init(&acc_full[s], 1);
-            umma::mbar_init(&act_ready[s], kEpiThreads);
+            umma::mbar_init(&act_ready[s], kEpiWarps);
         }
-        umma::mbar_init(&x0_ready, kEpiThreads);
+        umma::mbar_init(&x0_ready, kEpiWarps);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -823,33 +856,50 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
     __syncthreads();
     umma::tc_fence_after();
     const uint32_t tmem = tslot;
+    if (a.share > 1) {   // the first CTA has started before its shared memory is written to
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
 
-    if (warp == kEpiWarps) {
-        // ---- control warp: lane 0 issues the weight copies and the MMAs
+    if (warp == kEpiWarps + 1) {
+        // ---- copy warp: lane 0 streams the weight chunks in the order the
+        // MMAs take them, each into its stage once the MMAs that read the
+        // stage's previous chunk are done
+        if (lane == 0) {
+            const long long total = my_tiles * E * kChunksPerMember;
+            int j = 0, kq = 0;
+            long long q = 0;
+            for (; q < total; q++) {
+                const int st = (int)(q % kInferStages);
+                if (q >= kInferStages && !wait_or_abort(&empty[st], (uint32_t)((q / kInferStages - 1) & 1), abort))
+                    break;
+                int s, e, l;
+                job_of(j, E, s, e, l);
+                mbar_expect_tx(&full[st], kChunkBytes);
+                bulk_g2s(Ws + st * kChunkBytes, a.wimg + (long long)chunk_index(e0 + e, l, kq) * kChunkBytes,
+                         kChunkBytes, &full[st]);
+                if (++kq == job_chunks(l)) {
+                    kq = 0;
+                    j = j + 1 == jobs ? 0 : j + 1;
+                }
+            }
+            // copies still in flight complete before the CTA's shared memory
+            // goes away (bounded: a failed copy does not hold the exit)
+            for (long long p = q > kInferStages ? q - kInferStages : 0; p < q; p++)
+                wait_or_abort(&full[p % kInferStages], (uint32_t)((p / kInferStages) & 1), abort);
+        }
+        __syncwarp();
+    } else if (warp == kEpiWarps) {
+        // ---- MMA warp: lane 0 issues the MMAs and never waits for one
         if (lane == 0) {
             constexpr uint32_t idesc = umma::idesc_bf16_f32(kWidth);
-            const long long per_tile = (long long)a.E * kChunksPerMember;
-            const long long total = my_tiles * per_tile;
-            long long q_issue = 0, q_use = 0;
+            long long q = 0;
             uint32_t kjob[2] = {0u, 0u};
             bool ok = true;
-            // load weight chunk q into stage q % kInferStages once the MMAs that
-            // read that stage's previous chunk are done
-            auto issue = [&](long long q) -> bool {
-                const int st = (int)(q % kInferStages);
-                if (q >= kInferStages &&
-                    !wait_or_abort(&empty[st], (uint32_t)((q / kInferStages - 1) & 1), abort))
-                    return false;
-                mbar_expect_tx(&full[st], kChunkBytes);
-                bulk_g2s(Ws + st * kChunkBytes, a.wimg + (q % per_tile) * kChunkBytes, kChunkBytes, &full[st]);
-                return true;
-            };
-            for (; q_issue < total && q_issue < kInferStages - 1 && ok; q_issue++)
-                ok = issue(q_issue);
             for (long long ti = 0; ti < my_tiles && ok; ti++) {
                 for (int j = 0; j < jobs && ok; j++) {
                     int s, e, l;
-                    job_of(j, a.E, s, e, l);
+                    job_of(j, E, s, e, l);
                     // the operand: the tile's features (layer 0) or the stream's
                     // previous epilogue, which also freed its accumulator
                     if (j == 0)
@@ -861,9 +911,9 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
                     umma::tc_fence_after();
                     const uint8_t *A = l == 0 ? X0s : smem + kOffInferAct + s * kActBytes;
                     const int nk = job_chunks(l);
-                    for (int kc = 0; kc < nk; kc++, q_use++) {
-                        const int st = (int)(q_use % kInferStages);
-                        if (!wait_or_abort(&full[st], (uint32_t)((q_use / kInferStages) & 1), abort)) {
+                    for (int kc = 0; kc < nk; kc++, q++) {
+                        const int st = (int)(q % kInferStages);
+                        if (!wait_or_abort(&full[st], (uint32_t)((q / kInferStages) & 1), abort)) {
                             ok = false;
                             break;
                         }
@@ -877,154 +927,143 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
                                            umma::smem_desc(b0, 128, 512), idesc, (kc > 0 || kk > 0) ? 1u : 0u);
                         }
                         umma::mma_commit(&empty[st]);
-                        if (q_issue < total) {
-                            if (!issue(q_issue)) {
-                                ok = false;
-                                q_use++;
-                                break;
-                            }
-                            q_issue++;
-                        }
                     }
                     umma::mma_commit(&acc_full[s]);
                     kjob[s]++;
                 }
             }
-            // copies still in flight complete before the CTA's shared memory
-            // goes away (bounded: a failed copy does not hold the exit)
-            for (long long q = q_use; q < q_issue; q++)
-                wait_or_abort(&full[q % kInferStages], (uint32_t)((q / kInferStages) & 1), abort);
             if (!ok)
                 *abort = 1;
         }
+        __syncwarp();
     } else {
-        // ---- epilogue warps: features, bias + GELU per layer, head, ensemble
-        const int rl = 32 * (warp & 3) + lane;          // this thread's row of the tile (TMEM lane)
-        // its accumulator columns: warps 0-3 take 0..95, 4-7 96..175, 8-11 176..255
-        const int cb = warp < 4 ? 0 : (warp < 8 ? 96 : 176);
-        const int ce = warp < 4 ? 96 : (warp < 8 ? 176 : kWidth);
+        // ---- epilogue warps: features, bias + GELU per layer, head, ensemble.
+        // A warp whose wait runs out goes on through the loops without waiting
+        // or writing, so that the others still meet it at the barriers.
+        const int quarter = warp & 3;                   // TMEM lanes 32 * quarter ..
+        const int rl = 32 * quarter + lane;             // this thread's row of the tile
+        const int cb = 64 * (warp >> 2);                // its accumulator columns cb .. cb + 63
+        const uint32_t lane_base = (uint32_t)(32 * quarter) << 16;
+        const int jx0 = last_feature_job(E);
         uint32_t ejob[2] = {0u, 0u};
         bool ok = true;
-        for (long long ti = 0; ti < my_tiles && ok; ti++) {
-            const long long row0 = (blockIdx.x + ti * gridDim.x) * kTileRows;
-            if (tid < 2 * kTileRows) {
-                // Fourier features of the tile (features_kernel's expressions),
-                // BF16 into the layer-0 operand tile; rows past n are zeros
-                const int r = tid >> 1, h = tid & 1;
-                const long long i = row0 + r;
-                float sv[16], cv[16];
-#pragma unroll
-                for (int jj = 0; jj < 16; jj++) {
-                    sv[jj] = 0.0f;
-                    cv[jj] = 0.0f;
-                }
-                if (i < a.n) {
-                    const float *x = a.x7 + 7 * i;
-#pragma unroll
-                    for (int jj = 0; jj < 16; jj++) {
-                        const int j = 16 * h + jj;
-                        float p = 0.0f;
-#pragma unroll
-                        for (int q = 0; q < kIn; q++)
-                            p += a.Bf[j * kIn + q] * x[q];
-                        sincospif(2.0f * p, &sv[jj], &cv[jj]);
-                    }
-                }
-#pragma unroll
-                for (int part = 0; part < 4; part++) {   // features 16h.. (sin) and 32+16h.. (cos)
-                    const float *src = part < 2 ? sv + 8 * part : cv + 8 * (part - 2);
-                    const int f0 = (part < 2 ? 0 : kFeat / 2) + 16 * h + 8 * (part & 1);
-                    __align__(16) bf16 t[8];
-#pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        t[q] = __float2bfloat16_rn(src[q]);
-                    *reinterpret_cast<uint4 *>(X0s + umma::tile_off(r, f0)) = *reinterpret_cast<const uint4 *>(t);
-                }
-            }
-            umma::fence_async_smem();
-            mbar_arrive(&x0_ready);
+        if (my_tiles > 0) {
+            tile_features(a, first * kTileRows, tid, X0s);
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&x0_ready);
+        }
+        for (long long ti = 0; ti < my_tiles; ti++) {
+            const long long row0 = (first + ti * step) * kTileRows;
             for (int j = 0; j < jobs; j++) {
                 int s, e, l;
-                job_of(j, a.E, s, e, l);
-                float *cst = reinterpret_cast<float *>(smem + kOffInferC + s * kConstBytes);
+                job_of(j, E, s, e, l);
                 uint8_t *Act = smem + kOffInferAct + s * kActBytes;
-                if (l == 0) {
-                    // this member's constants (the stream's previous member is done with them)
-                    for (int i = tid; i < kMemberConsts; i += kEpiThreads)
-                        cst[i] = member_const(a.params + (long long)e * kParams, i);
-                }
-                ok = wait_or_abort(&acc_full[s], ejob[s] & 1u, abort) && ok;
+                float *gs = reinterpret_cast<float *>(Act + quarter * kQuarterBytes) + 32 * lane;
+                const float *P = a.params + (long long)(e0 + e) * kParams;
+                const float *bias = P + off_b(l) + cb;
+                const uint32_t acc = tmem + (uint32_t)(s * kWidth + cb) + lane_base;
+                ok = ok && wait_or_abort(&acc_full[s], ejob[s] & 1u, abort);
                 ejob[s]++;
-                ok = epi_sync_and(ok);   // also publishes the constants
-                if (!ok)
-                    break;
-                umma::tc_fence_after();
-                const float *bias = cst + l * kWidth;
-                const float *w5 = cst + kDepth * kWidth;
-                float *gs = reinterpret_cast<float *>(Act);
-                for (int c0 = cb; c0 < ce; c0 += 16) {
-                    float v[16];
-                    umma::tmem_ld16(tmem + (uint32_t)(s * kWidth) + ((uint32_t)(32 * (warp & 3)) << 16) +
-                                        (uint32_t)c0,
-                                    v);
+                ok = __all_sync(0xffffffffu, ok);
+                if (l == 0)
+                    quarter_sync(quarter);   // the stream's previous head sums have been read
+                if (ok) {
+                    umma::tc_fence_after();
+                    float v[2][16];
+                    umma::tmem_ld16_start(acc, v[0]);
 #pragma unroll
-                    for (int q = 0; q < 16; q++)
-                        v[q] += bias[c0 + q];
-                    uint32_t t2[8];
-                    gelu::values_bf16<8>(v, t2);
-                    if (l < kDepth - 1) {
-                        uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
-                        const int k = c0 % umma::kBK;
-                        *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) =
-                            make_uint4(t2[0], t2[1], t2[2], t2[3]);
-                        *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) =
-                            make_uint4(t2[4], t2[5], t2[6], t2[7]);
-                    } else {
-                        // the head's per-8-column partial sums, as head_kernel's lanes form them
+                    for (int g = 0; g < 4; g++) {
+                        float *x = v[g & 1];
+                        float bs[16];
 #pragma unroll
-                        for (int g = 0; g < 2; g++) {
-                            float acc = 0.0f;
+                        for (int q = 0; q < 4; q++)
+                            *reinterpret_cast<float4 *>(bs + 4 * q) =
+                                __ldg(reinterpret_cast<const float4 *>(bias + 16 * g) + q);
+                        umma::tmem_ld16_wait(x);
+                        if (g < 3)
+                            umma::tmem_ld16_start(acc + 16 * (g + 1), v[(g + 1) & 1]);
+                        uint32_t t[8];
+                        gelu::values_bf16<8>(x, bs, t);
+                        const int c0 = cb + 16 * g;
+                        if (l < kDepth - 1) {
+                            uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
+                            const int k = c0 % umma::kBK;
+                            *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) =
+                                make_uint4(t[0], t[1], t[2], t[3]);
+                            *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) =
+                                make_uint4(t[4], t[5], t[6], t[7]);
+                        } else {
+                            // the head's per-8-column partial sums, as head_kernel's lanes form them
+                            const float4 *w5 = reinterpret_cast<const float4 *>(P + kOffW5 + c0);
 #pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                const uint32_t w = t2[4 * g + (q >> 1)];
-                                acc += __uint_as_float(q & 1 ? w & 0xffff0000u : w << 16) * w5[c0 + 8 * g + q];
+                            for (int h = 0; h < 2; h++) {
+                                const float4 wa = __ldg(w5 + 2 * h), wb = __ldg(w5 + 2 * h + 1);
+                                const float ws[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+                                float sum = 0.0f;
+#pragma unroll
+                                for (int q = 0; q < 8; q++) {
+                                    const uint32_t w = t[4 * h + (q >> 1)];
+                                    sum += __uint_as_float(q & 1 ? w & 0xffff0000u : w << 16) * ws[q];
+                                }
+                                gs[(c0 / 8 + h) ^ lane] = sum;
                             }
-                            gs[rl * kGStride + (c0 + 8 * g) / 8] = acc;
                         }
                     }
+                    umma::tc_fence_before();
+                    umma::fence_async_smem();
                 }
-                umma::tc_fence_before();
-                umma::fence_async_smem();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(&act_ready[s]);
                 if (l == kDepth - 1) {
-                    epi_sync_and(true);
-                    if (tid < kTileRows) {
+                    quarter_sync(quarter);
+                    if (ok && warp < 4) {
                         // head_kernel's shuffle tree over the 32 partial sums (lane 0's order)
                         float g[32];
 #pragma unroll
                         for (int jj = 0; jj < 32; jj++)
-                            g[jj] = gs[tid * kGStride + jj];
+                            g[jj] = gs[jj ^ lane];
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
                             for (int jj = 0; jj < o; jj++)
                                 g[jj] = g[jj] + g[jj + o];
-                        ys[e * kTileRows + tid] = g[0] + cst[kDepth * kWidth + kWidth];
+                        const float y = g[0] + __ldg(P + kOffB5);
+                        if (rank == 0) {
+                            ys[(e0 + e) * kTileRows + rl] = y;
+                        } else {   // into the first CTA's shared memory
+                            uint32_t dst;
+                            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;"
+                                         : "=r"(dst)
+                                         : "r"(umma::smem_u32(ys + (e0 + e) * kTileRows + rl)));
+                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(y) : "memory");
+                        }
                     }
-                    epi_sync_and(true);
                 }
-                mbar_arrive(&act_ready[s]);
+                if (j == jx0 && ti + 1 < my_tiles) {
+                    // the tile's features have been read: the next tile's
+                    if (ok)
+                        tile_features(a, row0 + step * kTileRows, tid, X0s);
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(&x0_ready);
+                }
             }
-            if (!ok)
-                break;
-            if (tid < kTileRows && row0 + tid < a.n) {
+            __syncwarp();
+            if (a.share > 1) {   // one tile per cluster: the other CTAs' outputs arrive
+                asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            }
+            if (ok && rank == 0 && warp < 4 && row0 + rl < a.n) {
                 // ensemble_kernel's statistics (this thread's own row of ys)
-                const long long i = row0 + tid;
+                const long long i = row0 + rl;
                 float av[kInferMaxMembers];
                 float sum = 0.0f;
 #pragma unroll
                 for (int e = 0; e < kInferMaxMembers; e++) {
                     if (e < a.E) {
-                        const float la = a.mu + a.sd * ys[e * kTileRows + tid];
+                        const float la = a.mu + a.sd * ys[e * kTileRows + rl];
                         if (a.members)
                             a.members[e * a.ldm + i] = la;
                         av[e] = expf(la);
@@ -1041,6 +1080,10 @@ __global__ void __launch_bounds__(kInferThreads, 1) infer_kernel(InferArgs a)
                 a.spread[i] = sqrtf(var / a.E) / m;
             }
         }
+    }
+    if (a.share > 1 && warp >= kEpiWarps) {   // the MMA and copy warps' part of the cluster barrier
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     umma::tc_fence_before();
     __syncthreads();
@@ -1087,11 +1130,13 @@ __global__ void gelu_check_kernel(unsigned long long *counts)
     unsigned long long wrong = 0, open = 0;
     for (unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; t < (1ull << 31);
          t += (unsigned long long)gridDim.x * blockDim.x) {
-        const float v[2] = {__uint_as_float((uint32_t)(2 * t)), __uint_as_float((uint32_t)(2 * t + 1))};
+        float v[2] = {__uint_as_float((uint32_t)(2 * t)), __uint_as_float((uint32_t)(2 * t + 1))};
+        const uint32_t want = gelu::bf16x2(gelu::value(v[0]), gelu::value(v[1]));
         uint32_t r, o;
-        gelu::values_bf16<1>(v, &r);
-        gelu::value_bf16x2(v[0], v[1], o);
-        const uint32_t d = r ^ gelu::bf16x2(gelu::value(v[0]), gelu::value(v[1]));
+        const uint32_t p = gelu::value_bf16x2(gelu::f2(v[0], v[1]), o);
+        o ^= p;
+        gelu::values_bf16<1>(v, nullptr, &r);
+        const uint32_t d = r ^ want;
         wrong += ((d & 0xffffu) != 0) + ((d >> 16) != 0);
         open += ((o & 0xffffu) != 0) + ((o >> 16) != 0);
     }
@@ -1147,7 +1192,7 @@ struct anacor_surrogate {
     int graph_rows = 0;
     AdamArgs adam{1e-3f, 1e-5f, 0.9f, 0.999f, 1e-8f, 0u};
     int fused = 1;                  // inference by the fused kernel (1) or layer by layer (0)
-    uint8_t *wimg = nullptr;        // the fused kernel's weight image
+    uint8_t *wimg = nullptr;        // the fused kernel's weight image, kept up with the weights
 };
 
 namespace {
@@ -1241,6 +1286,18 @@ cudaError_t convert_all(anacor_surrogate *s, cudaStream_t st)
         const long long n = (long long)kWidth * in_dim(l) * s->E;
         convert_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(s->params, l, s->E, s->W[l], s->WT[l]);
     }
+    return cudaGetLastError();
+}
+
+// the fused kernel's weight image of the BF16 weights
+cudaError_t build_image(anacor_surrogate *s, cudaStream_t st)
+{
+    if (!s->wimg)
+        return cudaSuccess;   // more members than the fused kernel takes
+    WeightPtrs wp;
+    for (int l = 0; l < kDepth; l++)
+        wp.w[l] = s->W[l];
+    weight_image_kernel<<<256, 256, 0, st>>>(wp, s->E, s->wimg);
     return cudaGetLastError();
 }
 
@@ -1424,7 +1481,8 @@ anacor_surrogate *anacor_surrogate_create(int n_members, uint32_t seed, float fo
     const size_t np = (size_t)kParams * n_members;
     bool ok = !cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) && !dalloc(&s->params, np) &&
               !dalloc(&s->m, np) && !dalloc(&s->v, np) && !dalloc(&s->grad, np) && !dalloc(&s->Bf, 32 * kIn) &&
-              !dalloc(&s->loss_acc, 16) && !dalloc(&s->step, 1) && !dalloc(&s->err, 1);
+              !dalloc(&s->loss_acc, 16) && !dalloc(&s->step, 1) && !dalloc(&s->err, 1) &&
+              (n_members > kInferMaxMembers || !dalloc(&s->wimg, (size_t)n_members * kChunksPerMember * kChunkBytes));
     for (int l = 0; l < kDepth && ok; l++) {
         const size_t n = (size_t)kWidth * in_dim(l) * n_members;
         ok = !dalloc(&s->W[l], n) && !dalloc(&s->WT[l], n);
@@ -1443,7 +1501,7 @@ anacor_surrogate *anacor_surrogate_create(int n_members, uint32_t seed, float fo
                (e = cudaMemset(s->grad, 0, np * sizeof(float))) || (e = cudaMemset(s->step, 0, sizeof(unsigned))) ||
                (e = cudaMemset(s->err, 0, sizeof(int))) ||
                (e = cudaMemcpy(s->Bf, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
-               (e = convert_all(s, s->st)) || (e = cudaStreamSynchronize(s->st))))
+               (e = convert_all(s, s->st)) || (e = build_image(s, s->st)) || (e = cudaStreamSynchronize(s->st))))
         ok = false;
     if (!ok) {
         if (e)
@@ -1489,8 +1547,8 @@ int anacor_surrogate_params(anacor_surrogate *s, float *host, int to_device)
     if (!e)
         e = to_device ? cudaMemcpy(s->params, host, n, cudaMemcpyHostToDevice)
                       : cudaMemcpy(host, s->params, n, cudaMemcpyDeviceToHost);
-    if (!e && to_device)
-        e = convert_all(s, s->st);
+    if (!e && to_device && !(e = convert_all(s, s->st)))
+        e = build_image(s, s->st);
     if (!e)
         e = cudaStreamSynchronize(s->st);
     return e ? cuda_fail(e) : report_status(kOk, "");
@@ -1648,6 +1706,8 @@ int anacor_surrogate_train(anacor_surrogate *s, int steps, int batch, float lr_m
     for (int i = 0; i < steps; i++)
         if ((e = cudaGraphLaunch(s->exec, s->st)))
             return cuda_fail(e);
+    if (steps > 0 && (e = build_image(s, s->st)))
+        return cuda_fail(e);
     if (int st = check_err(s, s->st))
         return st;
     if (loss_out && steps > 0 &&
@@ -1715,12 +1775,6 @@ int anacor_surrogate_predict_device(anacor_surrogate *s, const float *d_x7, int6
         if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
             (e = infer_init(dev)))
             return cuda_fail(e);
-        if (!s->wimg && (e = dalloc(&s->wimg, (size_t)s->E * kChunksPerMember * kChunkBytes)))
-            return cuda_fail(e);
-        WeightPtrs wp;
-        for (int l = 0; l < kDepth; l++)
-            wp.w[l] = s->W[l];
-        weight_image_kernel<<<2 * sms, 256, 0, st>>>(wp, s->E, s->wimg);
         InferArgs ia;
         ia.x7 = d_x7;
         ia.n = n;
@@ -1736,8 +1790,24 @@ int anacor_surrogate_predict_device(anacor_surrogate *s, const float *d_x7, int6
         ia.ldm = n;
         ia.err = s->err;
         const long long tiles = (n + kTileRows - 1) / kTileRows;
-        const int grid = (int)std::min<long long>(tiles, sms);
-        infer_kernel<<<grid, kInferThreads, kInferSmem, st>>>(ia);
+        // few tiles: share each one's members between the CTAs of a cluster
+        // while every cluster still has SMs of its own
+        ia.share = 1;
+        while (ia.share * 2 <= s->E && tiles * ia.share * 2 <= sms)
+            ia.share *= 2;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(ia.share > 1 ? tiles * ia.share : std::min<long long>(tiles, sms)));
+        cfg.blockDim = dim3(kInferThreads);
+        cfg.dynamicSmemBytes = kInferSmem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)ia.share;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = ia.share > 1 ? 1 : 0;
+        if ((e = cudaLaunchKernelEx(&cfg, infer_kernel, ia)))
+            return cuda_fail(e);
         if ((e = cudaGetLastError()))
             return cuda_fail(e);
         return report_status(kOk, "");
@@ -1857,7 +1927,7 @@ int anacor_surrogate_load(anacor_surrogate *s, const char *path)
     if ((e = cudaStreamSynchronize(s->st)) ||
         (e = cudaMemcpy(s->params, p.data(), p.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(s->Bf, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
-        (e = convert_all(s, s->st)) || (e = cudaStreamSynchronize(s->st)))
+        (e = convert_all(s, s->st)) || (e = build_image(s, s->st)) || (e = cudaStreamSynchronize(s->st)))
         return cuda_fail(e);
     s->t_mean = scale[0];
     s->t_std = scale[1];
