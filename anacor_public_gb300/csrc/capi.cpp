@@ -1090,10 +1090,14 @@ bool tune_lookup(const anacor_plan *p, TuneVal &v)
 
 // Configuration of a plan run without autotuning (the drop-in entry points):
 // the process's tuned choice for this volume class when there is one; else
-// the distance-field march for volumes with an axis of 256 voxels or more
-// (long legs: it steps over most increments; 25-50 % faster there, while the
-// cooperative march is as fast on a 96^3 volume) and the cooperative march
-// below that.
+// the octant-field march where it saves more than building the fields costs,
+// and the cooperative march for the rest.  Measured on whole drop-in calls:
+// the field march saves about 0.16 ps per leg and voxel of the longest axis
+// (0.13 at 512, 0.19 at 96, 0.3 at 160), the fields cost 110 us (launches, a
+// synchronisation) and 9 ps per voxel, 19 where rows are not whole 4-byte
+// words.  E.g. 96^3 voxels, 9,346 of them sampled: 300 reflections 590 us
+// cooperative, 655 on fields; 1,200: 1,420 and 1,125.  512 x 509 x 505 with
+// 26,685 sampled: 10 reflections 2.0 and 4.5 ms, 400: 4.4 and 5.5 ms.
 int plan_default_config(anacor_plan *p)
 {
     TuneVal v{0, 0, 1, 0.0f};
@@ -1101,9 +1105,10 @@ int plan_default_config(anacor_plan *p)
         return plan_configure(p, v.variant, v.tile, v.order);
     int variant = 0;
     const int big = std::max(p->dims[0], std::max(p->dims[1], p->dims[2]));
-    if (!std::getenv("ANACOR_CTAS_PER_SM") && big >= 256) {
-        // the octant fields march 15-25 % faster than the centred field and
-        // take no longer to build (1.3 vs 1.5 ms on 512x512x400)
+    const double nvol = (double)p->dims[0] * p->dims[1] * p->dims[2];
+    const double saved_us = 0.16e-6 * 2.0 * (double)p->n_vox * (double)p->n_refl * big;
+    const double built_us = 110.0 + (p->dims[2] % 4 ? 19e-6 : 9e-6) * nvol;
+    if (!std::getenv("ANACOR_CTAS_PER_SM") && saved_us > built_us) {
         if (plan_ensure_field(p, 2) == kOk)
             variant = 12;
         succeed();   // labels outside 0..7: the cooperative march, no error
