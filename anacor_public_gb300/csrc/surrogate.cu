@@ -55,7 +55,7 @@ constexpr int kSplitK = 16;             // K splits of the weight-gradient GEMMs
 constexpr int kMaxMembers = 16;
 constexpr int kPredictChunk = 1 << 18;  // rows per inference pass
 
-enum Epi { kEpiStoreF32 = 0, kEpiBiasGelu = 1, kEpiGeluBwd = 2 };
+enum Epi { kEpiStoreF32 = 0, kEpiBiasGelu = 1 };
 
 struct GemmArgs {
     const bf16 *A;
@@ -71,10 +71,6 @@ struct GemmArgs {
     long long ldf, sF;
     bf16 *ob;              // bf16 [M][N]
     long long ldob, sOb;
-    bf16 *ot;              // bf16 [N][M]
-    long long ldot, sOt;
-    const float *aux;      // fp32 [M][N] pre-activation for the GELU derivative
-    long long ldaux, sAux;
     int *err;
 };
 
@@ -178,38 +174,10 @@ __global__ void __launch_bounds__(umma::kThreads, 1) gemm_kernel(GemmArgs g)
                     *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 continue;
             }
-            if (g.mode == kEpiBiasGelu) {
-                const float *bias = g.bias + e * g.sBias + n;
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    v[i] += bias[i];
-                if (g.of) {
-                    float *o = g.of + e * g.sF + (long long)row * g.ldf + n;
-#pragma unroll
-                    for (int i = 0; i < 16; i += 4)
-                        *reinterpret_cast<float4 *>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-                }
-                gelu::values_bf16<8>(v, nullptr, t);
-            } else {   // kEpiGeluBwd
-                const float *h = g.aux + e * g.sAux + (long long)row * g.ldaux + n;
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    v[i] *= gelu::grad(h[i]);
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                    t[i] = gelu::bf16x2(v[2 * i], v[2 * i + 1]);
-            }
-            if (g.ob) {
-                bf16 *o = g.ob + e * g.sOb + (long long)row * g.ldob + n;
-                *reinterpret_cast<uint4 *>(o) = make_uint4(t[0], t[1], t[2], t[3]);
-                *reinterpret_cast<uint4 *>(o + 8) = make_uint4(t[4], t[5], t[6], t[7]);
-            }
-            if (g.ot) {
-                uint16_t *o = reinterpret_cast<uint16_t *>(g.ot + e * g.sOt + row);
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    o[(long long)(n + i) * g.ldot] = (uint16_t)(t[i >> 1] >> (16 * (i & 1)));
-            }
+            gelu::values_bf16<8>(v, g.bias + e * g.sBias + n, t);
+            bf16 *o = g.ob + e * g.sOb + (long long)row * g.ldob + n;
+            *reinterpret_cast<uint4 *>(o) = make_uint4(t[0], t[1], t[2], t[3]);
+            *reinterpret_cast<uint4 *>(o + 8) = make_uint4(t[4], t[5], t[6], t[7]);
         }
     }
     umma::tc_fence_before();
@@ -353,37 +321,9 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x)
     return x;
 }
 
-// training batch of every member: rows drawn with replacement by a hash of
-// (seed, step, member, row); X0 [E][batch][64], X0T [E][64][batch]
-__global__ void gather_kernel(const bf16 *__restrict__ feat, const float *__restrict__ target, long long n_data,
-                              int batch, const unsigned *__restrict__ step, uint32_t seed, bf16 *__restrict__ X0,
-                              bf16 *__restrict__ X0T, float *__restrict__ tb)
-{
-    const int e = blockIdx.y;
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= batch)
-        return;
-    const uint32_t h = mix32(seed ^ mix32(*step * 0x9E3779B9u ^ mix32((uint32_t)e * 0x85EBCA6Bu ^ (uint32_t)b)));
-    const long long r = (long long)(((uint64_t)h * (uint64_t)n_data) >> 32);
-    const uint4 *src = reinterpret_cast<const uint4 *>(feat + r * kFeat);
-    uint4 *dst = reinterpret_cast<uint4 *>(X0 + ((long long)e * batch + b) * kFeat);
-#pragma unroll
-    for (int q = 0; q < kFeat / 8; q++)
-        dst[q] = src[q];
-    const bf16 *f = feat + r * kFeat;
-    bf16 *t = X0T + (long long)e * kFeat * batch + b;
-#pragma unroll 8
-    for (int q = 0; q < kFeat; q++)
-        t[(long long)q * batch] = f[q];
-    tb[(long long)e * batch + b] = target[r];
-}
-
-// output layer, one warp per row: y = A4 . w5 + b5; when training also the
-// loss and dH4 = bf16((dL/dy) w5 * gelu'(H4)) in [row][256] and [256][row]
-__global__ void head_kernel(const bf16 *__restrict__ A4, const float *__restrict__ H4,
-                            const float *__restrict__ params, const float *__restrict__ tb, int rows, int train,
-                            float *__restrict__ y, float *__restrict__ dy, bf16 *__restrict__ dH, bf16 *__restrict__ dHT,
-                            float *__restrict__ loss_acc)
+// output layer, one warp per row: y = A4 . w5 + b5
+__global__ void head_kernel(const bf16 *__restrict__ A4, const float *__restrict__ params, int rows,
+                            float *__restrict__ y)
 {
     const int e = blockIdx.y;
     const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -400,154 +340,8 @@ __global__ void head_kernel(const bf16 *__restrict__ A4, const float *__restrict
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
         acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    const float out = acc + P[kOffB5];
     if (lane == 0)
-        y[base] = out;
-    if (!train)
-        return;
-    const float diff = out - tb[base];
-    const float g = 2.0f * diff / (float)rows;
-    if (lane == 0) {
-        dy[base] = g;
-        atomicAdd(loss_acc + e, diff * diff / (float)rows);
-    }
-    const float *h = H4 + base * kWidth + lane * 8;
-    __align__(16) bf16 t[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        t[q] = __float2bfloat16_rn(g * P[kOffW5 + lane * 8 + q] * gelu::grad(h[q]));
-        dHT[((long long)e * kWidth + lane * 8 + q) * rows + r] = t[q];
-    }
-    reinterpret_cast<uint4 *>(dH + base * kWidth)[lane] = *reinterpret_cast<const uint4 *>(t);
-}
-
-// out[e][n] = sum_b M[e][n][b] * (w ? w[e][b] : 1), one block per (n, e)
-__global__ void rowsum_kernel(const bf16 *__restrict__ Mb, const float *__restrict__ w, int len, long long sM,
-                              long long sw, float *__restrict__ out, long long sOut)
-{
-    const int e = blockIdx.y, n = blockIdx.x;
-    const bf16 *m = Mb + e * sM + (long long)n * len;
-    const float *ww = w ? w + e * sw : nullptr;
-    float acc = 0.0f;
-    for (int b = threadIdx.x; b < len; b += blockDim.x)
-        acc += __bfloat162float(m[b]) * (ww ? ww[b] : 1.0f);
-    __shared__ float red[32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0)
-            out[e * sOut + n] = v;
-    }
-}
-
-// sum_b v[e][b] (output bias gradient), one block per member
-__global__ void vecsum_kernel(const float *__restrict__ v, int len, float *__restrict__ out, long long sOut)
-{
-    const int e = blockIdx.x;
-    float acc = 0.0f;
-    for (int b = threadIdx.x; b < len; b += blockDim.x)
-        acc += v[(long long)e * len + b];
-    __shared__ float red[32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0)
-            out[e * sOut] = s;
-    }
-}
-
-// weight gradient of one layer from its K-split partial products, summed in
-// split order: grad[e][i] = sum_s part[e * ks + s][i]
-__global__ void splitk_reduce_kernel(const float *__restrict__ part, int ks, long long len, float *__restrict__ grad,
-                                     long long sGrad)
-{
-    const int e = blockIdx.y;
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= len)
-        return;
-    float acc = 0.0f;
-    for (int s = 0; s < ks; s++)
-        acc += part[((long long)e * ks + s) * len + i];
-    grad[e * sGrad + i] = acc;
-}
-
-struct AdamArgs {
-    float lr_max, lr_min, b1, b2, eps;
-    unsigned total;   // cosine decay from lr_max to lr_min over `total` steps
-};
-
-// Adam on every member's FP32 masters, step t = *step + 1
-__global__ void adam_kernel(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v,
-                            const float *__restrict__ g, long long n, const unsigned *__restrict__ step, AdamArgs a)
-{
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const unsigned s = *step;
-    const float t = (float)(s + 1u);
-    const float frac = a.total ? fminf((float)s / (float)a.total, 1.0f) : 0.0f;
-    const float lr = a.lr_min + (a.lr_max - a.lr_min) * 0.5f * (1.0f + cospif(frac));
-    const float gi = g[i];
-    const float mi = a.b1 * m[i] + (1.0f - a.b1) * gi;
-    const float vi = a.b2 * v[i] + (1.0f - a.b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float mh = mi / (1.0f - powf(a.b1, t));
-    const float vh = vi / (1.0f - powf(a.b2, t));
-    p[i] -= lr * mh / (sqrtf(vh) + a.eps);
-}
-
-// BF16 copies of layer l's weights: W[e][n][k] and WT[e][k][n]
-__global__ void convert_kernel(const float *__restrict__ params, int l, int E, bf16 *__restrict__ W,
-                               bf16 *__restrict__ WT)
-{
-    const int K = in_dim(l);
-    const long long per = (long long)kWidth * K;
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= per * E)
-        return;
-    const int e = (int)(i / per);
-    const long long r = i - e * per;
-    const int n = (int)(r / K), k = (int)(r % K);
-    const bf16 w = __float2bfloat16_rn(params[e * kParams + off_w(l) + r]);
-    W[i] = w;
-    WT[e * per + (long long)k * kWidth + n] = w;
-}
-
-__global__ void zero_kernel(float *p, int n)
-{
-    if ((int)threadIdx.x < n)
-        p[threadIdx.x] = 0.0f;
-}
-
-__global__ void step_done_kernel(unsigned *step, float *loss_hist, const float *loss_acc, int E, int hist_len)
-{
-    if (threadIdx.x == 0) {
-        const unsigned s = *step;
-        if ((int)s < hist_len) {
-            float acc = 0.0f;
-            for (int e = 0; e < E; e++)
-                acc += loss_acc[e];
-            loss_hist[s] = acc / (float)E;
-        }
-        *step = s + 1u;
-    }
+        y[base] = acc + P[kOffB5];
 }
 
 // ensemble mean of A_h = exp(mu + sd * y) and its relative spread (standard
@@ -694,31 +488,6 @@ __host__ __device__ constexpr int job_chunks(int l) { return in_dim(l) / kWChunk
 __host__ __device__ constexpr int chunk_index(int e, int l, int kq)
 {
     return e * kChunksPerMember + (l == 0 ? 0 : job_chunks(0) + (l - 1) * job_chunks(1)) + kq;
-}
-
-struct WeightPtrs {
-    const bf16 *w[kDepth];
-};
-
-// The weight image: for every member its 26 K-chunks of W_l [256][K], layer by
-// layer, each in the canonical no-swizzle K-major layout of a 256 x 32 tile.
-__global__ void weight_image_kernel(WeightPtrs W, int E, uint8_t *__restrict__ img)
-{
-    constexpr int kPieces = kChunkBytes / 16;   // 16-byte pieces (8 BF16 along K) per chunk
-    const long long total = (long long)E * kChunksPerMember * kPieces;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(t / kPieces);
-        const int p = (int)(t - (long long)c * kPieces);
-        const int e = c / kChunksPerMember, m = c - e * kChunksPerMember;
-        const int l = m < job_chunks(0) ? 0 : 1 + (m - job_chunks(0)) / job_chunks(1);
-        const int kq = m - (l == 0 ? 0 : job_chunks(0) + (l - 1) * job_chunks(1));
-        const int K = in_dim(l);
-        const int r = p >> 2, kc = p & 3;
-        const bf16 *src = W.w[l] + (long long)e * kWidth * K + (long long)r * K + kq * kWChunkK + kc * 8;
-        *reinterpret_cast<uint4 *>(img + (long long)c * kChunkBytes + wchunk_off(r, kc * 8)) =
-            *reinterpret_cast<const uint4 *>(src);
-    }
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
@@ -1122,8 +891,9 @@ __global__ void wait_guard_kernel(unsigned limit, int *err)
         umma::tmem_dealloc(tslot, 32);
 }
 
-// every float through the layers' BF16 GELU: counts[0] the values whose bits
-// differ from the reference evaluation's, counts[1] those the approximation
+// every float through the layers' BF16 GELU and the bounds of its derivative:
+// counts[0] the values whose bits differ from the reference evaluation's or
+// whose derivative is out of bounds, counts[1] those the approximation
 // left to it
 __global__ void gelu_check_kernel(unsigned long long *counts)
 {
@@ -1138,6 +908,14 @@ __global__ void gelu_check_kernel(unsigned long long *counts)
         gelu::values_bf16<1>(v, nullptr, &r);
         const uint32_t d = r ^ want;
         wrong += ((d & 0xffffu) != 0) + ((d >> 16) != 0);
+        // the derivative lies between its bounds (finite values of it)
+        gelu::F2 lo, hi;
+        gelu::grad_bounds(gelu::f2(v[0], v[1]), lo, hi);
+        float l0, l1, h0, h1;
+        gelu::split(lo, l0, l1);
+        gelu::split(hi, h0, h1);
+        const float g0 = gelu::grad(v[0]), g1 = gelu::grad(v[1]);
+        wrong += (isfinite(g0) && !(l0 <= g0 && g0 <= h0)) + (isfinite(g1) && !(l1 <= g1 && g1 <= h1));
         open += ((o & 0xffffu) != 0) + ((o >> 16) != 0);
     }
     atomicAdd(&counts[0], wrong);
@@ -1159,6 +937,26 @@ cudaError_t infer_init(int dev)
     return g_infer_init_err[dev];
 }
 
+#include "surrogate_train.cuh"
+
+std::once_flag g_train_once[64];
+cudaError_t g_train_init_err[64];
+
+// opt the training kernels into their shared-memory sizes once per device
+// (outside any stream capture)
+cudaError_t train_init(int dev)
+{
+    if (dev < 0 || dev >= 64)
+        return cudaErrorInvalidDevice;
+    std::call_once(g_train_once[dev], [dev] {
+        cudaError_t e = cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
+        if (!e)
+            e = cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmem);
+        g_train_init_err[dev] = e;
+    });
+    return g_train_init_err[dev];
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ state
@@ -1167,22 +965,25 @@ struct anacor_surrogate {
     int E = 4;
     uint32_t seed = 0;
     cudaStream_t st = nullptr;
-    float *params = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *part = nullptr;
-    bf16 *W[kDepth] = {}, *WT[kDepth] = {};
+    float *params = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;
+    bf16 *W[kDepth] = {};                   // BF16 weights [E][256][K] (the layer-by-layer path)
+    uint8_t *wimg = nullptr, *wtimg = nullptr;   // and as the chunks of W and W^T that the fused kernels read
     float *Bf = nullptr;                    // Fourier matrix [32][7]
     double t_mean = 0.0, t_std = 1.0;       // log A_h = t_mean + t_std * y
     // training data
     long long n_data = 0;
     float *target = nullptr;
     bf16 *feat = nullptr;
-    // workspace for `rows` rows per member
+    // inference workspace of the layer-by-layer path for `rows` rows per member
     int rows = 0;
-    bool train_ws = false;
-    bf16 *X0 = nullptr, *X0T = nullptr;
-    float *H[kDepth] = {};
-    bf16 *A[kDepth] = {}, *AT[kDepth] = {};
-    bf16 *dH = nullptr, *dHT = nullptr, *dH2 = nullptr, *dHT2 = nullptr;
-    float *tb = nullptr, *y = nullptr, *dy = nullptr, *loss_acc = nullptr;
+    bf16 *X0 = nullptr, *A[2] = {};
+    float *y = nullptr;
+    // training workspace for `train_rows` rows per member (see surrogate_train.cuh)
+    int train_rows = 0;
+    uint4 *X0i = nullptr, *Ai[kDepth] = {}, *dHi[kDepth] = {};
+    float4 *Hi[2] = {}, *part = nullptr;
+    float *ty = nullptr, *dy = nullptr;
+    float *loss_acc = nullptr;              // zero between steps
     unsigned *step = nullptr;
     float *loss_hist = nullptr;
     int hist_len = 0;
@@ -1192,7 +993,6 @@ struct anacor_surrogate {
     int graph_rows = 0;
     AdamArgs adam{1e-3f, 1e-5f, 0.9f, 0.999f, 1e-8f, 0u};
     int fused = 1;                  // inference by the fused kernel (1) or layer by layer (0)
-    uint8_t *wimg = nullptr;        // the fused kernel's weight image, kept up with the weights
 };
 
 namespace {
@@ -1225,45 +1025,62 @@ void drop_graph(anacor_surrogate *s)
 
 void free_work(anacor_surrogate *s)
 {
-    drop_graph(s);
-    dfree(s->X0); dfree(s->X0T);
-    for (int l = 0; l < kDepth; l++) {
-        dfree(s->H[l]); dfree(s->A[l]); dfree(s->AT[l]);
-    }
-    dfree(s->dH); dfree(s->dHT); dfree(s->dH2); dfree(s->dHT2);
-    dfree(s->tb); dfree(s->y); dfree(s->dy); dfree(s->part);
+    dfree(s->X0); dfree(s->A[0]); dfree(s->A[1]); dfree(s->y);
     s->rows = 0;
-    s->train_ws = false;
 }
 
-// workspace for exactly `rows` rows per member: inference keeps two
-// activation buffers, training every layer's activations in both orders
-int ensure_work(anacor_surrogate *s, int rows, bool train)
+void free_train(anacor_surrogate *s)
+{
+    drop_graph(s);
+    dfree(s->X0i);
+    for (int l = 0; l < kDepth; l++) {
+        dfree(s->Ai[l]); dfree(s->dHi[l]);
+    }
+    dfree(s->Hi[0]); dfree(s->Hi[1]); dfree(s->part); dfree(s->ty); dfree(s->dy);
+    s->train_rows = 0;
+}
+
+// layer-by-layer inference for exactly `rows` rows per member
+int ensure_work(anacor_surrogate *s, int rows)
 {
     if (rows <= 0 || rows % umma::kBM)
         return report_status(kErrArgs, "surrogate: rows must be a positive multiple of 128");
-    if (train && rows % (umma::kBK * kSplitK))
-        return report_status(kErrArgs, "surrogate: the training batch must be a multiple of 1024");
-    if (s->rows == rows && s->train_ws == train)
+    if (s->rows == rows)
         return kOk;
     free_work(s);
     const size_t E = s->E, R = rows;
-    bool ok = !dalloc(&s->X0, E * R * kFeat) && !dalloc(&s->y, E * R) && !dalloc(&s->A[0], E * R * kWidth) &&
-              !dalloc(&s->A[1], E * R * kWidth);
-    if (ok && train) {
-        ok = !dalloc(&s->X0T, E * R * kFeat) && !dalloc(&s->dH, E * R * kWidth) && !dalloc(&s->dHT, E * R * kWidth) &&
-             !dalloc(&s->dH2, E * R * kWidth) && !dalloc(&s->dHT2, E * R * kWidth) && !dalloc(&s->tb, E * R) &&
-             !dalloc(&s->dy, E * R) && !dalloc(&s->part, E * kSplitK * (size_t)kWidth * kWidth);
-        for (int l = 0; l < kDepth && ok; l++)
-            ok = !dalloc(&s->H[l], E * R * kWidth) && !dalloc(&s->AT[l], E * R * kWidth) &&
-                 (l < 2 || !dalloc(&s->A[l], E * R * kWidth));
-    }
-    if (!ok) {
+    if (dalloc(&s->X0, E * R * kFeat) || dalloc(&s->y, E * R) || dalloc(&s->A[0], E * R * kWidth) ||
+        dalloc(&s->A[1], E * R * kWidth)) {
         free_work(s);
         return report_status(kErrCuda, "surrogate: device allocation failed");
     }
     s->rows = rows;
-    s->train_ws = train;
+    return kOk;
+}
+
+// training on batches of exactly `rows` rows per member
+int ensure_train(anacor_surrogate *s, int rows)
+{
+    if (rows <= 0 || rows % (umma::kBK * kSplitK))
+        return report_status(kErrArgs, "surrogate: the training batch must be a multiple of 1024");
+    int dev = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) || (e = train_init(dev)))
+        return report_status(kErrCuda, cudaGetErrorString(e));
+    if (s->train_rows == rows)
+        return kOk;
+    free_train(s);
+    const size_t E = s->E, R = rows;
+    bool ok = !dalloc(&s->X0i, E * R * kFeat / 8) && !dalloc(&s->ty, E * R) && !dalloc(&s->dy, E * R) &&
+              !dalloc(&s->part, E * (size_t)kPartFloats / 4) && !dalloc(&s->Hi[0], E * R * kWidth / 4) &&
+              !dalloc(&s->Hi[1], E * R * kWidth / 4);
+    for (int l = 0; l < kDepth && ok; l++)
+        ok = !dalloc(&s->Ai[l], E * R * kWidth / 8) && !dalloc(&s->dHi[l], E * R * kWidth / 8);
+    if (!ok) {
+        free_train(s);
+        return report_status(kErrCuda, "surrogate: device allocation failed");
+    }
+    s->train_rows = rows;
     return kOk;
 }
 
@@ -1280,32 +1097,26 @@ int check_err(anacor_surrogate *s, cudaStream_t st)
     return report_status(kOk, "");
 }
 
+WeightCopies weight_copies(const anacor_surrogate *s)
+{
+    WeightCopies c;
+    for (int l = 0; l < kDepth; l++)
+        c.w[l] = s->W[l];
+    c.wimg = s->wimg;
+    c.wtimg = s->wtimg;
+    return c;
+}
+
+// the BF16 copies of the weights, after the masters have changed
 cudaError_t convert_all(anacor_surrogate *s, cudaStream_t st)
 {
-    for (int l = 0; l < kDepth; l++) {
-        const long long n = (long long)kWidth * in_dim(l) * s->E;
-        convert_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(s->params, l, s->E, s->W[l], s->WT[l]);
-    }
+    copies_kernel<<<512, 256, 0, st>>>(s->params, s->E, weight_copies(s));
     return cudaGetLastError();
 }
 
-// the fused kernel's weight image of the BF16 weights
-cudaError_t build_image(anacor_surrogate *s, cudaStream_t st)
-{
-    if (!s->wimg)
-        return cudaSuccess;   // more members than the fused kernel takes
-    WeightPtrs wp;
-    for (int l = 0; l < kDepth; l++)
-        wp.w[l] = s->W[l];
-    weight_image_kernel<<<256, 256, 0, st>>>(wp, s->E, s->wimg);
-    return cudaGetLastError();
-}
-
-// Forward of every member over `rows` rows of X0 ([E][rows][64], or one
-// shared [rows][64] when x_shared).  With keep, every layer's pre-activation
-// and both orders of its activation stay for the backward pass.  Returns the
+// Forward of every member over `rows` rows of the shared X0 [rows][64]; the
 // buffer that holds the last hidden activation.
-bf16 *forward(anacor_surrogate *s, int rows, bool x_shared, bool keep, cudaStream_t st, cudaError_t &err)
+bf16 *forward(anacor_surrogate *s, int rows, cudaStream_t st, cudaError_t &err)
 {
     const long long R = rows;
     const bf16 *in = s->X0;
@@ -1313,10 +1124,10 @@ bf16 *forward(anacor_surrogate *s, int rows, bool x_shared, bool keep, cudaStrea
     for (int l = 0; l < kDepth; l++) {
         GemmArgs g{};
         const int K = in_dim(l);
-        out = keep ? s->A[l] : s->A[l & 1];
+        out = s->A[l & 1];
         g.A = in;
         g.lda = K;
-        g.sA = (l == 0 && x_shared) ? 0 : R * K;
+        g.sA = l == 0 ? 0 : R * K;
         g.B = s->W[l];
         g.ldb = K;
         g.sB = (long long)kWidth * K;
@@ -1324,12 +1135,8 @@ bf16 *forward(anacor_surrogate *s, int rows, bool x_shared, bool keep, cudaStrea
         g.mode = kEpiBiasGelu;
         g.bias = s->params + off_b(l);
         g.sBias = kParams;
-        g.of = keep ? s->H[l] : nullptr;
-        g.ldf = kWidth; g.sF = R * kWidth;
         g.ob = out;
         g.ldob = kWidth; g.sOb = R * kWidth;
-        g.ot = keep ? s->AT[l] : nullptr;
-        g.ldot = R; g.sOt = R * kWidth;
         g.err = s->err;
         if ((err = gemm(g, s->E, st)))
             return nullptr;
@@ -1339,74 +1146,70 @@ bf16 *forward(anacor_surrogate *s, int rows, bool x_shared, bool keep, cudaStrea
     return out;
 }
 
-// backward from the head's dH4 down to every weight and bias gradient
-cudaError_t backward(anacor_surrogate *s, int rows, cudaStream_t st)
+// One step on batches of s->train_rows rows: drawn from the training set, or
+// (ordered) the first rows of `feat` and `target` for every member.  With
+// `update` the Adam step, the weight copies and the step count, else the
+// gradients into s->grad.
+cudaError_t train_step(anacor_surrogate *s, const bf16 *feat, const float *target, long long n, bool ordered,
+                       bool update, int sms, cudaStream_t st)
 {
-    cudaError_t e;
-    const long long R = rows;
-    rowsum_kernel<<<dim3(kWidth, s->E), 256, 0, st>>>(s->AT[kDepth - 1], s->dy, rows, R * kWidth, R,
-                                                       s->grad + kOffW5, kParams);
-    vecsum_kernel<<<s->E, 256, 0, st>>>(s->dy, rows, s->grad + kOffB5, kParams);
-    bf16 *dH = s->dH, *dHT = s->dHT, *dH2 = s->dH2, *dHT2 = s->dHT2;
-    for (int l = kDepth - 1; l >= 0; l--) {
-        const int K = in_dim(l);
-        // dW_l = dH_l^T A_{l-1} (A_{-1} = X0): [256][K], K-split over the rows
-        GemmArgs g{};
-        g.A = dHT; g.lda = R; g.sA = R * kWidth;
-        g.B = l == 0 ? s->X0T : s->AT[l - 1]; g.ldb = R; g.sB = R * K;
-        g.M = kWidth; g.N = K; g.K = rows;
-        g.ksplit = kSplitK;
-        g.mode = kEpiStoreF32;
-        g.of = s->part; g.ldf = K; g.sF = (long long)kWidth * K;
-        g.err = s->err;
-        if ((e = gemm(g, s->E, st)))
-            return e;
-        const long long len = (long long)kWidth * K;
-        splitk_reduce_kernel<<<dim3((unsigned)((len + 255) / 256), s->E), 256, 0, st>>>(s->part, kSplitK, len,
-                                                                                       s->grad + off_w(l), kParams);
-        rowsum_kernel<<<dim3(kWidth, s->E), 256, 0, st>>>(dHT, nullptr, rows, R * kWidth, 0, s->grad + off_b(l),
-                                                           kParams);
-        if (l == 0)
-            break;
-        // dH_{l-1} = bf16((dH_l W_l) * gelu'(H_{l-1})): [rows][256]
-        GemmArgs b{};
-        b.A = dH; b.lda = kWidth; b.sA = R * kWidth;
-        b.B = s->WT[l]; b.ldb = kWidth; b.sB = (long long)kWidth * K;
-        b.M = rows; b.N = K; b.K = kWidth;
-        b.mode = kEpiGeluBwd;
-        b.aux = s->H[l - 1]; b.ldaux = kWidth; b.sAux = R * kWidth;
-        b.ob = dH2; b.ldob = kWidth; b.sOb = R * kWidth;
-        b.ot = dHT2; b.ldot = R; b.sOt = R * kWidth;
-        b.err = s->err;
-        if ((e = gemm(b, s->E, st)))
-            return e;
-        std::swap(dH, dH2);
-        std::swap(dHT, dHT2);
+    ChainArgs c{};
+    c.feat = feat;
+    c.target = target;
+    c.n_data = n;
+    c.batch = s->train_rows;
+    c.ordered = ordered;
+    c.seed = s->seed;
+    c.step = s->step;
+    c.params = s->params;
+    c.wimg = s->wimg;
+    c.wtimg = s->wtimg;
+    c.E = s->E;
+    c.X0 = s->X0i;
+    for (int l = 0; l < kDepth; l++) {
+        c.A[l] = s->Ai[l];
+        c.dH[l] = s->dHi[l];
     }
-    return cudaGetLastError();
-}
-
-// forward + loss + backward on the batch in X0 / X0T / tb, then (update)
-// the Adam step, the BF16 weight copies and the step counter
-cudaError_t train_step_body(anacor_surrogate *s, int rows, bool update, cudaStream_t st)
-{
-    cudaError_t e;
-    zero_kernel<<<1, 32, 0, st>>>(s->loss_acc, s->E);
-    bf16 *a4 = forward(s, rows, false, true, st, e);
-    if (e)
-        return e;
-    head_kernel<<<dim3((rows * 32 + 255) / 256, s->E), 256, 0, st>>>(a4, s->H[kDepth - 1], s->params, s->tb, rows,
-                                                                      1, s->y, s->dy, s->dH, s->dHT, s->loss_acc);
-    if ((e = backward(s, rows, st)))
-        return e;
-    if (update) {
-        const long long n = kParams * s->E;
-        adam_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(s->params, s->m, s->v, s->grad, n, s->step,
-                                                                  s->adam);
-        if ((e = convert_all(s, st)))
-            return e;
-        step_done_kernel<<<1, 32, 0, st>>>(s->step, s->loss_hist, s->loss_acc, s->E, s->hist_len);
+    c.H[0] = s->Hi[0];
+    c.H[1] = s->Hi[1];
+    c.y = s->ty;
+    c.dy = s->dy;
+    c.loss_acc = s->loss_acc;
+    c.err = s->err;
+    const int units = s->train_rows / kTileRows * s->E;
+    chain_kernel<<<std::min(units, sms), kInferThreads, kChainSmem, st>>>(c);
+    DwArgs d{};
+    d.X0 = s->X0i;
+    UpdateArgs u{};
+    for (int l = 0; l < kDepth; l++) {
+        d.A[l] = s->Ai[l];
+        d.dH[l] = s->dHi[l];
+        u.dH[l] = s->dHi[l];
     }
+    d.batch = s->train_rows;
+    d.part = s->part;
+    d.step = s->step;
+    d.loss_acc = s->loss_acc;
+    d.loss_hist = s->loss_hist;
+    d.E = s->E;
+    d.hist_len = s->hist_len;
+    d.count_step = update;
+    d.err = s->err;
+    dw_kernel<<<dim3(2 * kSplitK * kDepth, s->E), kDwThreads, kDwSmem, st>>>(d);
+    u.part = s->part;
+    u.A3 = s->Ai[kDepth - 1];
+    u.dy = s->dy;
+    u.batch = s->train_rows;
+    u.E = s->E;
+    u.params = s->params;
+    u.m = s->m;
+    u.v = s->v;
+    u.grad = s->grad;
+    u.step = s->step;
+    u.adam = s->adam;
+    u.update = update;
+    u.copies = weight_copies(s);
+    update_kernel<<<dim3(kPatches + kVectors, s->E), 256, 0, st>>>(u);
     return cudaGetLastError();
 }
 
@@ -1438,11 +1241,10 @@ cudaError_t predict_pass(anacor_surrogate *s, const float *d_x7, long long n, in
     cudaError_t e;
     features_kernel<<<(unsigned)(((long long)rows_pad * (kFeat / 2) + 255) / 256), 256, 0, st>>>(d_x7, s->Bf, n,
                                                                                                  rows_pad, s->X0);
-    bf16 *a4 = forward(s, rows_pad, true, false, st, e);
+    bf16 *a4 = forward(s, rows_pad, st, e);
     if (e)
         return e;
-    head_kernel<<<dim3((rows_pad * 32 + 255) / 256, s->E), 256, 0, st>>>(a4, nullptr, s->params, nullptr, rows_pad,
-                                                                          0, s->y, nullptr, nullptr, nullptr, nullptr);
+    head_kernel<<<dim3((rows_pad * 32 + 255) / 256, s->E), 256, 0, st>>>(a4, s->params, rows_pad, s->y);
     ensemble_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(s->y, s->E, n, rows_pad, (float)s->t_mean,
                                                                  (float)s->t_std, d_mean, d_spread, d_members, ldm);
     return cudaGetLastError();
@@ -1482,10 +1284,11 @@ anacor_surrogate *anacor_surrogate_create(int n_members, uint32_t seed, float fo
     bool ok = !cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) && !dalloc(&s->params, np) &&
               !dalloc(&s->m, np) && !dalloc(&s->v, np) && !dalloc(&s->grad, np) && !dalloc(&s->Bf, 32 * kIn) &&
               !dalloc(&s->loss_acc, 16) && !dalloc(&s->step, 1) && !dalloc(&s->err, 1) &&
-              (n_members > kInferMaxMembers || !dalloc(&s->wimg, (size_t)n_members * kChunksPerMember * kChunkBytes));
+              !dalloc(&s->wimg, (size_t)n_members * kChunksPerMember * kChunkBytes) &&
+              !dalloc(&s->wtimg, (size_t)n_members * kChunksBack * kChunkBytes);
     for (int l = 0; l < kDepth && ok; l++) {
         const size_t n = (size_t)kWidth * in_dim(l) * n_members;
-        ok = !dalloc(&s->W[l], n) && !dalloc(&s->WT[l], n);
+        ok = !dalloc(&s->W[l], n);
     }
     std::vector<float> p(np, 0.0f);
     init_params(p, n_members, seed);
@@ -1499,9 +1302,9 @@ anacor_surrogate *anacor_surrogate_create(int n_members, uint32_t seed, float fo
     if (ok && ((e = cudaMemcpy(s->params, p.data(), np * sizeof(float), cudaMemcpyHostToDevice)) ||
                (e = cudaMemset(s->m, 0, np * sizeof(float))) || (e = cudaMemset(s->v, 0, np * sizeof(float))) ||
                (e = cudaMemset(s->grad, 0, np * sizeof(float))) || (e = cudaMemset(s->step, 0, sizeof(unsigned))) ||
-               (e = cudaMemset(s->err, 0, sizeof(int))) ||
+               (e = cudaMemset(s->err, 0, sizeof(int))) || (e = cudaMemset(s->loss_acc, 0, 16 * sizeof(float))) ||
                (e = cudaMemcpy(s->Bf, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
-               (e = convert_all(s, s->st)) || (e = build_image(s, s->st)) || (e = cudaStreamSynchronize(s->st))))
+               (e = convert_all(s, s->st)) || (e = cudaStreamSynchronize(s->st))))
         ok = false;
     if (!ok) {
         if (e)
@@ -1522,12 +1325,12 @@ void anacor_surrogate_destroy(anacor_surrogate *s)
     if (s->st)
         cudaStreamSynchronize(s->st);
     free_work(s);
+    free_train(s);
     dfree(s->params); dfree(s->m); dfree(s->v); dfree(s->grad); dfree(s->Bf);
-    dfree(s->loss_acc); dfree(s->step); dfree(s->err); dfree(s->loss_hist); dfree(s->wimg);
+    dfree(s->loss_acc); dfree(s->step); dfree(s->err); dfree(s->loss_hist); dfree(s->wimg); dfree(s->wtimg);
     dfree(s->target); dfree(s->feat);
     for (int l = 0; l < kDepth; l++) {
         dfree(s->W[l]);
-        dfree(s->WT[l]);
     }
     if (s->st)
         cudaStreamDestroy(s->st);
@@ -1547,8 +1350,8 @@ int anacor_surrogate_params(anacor_surrogate *s, float *host, int to_device)
     if (!e)
         e = to_device ? cudaMemcpy(s->params, host, n, cudaMemcpyHostToDevice)
                       : cudaMemcpy(host, s->params, n, cudaMemcpyDeviceToHost);
-    if (!e && to_device && !(e = convert_all(s, s->st)))
-        e = build_image(s, s->st);
+    if (!e && to_device)
+        e = convert_all(s, s->st);
     if (!e)
         e = cudaStreamSynchronize(s->st);
     return e ? cuda_fail(e) : report_status(kOk, "");
@@ -1662,11 +1465,14 @@ int anacor_surrogate_train(anacor_surrogate *s, int steps, int batch, float lr_m
 {
     if (!s || steps < 0 || batch <= 0 || !s->n_data || !(lr_max > 0.0f) || lr_min < 0.0f || total_steps < 0)
         return report_status(kErrArgs, "surrogate: bad training arguments");
-    if (int st = ensure_work(s, batch, true))
+    if (int st = ensure_train(s, batch))
         return st;
+    int dev = 0, sms = 0;
     unsigned start = 0;
     cudaError_t e;
-    if ((e = cudaStreamSynchronize(s->st)) || (e = cudaMemcpy(&start, s->step, sizeof(unsigned), cudaMemcpyDeviceToHost)))
+    if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) ||
+        (e = cudaStreamSynchronize(s->st)) ||
+        (e = cudaMemcpy(&start, s->step, sizeof(unsigned), cudaMemcpyDeviceToHost)))
         return cuda_fail(e);
     const AdamArgs a{lr_max, lr_min, 0.9f, 0.999f, 1e-8f, (unsigned)total_steps};
     if (std::memcmp(&a, &s->adam, sizeof(a)) != 0) {
@@ -1689,9 +1495,7 @@ int anacor_surrogate_train(anacor_surrogate *s, int steps, int batch, float lr_m
         drop_graph(s);
         if ((e = cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal)))
             return cuda_fail(e);
-        gather_kernel<<<dim3((batch + 255) / 256, s->E), 256, 0, s->st>>>(s->feat, s->target, s->n_data, batch,
-                                                                          s->step, s->seed, s->X0, s->X0T, s->tb);
-        cudaError_t le = train_step_body(s, batch, true, s->st);
+        const cudaError_t le = train_step(s, s->feat, s->target, s->n_data, false, true, sms, s->st);
         e = cudaStreamEndCapture(s->st, &s->graph);
         if (le || e) {
             drop_graph(s);
@@ -1706,8 +1510,6 @@ int anacor_surrogate_train(anacor_surrogate *s, int steps, int batch, float lr_m
     for (int i = 0; i < steps; i++)
         if ((e = cudaGraphLaunch(s->exec, s->st)))
             return cuda_fail(e);
-    if (steps > 0 && (e = build_image(s, s->st)))
-        return cuda_fail(e);
     if (int st = check_err(s, s->st))
         return st;
     if (loss_out && steps > 0 &&
@@ -1721,39 +1523,26 @@ int anacor_surrogate_gradients(anacor_surrogate *s, const float *x7, const float
 {
     if (!s || rows <= 0 || !x7 || !target)
         return report_status(kErrArgs, "bad arguments");
-    if (int st = ensure_work(s, rows, true))
+    if (int st = ensure_train(s, rows))
         return st;
     const size_t R = rows;
     float *d_x = nullptr, *d_t = nullptr;
     bf16 *d_f = nullptr;
+    int dev = 0, sms = 0;
     cudaError_t e;
-    std::vector<bf16> hx(R * kFeat), ht(R * kFeat);
-    if (!(e = cudaStreamSynchronize(s->st)) && !(e = dalloc(&d_x, 7 * R)) && !(e = dalloc(&d_t, R)) &&
+    if (!(e = cudaGetDevice(&dev)) && !(e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) &&
+        !(e = cudaStreamSynchronize(s->st)) && !(e = dalloc(&d_x, 7 * R)) && !(e = dalloc(&d_t, R)) &&
         !(e = dalloc(&d_f, R * kFeat)) && !(e = cudaMemcpy(d_x, x7, 7 * R * sizeof(float), cudaMemcpyHostToDevice)) &&
         !(e = cudaMemcpy(d_t, target, R * sizeof(float), cudaMemcpyHostToDevice))) {
         features_kernel<<<(unsigned)((R * (kFeat / 2) + 255) / 256), 256, 0, s->st>>>(d_x, s->Bf, rows, rows, d_f);
-        if (!(e = cudaGetLastError()) &&
-            !(e = cudaMemcpyAsync(hx.data(), d_f, hx.size() * sizeof(bf16), cudaMemcpyDeviceToHost, s->st)))
+        // the same batch, rows in order, for every member
+        if (!(e = cudaGetLastError()) && !(e = train_step(s, d_f, d_t, rows, true, false, sms, s->st)))
             e = cudaStreamSynchronize(s->st);
     }
-    if (!e) {
-        for (size_t r = 0; r < R; r++)
-            for (int q = 0; q < kFeat; q++)
-                ht[(size_t)q * R + r] = hx[r * kFeat + q];
-        // the same batch, rows in order, for every member
-        for (int m = 0; m < s->E && !e; m++)
-            if (!(e = cudaMemcpy(s->X0 + m * R * kFeat, d_f, R * kFeat * sizeof(bf16), cudaMemcpyDeviceToDevice)) &&
-                !(e = cudaMemcpy(s->X0T + m * R * kFeat, ht.data(), ht.size() * sizeof(bf16), cudaMemcpyHostToDevice)))
-                e = cudaMemcpy(s->tb + m * R, d_t, R * sizeof(float), cudaMemcpyDeviceToDevice);
-    }
-    if (!e)
-        e = train_step_body(s, rows, false, s->st);
-    if (!e)
-        e = cudaStreamSynchronize(s->st);
     if (!e && grads_out)
         e = cudaMemcpy(grads_out, s->grad, (size_t)kParams * s->E * sizeof(float), cudaMemcpyDeviceToHost);
     if (!e && y_out)
-        e = cudaMemcpy(y_out, s->y, R * s->E * sizeof(float), cudaMemcpyDeviceToHost);
+        e = cudaMemcpy(y_out, s->ty, R * s->E * sizeof(float), cudaMemcpyDeviceToHost);
     dfree(d_x); dfree(d_t); dfree(d_f);
     if (e)
         return cuda_fail(e);
@@ -1813,12 +1602,12 @@ int anacor_surrogate_predict_device(anacor_surrogate *s, const float *d_x7, int6
         return report_status(kOk, "");
     }
     const int chunk = (int)std::min<int64_t>(kPredictChunk, (n + umma::kBM - 1) / umma::kBM * umma::kBM);
-    if (s->rows != chunk || s->train_ws) {
+    if (s->rows != chunk) {
         // the workspace is about to be replaced: nothing may still use it
         cudaError_t e;
         if ((e = cudaStreamSynchronize(s->st)) || (stream && (e = cudaStreamSynchronize(st))))
             return cuda_fail(e);
-        if (int r = ensure_work(s, chunk, false))
+        if (int r = ensure_work(s, chunk))
             return r;
     }
     for (int64_t i0 = 0; i0 < n; i0 += chunk) {
@@ -1927,7 +1716,7 @@ int anacor_surrogate_load(anacor_surrogate *s, const char *path)
     if ((e = cudaStreamSynchronize(s->st)) ||
         (e = cudaMemcpy(s->params, p.data(), p.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
         (e = cudaMemcpy(s->Bf, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
-        (e = convert_all(s, s->st)) || (e = build_image(s, s->st)) || (e = cudaStreamSynchronize(s->st)))
+        (e = convert_all(s, s->st)) || (e = cudaStreamSynchronize(s->st)))
         return cuda_fail(e);
     s->t_mean = scale[0];
     s->t_std = scale[1];
