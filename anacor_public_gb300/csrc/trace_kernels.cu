@@ -897,15 +897,18 @@ __device__ __forceinline__ void trace_leg(const LegHead &h, const FaceRule *rule
 //  * a leg whose non-vacuum labels keep room from the walls ahead of it needs
 //    no step count and no wall limit: it meets vacuum first;
 //  * the inner loop holds no call (what lives across one is kept in local
-//    memory: 92 local loads a warp and leg before, 9 now), and the kernel fits
-//    48 registers, five CTAs an SM (six, at 40 registers: 3 % slower);
+//    memory: 92 local loads a warp and leg then), what a march need not hold
+//    lies in shared memory at constant addresses (FieldShared; 10.2 -> 2.7
+//    local loads), and the kernel fits 48 registers, five CTAs an SM (six, at
+//    40 registers: 3 % slower);
 //  * everything rare (close exit-face calls, ratios beyond fixed point,
 //    full_iteration, legs that reach the wall limit, more than kMaxSegments
 //    class changes) is out of line in leg_slow, which reads the full rule
 //    from global memory.
-// 512x512x400, 13,266 voxels, 20,000 reflections: 30.0 -> 20.6 ms (1,430 ->
+// 512x512x400, 13,266 voxels, 20,000 reflections: 30.0 -> 20.2 ms (1,430 ->
 // 915 warp instructions per 32 legs; L1 misses at 70 %, L2 at 59 % of their
-// peak rates, issue slots at 56 %).
+// peak rates, issue slots at 56 %).  1024x1024x800, all 11.7 million voxels,
+// 32 reflections: 22.9 -> 17.0 ms (18.6 with those 10.2 local loads).
 
 // One leg's rule for one exit axis.  q: the 32.32 ratios of the two other
 // axes a and b (lo, hi words).  off: their initial low words -- the rounding
@@ -941,6 +944,8 @@ struct alignas(16) WarpTab {
     int dy, dx, is_exp, count_steps;
     const ReflTable *refl;
     const SampleDesc *desc;
+    const short4 *coords;    // the item's voxels
+    int n;
 };
 
 // Half-width of the ambiguous zone around a rounding boundary, in 2^-32
@@ -953,7 +958,7 @@ constexpr uint32_t kFieldMargin = 4096u + 16u;
 // Fills a warp's table for reflection table T: lanes 0..5 a rule each (leg,
 // axis), lanes 8..13 the exit-face operands, lanes 16..23 the sample's constants.
 __device__ __forceinline__ void fill_warp_tab(WarpTab &w, const ReflTable *__restrict__ T, const SampleDesc &D,
-                                              int lane)
+                                              int tile, int lane)
 {
     const int part = lane >> 3, k = lane & 7;
     if (part < 2 && k < 6) {
@@ -1025,6 +1030,8 @@ __device__ __forceinline__ void fill_warp_tab(WarpTab &w, const ReflTable *__res
             w.count_steps = D.steps != nullptr;
             w.refl = T;
             w.desc = &D;
+            w.coords = D.coords + (long long)tile * D.tile;
+            w.n = min(D.tile, D.n_vox - tile * D.tile);
         }
     }
 }
@@ -1067,6 +1074,33 @@ __device__ __forceinline__ uint32_t field_byte(const uint8_t *start, const HotRu
 // that would be longer than kMaxSegments parks in the row after the last.
 constexpr int kSegRows = kMaxSegments + 1;
 
+// Shared memory of the field kernels.  It is dynamic, so that every function
+// reaches it by a constant address, and a lane's place in it comes from its
+// thread number, read anew where it is needed: the march's registers are what
+// limits the warps an SM holds, and a pointer kept across a leg ended up in
+// local memory, whose loads miss L1 among the field's.
+struct FieldShared {
+    WarpTab tabs[kWarps];
+    uint16_t seg[kSegRows * kBlock];
+    float4 incident[kBlock];     // the incident leg's lengths while the diffracted leg marches
+    float2 total[kBlock];        // compensated sums
+    unsigned steps[kBlock];
+    FloatPair consts[7];         // map kernel: squared voxel edges (z, y, x), mu
+};
+extern __shared__ __align__(16) uint8_t field_smem[];
+
+__device__ __forceinline__ FieldShared &field_shared() { return *reinterpret_cast<FieldShared *>(field_smem); }
+
+__device__ __forceinline__ int thread_now()
+{
+    int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+}
+
+__device__ __forceinline__ WarpTab &warp_tab() { return field_shared().tabs[thread_now() >> 5]; }
+__device__ __forceinline__ uint16_t *seg_list() { return field_shared().seg + thread_now(); }
+
 struct SlowLeg {
     float4 L;
     int len;
@@ -1079,10 +1113,12 @@ enum SlowFrom { kFromStart = 0, kFromLimit = 1, kFromStop = 2 };
 // The rest of a leg that the field march does not finish by itself: FP32
 // lengths (out.Lf), or FP64 ones in the reference's order (out.L).
 template <bool kF32>
-__device__ __forceinline__ void leg_rest(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int from,
-                                         int axis, int i, int nseg, int prev, int lim, LegResult &out)
+__device__ __forceinline__ void leg_rest(int leg, int vi, int from, int axis, int i, int nseg, int prev, int lim,
+                                         LegResult &out)
 {
-    const short4 cv = __ldg(voxel);
+    const WarpTab &W = warp_tab();
+    uint16_t *seg = seg_list();
+    const short4 cv = __ldg(W.coords + vi);
     const SampleDesc &D = *W.desc;
     const ReflTable *T = W.refl;
     const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
@@ -1117,13 +1153,12 @@ __device__ __forceinline__ void leg_rest(const WarpTab &W, int leg, const short4
                             out, D.voxelf);
 }
 
-__device__ __noinline__ SlowLeg leg_slow(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int from,
-                                         int axis, int i, int nseg, int prev, int lim)
+__device__ __noinline__ SlowLeg leg_slow(int leg, int vi, int from, int axis, int i, int nseg, int prev, int lim)
 {
     LegResult out;
-    leg_rest<true>(W, leg, voxel, seg, from, axis, i, nseg, prev, lim, out);
+    leg_rest<true>(leg, vi, from, axis, i, nseg, prev, lim, out);
     if (out.status)
-        atomicOr(W.desc->status, 1 << out.status);
+        atomicOr(warp_tab().desc->status, 1 << out.status);
     SlowLeg r;
     r.L = make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
     r.len = out.len;
@@ -1132,11 +1167,11 @@ __device__ __noinline__ SlowLeg leg_slow(const WarpTab &W, int leg, const short4
 
 // Displacement of increment i on the two non-step axes from the reference's
 // FP64 expression (a position near a rounding boundary, inside the volume).
-__device__ __forceinline__ void exact_displacement(const WarpTab &W, int leg, const HotRule &R, int axis,
-                                                   const short4 *voxel, int i, int &da, int &db)
+__device__ __forceinline__ void exact_displacement(int leg, int axis, int vi, int i, int &da, int &db)
 {
-    const short4 cv = __ldg(voxel);
-    const FaceRule &F = W.refl->rule[leg][R.face - 1];
+    const WarpTab &W = warp_tab();
+    const short4 cv = __ldg(W.coords + vi);
+    const FaceRule &F = W.refl->rule[leg][W.rule[leg][axis].face - 1];
     const int a = axis == 0 ? 1 : 0, b = axis == 2 ? 1 : 2;
     const int ca = axis == 0 ? cv.y : cv.x, cb = axis == 2 ? cv.y : cv.z;
     const double va = __dadd_rn((double)ca, __dmul_rn((double)i, F.q[a]));
@@ -1191,12 +1226,13 @@ __device__ __noinline__ int leg_limit(const FaceRule *R, int cz, int cy, int cx,
 // legs keep a voxel of room, the others their wall limit); the outer loop
 // takes that increment with the exact position.
 template <bool kBrick, class None, class Done, class Slow>
-__device__ __forceinline__ auto field_march(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, None none,
-                                            Done done, Slow slow)
+__device__ __forceinline__ auto field_march(int leg, int vi, None none, Done done, Slow slow)
 {
+    const WarpTab &W = warp_tab();
+    uint16_t *seg = seg_list();
     // the coordinates are loaded per leg (and again where they are rarely
     // needed) rather than kept across the march
-    const short4 cv = __ldg(voxel);
+    const short4 cv = __ldg(W.coords + vi);
     const int cz = cv.x, cy = cv.y, cx = cv.z;
     // ---- exit face: the smallest of the three distances n_a / |e_a| (n_a
     // exact, the estimates within 2^-22), when the next one is clearly larger
@@ -1256,7 +1292,7 @@ __device__ __forceinline__ auto field_march(const WarpTab &W, int leg, const sho
                 break;
             if (near) {
                 int da, db;
-                exact_displacement(W, leg, R, axis, voxel, i, da, db);
+                exact_displacement(leg, axis, vi, i, da, db);
                 b = field_byte<kBrick>(start, R, W.desc, axis, cz, cy, cx, i, da, db, dS, Sa, Sb);
                 if (b & 7u) {
                     take((int)(b & 7u));
@@ -1275,7 +1311,7 @@ __device__ __forceinline__ auto field_march(const WarpTab &W, int leg, const sho
             int da = fixed_at(last_i, qa_lo, qa_hi, off_a, fa);
             int db = fixed_at(last_i, qb_lo, qb_hi, off_b, fb);
             if (min(fa, fb) < 2u * kFieldMargin)
-                exact_displacement(W, leg, R, axis, voxel, last_i, da, db);
+                exact_displacement(leg, axis, vi, last_i, da, db);
             const int d0 = axis == 0 ? last_i : abs(da);
             const int d1 = axis == 1 ? last_i : (axis == 0 ? abs(da) : abs(db));
             const int d2 = axis == 2 ? last_i : abs(db);
@@ -1287,22 +1323,22 @@ __device__ __forceinline__ auto field_march(const WarpTab &W, int leg, const sho
     return slow(from, axis, i, nseg, prev, lim);
 }
 
-// One leg of one voxel: FP32 lengths (liquor, loop, crystal, bubble).
+// One leg of voxel vi of the item: FP32 lengths (liquor, loop, crystal, bubble).
 template <bool kBrick>
-__device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const short4 *voxel, uint16_t *seg, int &len)
+__device__ __forceinline__ float4 field_leg(int leg, int vi, int &len)
 {
     len = 1;
     return field_march<kBrick>(
-        W, leg, voxel, seg, [] { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); },
+        leg, vi, [] { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); },
         [&](int i, int nseg, int d0, int d1, int d2) {
             len = i;
             LegResult out;
             out.Lf[0] = out.Lf[1] = out.Lf[2] = out.Lf[3] = 0.0f;
-            lengths_f32(d0, d1, d2, i, nseg, seg, nullptr, W.voxel, out);
+            lengths_f32(d0, d1, d2, i, nseg, seg_list(), nullptr, warp_tab().voxel, out);
             return make_float4(out.Lf[0], out.Lf[1], out.Lf[2], out.Lf[3]);
         },
         [&](int from, int axis, int i, int nseg, int prev, int lim) {
-            const SlowLeg r = leg_slow(W, leg, voxel, seg, from, axis, i, nseg, prev, lim);
+            const SlowLeg r = leg_slow(leg, vi, from, axis, i, nseg, prev, lim);
             len = r.len;
             return r.L;
         });
@@ -1311,17 +1347,17 @@ __device__ __forceinline__ float4 field_leg(const WarpTab &W, int leg, const sho
 // A map value (cal_rate with a zero incident leg) of a leg
 // in the reference's FP64 operations: legs the march leaves, and values too
 // close to a rounding boundary of float.
-__device__ __noinline__ float map_slow(const WarpTab &W, const short4 *voxel, uint16_t *seg, int from, int axis, int i,
-                                       int nseg, int prev, int lim, int d0, int d1, int d2)
+__device__ __noinline__ float map_slow(int vi, int from, int axis, int i, int nseg, int prev, int lim, int d0, int d1,
+                                       int d2)
 {
-    const SampleDesc &D = *W.desc;
+    const SampleDesc &D = *warp_tab().desc;
     LegResult out;
     if (d0 >= 0) {   // marched to its stop: the lengths alone
         out.L[0] = out.L[1] = out.L[2] = out.L[3] = 0.0;
         out.status = kOk;
-        lengths_f64(d0, d1, d2, i, nseg, seg, D.voxel, D.sq, D.sq_stride, D.qtab, out);
+        lengths_f64(d0, d1, d2, i, nseg, seg_list(), D.voxel, D.sq, D.sq_stride, D.qtab, out);
     } else {
-        leg_rest<false>(W, 1, voxel, seg, from, axis, i, nseg, prev, lim, out);
+        leg_rest<false>(1, vi, from, axis, i, nseg, prev, lim, out);
     }
     if (out.status) {
         atomicOr(D.status, 1 << out.status);
@@ -1525,16 +1561,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks + 1) field_kernel(const Sam
                                                                    long long total_items,
                                                                    unsigned long long *__restrict__ work_counter)
 {
-    __shared__ WarpTab tabs[kWarps];
-    __shared__ uint16_t seg[kSegRows * kBlock];
-    __shared__ float4 incident[kBlock];
-    __shared__ float2 total[kBlock];   // compensated sums; in shared memory to leave the march its registers
-
     if (!block_shape_ok(n_desc > 0 ? descs[0].status : nullptr))
         return;
-    const int tid = threadIdx.x, lane = tid & 31;
-    WarpTab &W = tabs[tid >> 5];
+    FieldShared &S = field_shared();
     for (;;) {
+        const int lane = thread_now() & 31;
         unsigned long long it = 0;
         if (lane == 0)
             it = atomicAdd(work_counter, 1ull);
@@ -1554,46 +1585,49 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks + 1) field_kernel(const Sam
         const long long r = D.order ? (long long)__ldg(D.order + k) : k;
         const int t = (int)(local - k * D.tiles);
         __syncwarp();   // the previous item's reads of the table are done
-        fill_warp_tab(W, D.refl + r, D, lane);
+        fill_warp_tab(warp_tab(), D.refl + r, D, t, lane);
         __syncwarp();
 
-        total[tid] = make_float2(0.0f, 0.0f);
-        unsigned nsteps = 0;
-        const int n = min(D.tile, D.n_vox - t * D.tile);
-        const short4 *coords = D.coords + (long long)t * D.tile;
-        for (int vi = lane; vi < n; vi += 32) {
+        S.total[thread_now()] = make_float2(0.0f, 0.0f);
+        S.steps[thread_now()] = 0u;
+        for (int vi = lane; vi < warp_tab().n; vi += 32) {
             float4 L;
 #pragma unroll 1
             for (int leg = 0; leg < 2; leg++) {
                 int len;
-                L = field_leg<kBrick>(W, leg, coords + vi, seg + tid, len);
-                if (W.count_steps)
-                    nsteps += (unsigned)len;
-                // the incident leg's lengths wait in shared memory
+                L = field_leg<kBrick>(leg, vi, len);
+                const int tid = thread_now();
+                if (warp_tab().count_steps)
+                    S.steps[tid] += (unsigned)len;
                 if (leg == 0)
-                    incident[tid] = L;
+                    S.incident[tid] = L;
             }
             // L_incident + L_diffracted per class and cal_rate's exponent
             // (AnACor/src/ray_tracing_basic.c:1573-1576), in FP32
-            const float4 I = incident[tid];
+            const int tid = thread_now();
+            const WarpTab &W = warp_tab();
+            const float4 I = S.incident[tid];
             const float ex = W.mu[0] * (I.x + L.x) + W.mu[1] * (I.y + L.y) + W.mu[2] * (I.z + L.z) +
                              W.mu[3] * (I.w + L.w);
             const float term = W.is_exp ? expf(-ex) : ex;
-            const float2 sc = total[tid];
+            const float2 sc = S.total[tid];
             float ns, e;
             two_sum(sc.x, term, ns, e);
-            total[tid] = make_float2(ns, sc.y + e);
+            S.total[tid] = make_float2(ns, sc.y + e);
         }
         __syncwarp();
         if (D.steps) {
-            unsigned long long w = nsteps;
+            unsigned long long w = S.steps[thread_now()];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
                 w += __shfl_down_sync(kAll, w, o);
             if (lane == 0)
                 atomicAdd(D.steps, w);
         }
-        finish_warp_item(total[tid].x, total[tid].y, D, r, t, lane);
+        {
+            const float2 sc = S.total[thread_now()];
+            finish_warp_item(sc.x, sc.y, D, r, t, lane);
+        }
     }
 }
 
@@ -2040,7 +2074,7 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
         const long long refl = D.order ? (long long)__ldg(D.order + k) : k;
         const int t = (int)(local - k * D.tiles);
         __syncwarp();   // the previous item's reads of the table are done
-        fill_warp_tab(W, D.refl + refl, D, lane);
+        fill_warp_tab(W, D.refl + refl, D, t, lane);
         if (lane < 3)
             K[lane] = pair_of(__dmul_rn(D.voxel[lane], D.voxel[lane]));
         else if (lane < 7)
@@ -2204,14 +2238,12 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
                                                               float *__restrict__ out, long long ld,
                                                               const int *__restrict__ col)
 {
-    __shared__ WarpTab tabs[kWarps];
-    __shared__ uint16_t seg[kSegRows * kBlock];
-    __shared__ FloatPair consts[7];   // squared voxel edges (z, y, x), mu
+    FloatPair *consts = field_shared().consts;
     const SampleDesc &D = *dp;
     if (!block_shape_ok(D.status))
         return;
     const int tid = threadIdx.x, lane = tid & 31;
-    WarpTab &W = tabs[tid >> 5];
+    WarpTab &W = field_shared().tabs[tid >> 5];
     if (tid < 3)
         consts[tid] = pair_of(__dmul_rn(D.voxel[tid], D.voxel[tid]));
     else if (tid < 7)
@@ -2229,13 +2261,11 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
         const long long d = item / D.tiles;
         const int t = (int)(item - d * D.tiles);
         __syncwarp();   // the previous item's reads of the table are done
-        fill_warp_tab(W, D.refl + d, D, lane);
+        fill_warp_tab(W, D.refl + d, D, t, lane);
         __syncwarp();
-        const int n = min(D.tile, D.n_vox - t * D.tile);
-        const short4 *coords = D.coords + (long long)t * D.tile;
-        for (int vi = lane; vi < n; vi += 32) {
+        for (int vi = lane; vi < W.n; vi += 32) {
             const float val = field_march<false>(
-                W, 1, coords + vi, seg + tid, [&] { return W.is_exp ? 1.0f : 0.0f; },
+                1, vi, [&] { return W.is_exp ? 1.0f : 0.0f; },
                 [&](int i, int nseg, int d0, int d1, int d2) {
                     const FloatPair tot = pair_sqrt(
                         pair_add(pair_add(pair_mul(consts[0], (float)(d0 * d0)), pair_mul(consts[1], (float)(d1 * d1))),
@@ -2243,7 +2273,7 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
                     FloatPair sum = {0.0f, 0.0f};
                     int cur = 3 << 13;
                     for (int j = 1; j <= nseg; j++) {
-                        const int nxt = j < nseg ? (int)seg[j * kBlock + tid] : i;
+                        const int nxt = j < nseg ? (int)seg_list()[j * kBlock] : i;
                         const int cls = cur >> 13, span = (nxt & 0x1fff) - (cur & 0x1fff);
                         if (cls >= 1)
                             sum = pair_add(sum, pair_mul(consts[2 + cls], (float)span));
@@ -2267,10 +2297,10 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
                         sure = __fadd_rn(r.h, r.l + err) == r.h && __fadd_rn(r.h, r.l - err) == r.h && r.h > 0x1p-80f;
                     }
                     return positive && sure ? v
-                                            : map_slow(W, coords + vi, seg + tid, kFromStop, 0, i, nseg, 0, 0, d0, d1, d2);
+                                            : map_slow(vi, kFromStop, 0, i, nseg, 0, 0, d0, d1, d2);
                 },
                 [&](int from, int axis, int i, int nseg, int prev, int lim) {
-                    return map_slow(W, coords + vi, seg + tid, from, axis, i, nseg, prev, lim, -1, 0, 0);
+                    return map_slow(vi, from, axis, i, nseg, prev, lim, -1, 0, 0);
                 });
             const int k = t * D.tile + vi;
             out[d * ld + (col ? __ldg(col + k) : k)] = val;
@@ -2414,7 +2444,7 @@ cudaError_t launch_absorption(const SampleDesc *d_descs, int n_desc, long long t
     if (e != cudaSuccess)
         return e;
 #define ANACOR_COOP(B) absorption_kernel<B><<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter)
-#define ANACOR_FIELD(B, K) field_kernel<B, K><<<grid, kBlock, 0, st>>>(d_descs, n_desc, total_items, d_counter)
+#define ANACOR_FIELD(B, K) field_kernel<B, K><<<grid, kBlock, sizeof(FieldShared), st>>>(d_descs, n_desc, total_items, d_counter)
     switch (variant > 0 ? variant : absorption_variant()) {
     case 1: ANACOR_COOP(1); break;
     case 3: ANACOR_COOP(3); break;
@@ -2490,13 +2520,13 @@ cudaError_t launch_field_map(const SampleDesc *d_desc, long long total_items, un
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess)
         return e;
-    field_map_kernel<<<grid, kBlock, 0, st>>>(d_desc, total_items, d_counter, out, ld, col);
+    field_map_kernel<<<grid, kBlock, sizeof(FieldShared), st>>>(d_desc, total_items, d_counter, out, ld, col);
     return cudaGetLastError();
 }
 
 int field_map_occupancy(int *blocks_per_sm)
 {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, field_map_kernel, kBlock, 0) == cudaSuccess
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, field_map_kernel, kBlock, sizeof(FieldShared)) == cudaSuccess
                ? kOk
                : kErrCuda;
 }
@@ -2575,20 +2605,20 @@ int absorption_set_carveout(int pct)
 int absorption_occupancy(int *blocks_per_sm, int variant)
 {
     cudaError_t e;
-#define ANACOR_OCC(K) cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, K, kBlock, 0)
+#define ANACOR_OCC(K, S) cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, K, kBlock, S)
     switch (variant > 0 ? variant : absorption_variant()) {
-    case 1: e = ANACOR_OCC(absorption_kernel<1>); break;
-    case 3: e = ANACOR_OCC(absorption_kernel<3>); break;
-    case 4: e = ANACOR_OCC(absorption_kernel<4>); break;
-    case 5: e = ANACOR_OCC((field_kernel<1, false>)); break;
-    case 6: e = ANACOR_OCC((field_kernel<2, false>)); break;
-    case 7: e = ANACOR_OCC((field_kernel<3, false>)); break;
-    case 8: e = ANACOR_OCC((field_kernel<4, false>)); break;
-    case 9: e = ANACOR_OCC((field_kernel<1, true>)); break;
-    case 10: e = ANACOR_OCC((field_kernel<2, true>)); break;
-    case 11: e = ANACOR_OCC((field_kernel<3, true>)); break;
-    case 12: e = ANACOR_OCC((field_kernel<4, true>)); break;
-    default: e = ANACOR_OCC(absorption_kernel<2>); break;
+    case 1: e = ANACOR_OCC(absorption_kernel<1>, 0); break;
+    case 3: e = ANACOR_OCC(absorption_kernel<3>, 0); break;
+    case 4: e = ANACOR_OCC(absorption_kernel<4>, 0); break;
+    case 5: e = ANACOR_OCC((field_kernel<1, false>), sizeof(FieldShared)); break;
+    case 6: e = ANACOR_OCC((field_kernel<2, false>), sizeof(FieldShared)); break;
+    case 7: e = ANACOR_OCC((field_kernel<3, false>), sizeof(FieldShared)); break;
+    case 8: e = ANACOR_OCC((field_kernel<4, false>), sizeof(FieldShared)); break;
+    case 9: e = ANACOR_OCC((field_kernel<1, true>), sizeof(FieldShared)); break;
+    case 10: e = ANACOR_OCC((field_kernel<2, true>), sizeof(FieldShared)); break;
+    case 11: e = ANACOR_OCC((field_kernel<3, true>), sizeof(FieldShared)); break;
+    case 12: e = ANACOR_OCC((field_kernel<4, true>), sizeof(FieldShared)); break;
+    default: e = ANACOR_OCC(absorption_kernel<2>, 0); break;
     }
 #undef ANACOR_OCC
     return e == cudaSuccess ? kOk : kErrCuda;
