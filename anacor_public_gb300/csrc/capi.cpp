@@ -748,10 +748,13 @@ bool plan_field_bricked(const anacor_plan *p)
     return field_kind(p->variant) == 3 && p->field8b_state == 1;
 }
 
+// Items per reflection: as plan_split left them, or whole configured tiles.
+int tiles_of(const anacor_plan *p, bool whole) { return whole ? (p->n_vox + p->tile - 1) / p->tile : p->tiles; }
+
 // The plan's sample as a launch descriptor; fk >= 0 names the field it
 // marches on (0 none, 1 centred, 2 octant, 3 bricked octant; the field must be
 // built), else the field of the plan's own variant.
-SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1)
+SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1, bool whole = false)
 {
     SampleDesc d;
     std::memset(&d, 0, sizeof(d));
@@ -769,8 +772,8 @@ SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1)
     d.coords = p->d_coords;
     d.refl = p->d_refl;
     d.n_refl = p->n_refl;
-    d.tiles = p->tiles;
-    d.tile = p->work_tile;
+    d.tiles = tiles_of(p, whole);
+    d.tile = whole ? p->tile : p->work_tile;
     d.full_iteration = p->full;
     d.is_exp = p->is_exp;
     d.out = p->d_out;
@@ -1143,12 +1146,24 @@ struct anacor_batch {
 
 namespace {
 
+// Whether the samples of a launch give enough items without plan_split, which
+// counts one sample's only (six samples of 2,000 reflections: 4.09 ms in split
+// items, 4.02 whole; alone, each would be the slower for it).
+bool whole_items(anacor_plan *const *plans, size_t n)
+{
+    long long items = 0;
+    for (size_t i = 0; i < n; i++)
+        items += (long long)plans[i]->n_refl * tiles_of(plans[i], true);
+    return n > 0 && items >= wanted_items(plans[0]);
+}
+
 // The batch's samples as descriptors.  Under a field variant every sample
 // marches on its field of that kind (built here if needed), so the batch is
 // one launch; a sample whose labels allow no field (outside 0..7) runs in a
 // first, cooperative launch of the same register budget.
 int batch_upload(anacor_batch *b)
 {
+    const bool whole = whole_items(b->plans.data(), b->plans.size());
     std::vector<anacor_plan *> coop, field;
     const int fk = field_kind(b->variant);
     for (anacor_plan *p : b->plans) {
@@ -1167,15 +1182,15 @@ int batch_upload(anacor_batch *b)
     std::vector<SampleDesc> descs, descs_field;
     long long total = 0, items_coop = 0;
     for (anacor_plan *p : coop) {
-        descs.push_back(plan_desc(p, total, 0));
-        total += (long long)p->n_refl * p->tiles;
+        descs.push_back(plan_desc(p, total, 0, whole));
+        total += (long long)p->n_refl * tiles_of(p, whole);
     }
     items_coop = total;
     long long rebased = 0;
     for (anacor_plan *p : field) {
-        descs.push_back(plan_desc(p, total, fk));
-        descs_field.push_back(plan_desc(p, rebased, fk));
-        const long long n = (long long)p->n_refl * p->tiles;
+        descs.push_back(plan_desc(p, total, fk, whole));
+        descs_field.push_back(plan_desc(p, rebased, fk, whole));
+        const long long n = (long long)p->n_refl * tiles_of(p, whole);
         total += n;
         rebased += n;
     }
@@ -1566,11 +1581,13 @@ int anacor_batch_run(anacor_plan *const *plans, int n_plans, void *stream)
     cudaStream_t st = stream ? (cudaStream_t)stream : p0->stream;
     std::vector<SampleDesc> descs;
     long long total = 0;
-    for (int i = 0; i < n_plans; i++) {
+    for (int i = 0; i < n_plans; i++)
         if (!plans[i])
             return fail(kErrArgs, "null plan in batch");
-        descs.push_back(plan_desc(plans[i], total));
-        total += (long long)plans[i]->n_refl * plans[i]->tiles;
+    const bool whole = whole_items(plans, (size_t)n_plans);
+    for (int i = 0; i < n_plans; i++) {
+        descs.push_back(plan_desc(plans[i], total, -1, whole));
+        total += (long long)plans[i]->n_refl * tiles_of(plans[i], whole);
     }
     // batch descriptors live in a device buffer owned by the first plan's device state
     static thread_local SampleDesc *d_descs = nullptr;
