@@ -224,12 +224,17 @@ const int8_t *flat_base(int8_t ***table, const int64_t *shape)
         return nullptr;
     const int8_t *base = table[0][0];
     const int64_t Y = shape[1], X = shape[2];
+    uintptr_t expect = (uintptr_t)base;
     for (int64_t z = 0; z < shape[0]; z++) {
         if (!table[z])
             return nullptr;
+        // a plane's rows without an exit in between: the loop is a vector one
+        uintptr_t bad = 0;
         for (int64_t y = 0; y < Y; y++)
-            if (table[z][y] != base + (z * Y + y) * X)
-                return nullptr;
+            bad |= (uintptr_t)table[z][y] ^ (expect + (uintptr_t)(y * X));
+        if (bad)
+            return nullptr;
+        expect += (uintptr_t)(Y * X);
     }
     return base;
 }
@@ -286,6 +291,14 @@ struct anacor_plan {
     uint8_t *d_field8b = nullptr;  // the same in 4^3 bricks, built on first use by variants 13..16
     int field8b_state = 0;
     int *d_walls = nullptr;        // [6] room between the non-vacuum labels and the walls, built with a field
+    // One allocation each: status, counter, descriptor and squared lengths;
+    // and what is sized by the reflections (tables, results, arrivals, order).
+    uint8_t *d_fixed = nullptr, *d_per_refl = nullptr;
+    // A plan that lives for one call.  What it uploads is the caller's or lies
+    // in the calling thread's staging, both of which outlast the call, so the
+    // only synchronisation is the one that fetches the result.
+    bool once = false;
+    bool idle = false;             // fetched: nothing of the plan's is in flight
 };
 
 namespace {
@@ -295,25 +308,20 @@ void plan_release(anacor_plan *p)
     cudaStream_t st = p->stream;
     dev_free(p->d_vol, st);
     dev_free(p->d_coords, st);
-    dev_free(p->d_refl, st);
-    dev_free(p->d_out, st);
+    dev_free(p->d_per_refl, st);
     dev_free(p->d_partial, st);
-    dev_free(p->d_arrive, st);
-    dev_free(p->d_status, st);
-    dev_free(p->d_counter, st);
-    dev_free(p->d_desc, st);
+    dev_free(p->d_fixed, st);
     dev_free(p->d_steps, st);
-    dev_free(p->d_sq, st);
     dev_free(p->d_c64, st);
     dev_free(p->d_field, st);
     dev_free(p->d_field8, st);
     dev_free(p->d_field8b, st);
     dev_free(p->d_walls, st);
-    dev_free(p->d_order, st);
     if (p->h_refl && !p->h_refl_borrowed)
         cudaFreeHost(p->h_refl);
     p->h_refl = nullptr;
-    cudaStreamSynchronize(st);
+    if (!(p->once && p->idle))
+        cudaStreamSynchronize(st);
 }
 
 // True when p lies in page-locked host memory (cudaHostAlloc'd or registered).
@@ -355,6 +363,46 @@ ReflTable *thread_staging(int64_t n_refl)
         s.cap = cap;
     }
     return s.p;
+}
+
+// The calling thread's staging for small transfers: a plan's fixed block, its
+// descriptor, its status and results.  Page-locked, because a copy from or to
+// pageable memory costs about 10 us more than its bytes and a result waits
+// for each such copy; half a megabyte a thread, given back when it ends.
+struct SmallStaging {
+    static constexpr size_t kFixed = 256 << 10, kDesc = 4096, kStatus = 256, kResults = 32768;
+    uint8_t *p = nullptr;
+    bool pinned = false;
+    ~SmallStaging()
+    {
+        if (pinned)
+            cudaFreeHost(p);
+        else
+            std::free(p);
+    }
+    bool ready()
+    {
+        if (!p) {
+            const size_t bytes = kFixed + kDesc + kStatus + kResults * sizeof(double);
+            pinned = cudaMallocHost(reinterpret_cast<void **>(&p), bytes) == cudaSuccess;
+            if (!pinned) {
+                cudaGetLastError();
+                p = static_cast<uint8_t *>(std::malloc(bytes));   // slower, as good
+            }
+        }
+        return p != nullptr;
+    }
+    uint8_t *fixed() { return p; }
+    SampleDesc *desc() { return reinterpret_cast<SampleDesc *>(p + kFixed); }
+    int *status() { return reinterpret_cast<int *>(p + kFixed + kDesc); }
+    double *results() { return reinterpret_cast<double *>(p + kFixed + kDesc + kStatus); }
+};
+static_assert(sizeof(SampleDesc) <= SmallStaging::kDesc, "descriptor staging");
+
+SmallStaging &small_staging()
+{
+    static thread_local SmallStaging s;
+    return s;
 }
 
 // A helper thread per calling thread, kept between calls, for the
@@ -506,24 +554,34 @@ int plan_init_volume(anacor_plan *p, const int8_t *label, const int64_t *shape, 
     cudaStream_t st = p->stream;
     const size_t nvol = (size_t)shape[0] * shape[1] * shape[2];
     cudaError_t e;
-    if ((e = dev_alloc(&p->d_vol, nvol, st)) != cudaSuccess || (e = dev_alloc(&p->d_status, 1, st)) ||
-        (e = dev_alloc(&p->d_counter, 1, st)) || (e = dev_alloc(&p->d_desc, 1, st)))
+    // the fixed block: status, counter, descriptor, squared lengths
+    constexpr size_t kCounterAt = 128, kDescAt = 256;
+    constexpr size_t kSqAt = kDescAt + (sizeof(SampleDesc) + 255) / 256 * 256;
+    static_assert(kSqAt + 3 * sizeof(double) * kMaxDim <= SmallStaging::kFixed, "fixed block staging");
+    p->sq_stride = std::max(p->dims[0], std::max(p->dims[1], p->dims[2]));
+    const size_t fixed_bytes = kSqAt + (size_t)3 * p->sq_stride * sizeof(double);
+    SmallStaging &host = small_staging();
+    if (!host.ready())
+        return fail(kErrNoMem, "out of host memory");
+    if ((e = dev_alloc(&p->d_vol, nvol, st)) != cudaSuccess || (e = dev_alloc(&p->d_fixed, fixed_bytes, st)))
         return cuda_fail(e, "device allocation");
-    if ((e = cudaMemcpyAsync(p->d_vol, label, nvol, cudaMemcpyHostToDevice, st)) ||
-        (e = cudaMemsetAsync(p->d_status, 0, sizeof(int), st)))
+    p->d_status = reinterpret_cast<int *>(p->d_fixed);
+    p->d_counter = reinterpret_cast<unsigned long long *>(p->d_fixed + kCounterAt);
+    p->d_desc = reinterpret_cast<SampleDesc *>(p->d_fixed + kDescAt);
+    p->d_sq = reinterpret_cast<double *>(p->d_fixed + kSqAt);
+    if ((e = cudaMemcpyAsync(p->d_vol, label, nvol, cudaMemcpyHostToDevice, st)))
         return cuda_fail(e, "volume upload");
     // squared axis lengths for cal_path2_plus's total, as the reference
     // computes them: pow((last - first) * voxel, 2) == t * t, t = d * voxel
-    p->sq_stride = std::max(p->dims[0], std::max(p->dims[1], p->dims[2]));
-    std::vector<double> sq((size_t)3 * p->sq_stride, 0.0);
+    std::memset(host.fixed(), 0, kSqAt);
+    double *sq = reinterpret_cast<double *>(host.fixed() + kSqAt);
     for (int a = 0; a < 3; a++)
-        for (int d = 0; d < p->dims[a]; d++) {
+        for (int d = 0; d < p->sq_stride; d++) {
             const double t = (double)d * voxel[a];
-            sq[(size_t)a * p->sq_stride + d] = t * t;
+            sq[(size_t)a * p->sq_stride + d] = d < p->dims[a] ? t * t : 0.0;
         }
-    if ((e = dev_alloc(&p->d_sq, sq.size(), st)) ||
-        (e = cudaMemcpyAsync(p->d_sq, sq.data(), sq.size() * sizeof(double), cudaMemcpyHostToDevice, st)) ||
-        (e = cudaStreamSynchronize(st)))
+    if ((e = cudaMemcpyAsync(p->d_fixed, host.fixed(), fixed_bytes, cudaMemcpyHostToDevice, st)) ||
+        (!p->once && (e = cudaStreamSynchronize(st))))
         return cuda_fail(e, "table upload");
     p->d_qtab = quotient_table(dev, p->sq_stride);
     return kOk;
@@ -551,7 +609,7 @@ int plan_set_voxels(anacor_plan *p, const int64_t *coords, int64_t n, bool on_de
         if ((e = cudaMemcpyAsync(p->d_c64, coords, (size_t)n * 3 * sizeof(long long),
                                  on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st)) ||
             (e = launch_pack_coords_order(p->d_c64, (int)n, p->dims, p->order, p->d_coords, p->d_status, st)) ||
-            (e = cudaStreamSynchronize(st)))
+            (!p->once && (e = cudaStreamSynchronize(st))))
             return cuda_fail(e, "coordinate upload");
     }
     return kOk;
@@ -642,20 +700,22 @@ int plan_reserve_refl(anacor_plan *p, int64_t n_refl)
     cudaStream_t st = p->stream;
     cudaError_t e;
     if (n_refl > p->refl_cap) {
-        dev_free(p->d_refl, st);
-        dev_free(p->d_out, st);
+        dev_free(p->d_per_refl, st);
         dev_free(p->d_partial, st);
-        dev_free(p->d_arrive, st);
-        dev_free(p->d_order, st);
         if (p->h_refl && !p->h_refl_borrowed) {
             cudaStreamSynchronize(st);
             cudaFreeHost(p->h_refl);
             p->h_refl = nullptr;
         }
         p->partial_cap = 0;
-        if ((e = dev_alloc(&p->d_refl, (size_t)n_refl, st)) || (e = dev_alloc(&p->d_out, (size_t)n_refl, st)) ||
-            (e = dev_alloc(&p->d_arrive, (size_t)n_refl, st)) || (e = dev_alloc(&p->d_order, (size_t)n_refl, st)))
+        p->refl_cap = p->n_refl = 0;
+        const size_t n = (size_t)n_refl;
+        if ((e = dev_alloc(&p->d_per_refl, n * (sizeof(ReflTable) + sizeof(double) + 2 * sizeof(int)), st)))
             return cuda_fail(e, "device allocation");
+        p->d_refl = reinterpret_cast<ReflTable *>(p->d_per_refl);
+        p->d_out = reinterpret_cast<double *>(p->d_refl + n);
+        p->d_arrive = reinterpret_cast<unsigned *>(p->d_out + n);
+        p->d_order = reinterpret_cast<int *>(p->d_arrive + n);
         if ((e = cudaMemsetAsync(p->d_arrive, 0, (size_t)n_refl * sizeof(unsigned), st)))
             return cuda_fail(e, "cudaMemset");
         if (!p->h_refl_borrowed &&
@@ -808,12 +868,17 @@ SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1, bo
 int plan_upload_desc(anacor_plan *p, unsigned long long *steps)
 {
     cudaError_t e;
-    SampleDesc d = plan_desc(p, 0);
-    d.steps = steps;
-    if ((e = cudaMemcpyAsync(p->d_desc, &d, sizeof(d), cudaMemcpyHostToDevice, p->stream)))
+    SmallStaging &host = small_staging();
+    if (!host.ready())
+        return fail(kErrNoMem, "out of host memory");
+    SampleDesc *d = host.desc();
+    *d = plan_desc(p, 0);
+    d->steps = steps;
+    if ((e = cudaMemcpyAsync(p->d_desc, d, sizeof(*d), cudaMemcpyHostToDevice, p->stream)))
         return cuda_fail(e, "descriptor upload");
-    // the descriptor lives on the stack: make sure it has been read
-    if ((e = cudaStreamSynchronize(p->stream)))
+    // the staging's next user may be another plan, on another stream; a plan
+    // of one call uploads its descriptor once
+    if (!p->once && (e = cudaStreamSynchronize(p->stream)))
         return cuda_fail(e, "upload");
     return kOk;
 }
@@ -871,14 +936,20 @@ int plan_launch(anacor_plan *p, cudaStream_t st)
 
 int plan_fetch(anacor_plan *p, double *out, cudaStream_t st)
 {
-    int status = 0;
     cudaError_t e;
-    if (p->n_refl > 0 && p->n_vox > 0 &&
-        (e = cudaMemcpyAsync(out, p->d_out, (size_t)p->n_refl * sizeof(double), cudaMemcpyDeviceToHost, st)))
-        return cuda_fail(e, "result download");
-    if ((e = cudaMemcpyAsync(&status, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
+    SmallStaging &host = small_staging();
+    if (!host.ready())
+        return fail(kErrNoMem, "out of host memory");
+    const bool any = p->n_refl > 0 && p->n_vox > 0, staged = (size_t)p->n_refl <= SmallStaging::kResults;
+    if ((any && (e = cudaMemcpyAsync(staged ? host.results() : out, p->d_out, (size_t)p->n_refl * sizeof(double),
+                                     cudaMemcpyDeviceToHost, st))) ||
+        (e = cudaMemcpyAsync(host.status(), p->d_status, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
         (e = cudaStreamSynchronize(st)))
         return cuda_fail(e, "result download");
+    p->idle = true;
+    const int status = *host.status();
+    if (any && staged)
+        std::memcpy(out, host.results(), (size_t)p->n_refl * sizeof(double));
     if (p->n_vox == 0)
         for (int64_t i = 0; i < p->n_refl; i++)
             out[i] = std::nan("");   // the reference's 0/0 mean
@@ -921,8 +992,9 @@ int run_once(const int8_t *flat, const int64_t *shape, const int64_t *coords, in
     // The reflections' host set-up (FP64 rotation, angles, face rules) does
     // not depend on the device: it runs on this thread's helper while this
     // one uploads the volume and voxels and builds the march's fields.
+    // (A few are done here before the helper would have woken: 0.8 us each.)
     static thread_local SetupHelper helper;
-    const bool on_helper = staged && !tables && helper.submit([=] {
+    const bool on_helper = staged && !tables && n_refl > 16 && helper.submit([=] {
         return setup_reflections(axis, omega, F, xray, s1, n_refl, staged, threads);
     });
     // A volume in pageable memory is page-locked for the upload (about 0.2 ms
@@ -946,10 +1018,10 @@ int run_once(const int8_t *flat, const int64_t *shape, const int64_t *coords, in
         }
     }
     anacor_plan p;
+    p.once = true;
     int st = plan_init(&p, flat, shape, coords, n, voxel, mu, full, is_exp);
     if (registered) {
-        // plan_init synchronised its stream: the volume is on the device
-        cudaStreamSynchronize(p.stream);
+        cudaStreamSynchronize(p.stream);   // the volume is on the device
         cudaHostUnregister(const_cast<int8_t *>(flat));
         cudaGetLastError();
     }
@@ -1010,7 +1082,7 @@ int plan_configure(anacor_plan *p, int variant, int tile, int order)
             return st;
     }
     p->variant = variant;
-    return plan_upload_desc(p, nullptr);
+    return p->once ? kOk : plan_upload_desc(p, nullptr);   // once: with the tables
 }
 
 // Time `reps` launches over the first k reflections of the plan (ms each).
@@ -1254,14 +1326,23 @@ int batch_kernels(const anacor_batch *b)
 int batch_check(anacor_batch *b, cudaStream_t st)
 {
     cudaError_t e;
-    for (anacor_plan *p : b->plans) {
-        int status = 0;
-        if ((e = cudaMemcpyAsync(&status, p->d_status, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
-            (e = cudaStreamSynchronize(st)))
+    SmallStaging &host = small_staging();
+    if (!host.ready())
+        return fail(kErrNoMem, "out of host memory");
+    // the samples' status words together, one wait for as many as fit
+    constexpr size_t kWords = SmallStaging::kStatus / sizeof(int);
+    for (size_t k = 0; k < b->plans.size(); k += kWords) {
+        const size_t m = std::min(kWords, b->plans.size() - k);
+        for (size_t j = 0; j < m; j++)
+            if ((e = cudaMemcpyAsync(host.status() + j, b->plans[k + j]->d_status, sizeof(int),
+                                     cudaMemcpyDeviceToHost, st)))
+                return cuda_fail(e, "status");
+        if ((e = cudaStreamSynchronize(st)))
             return cuda_fail(e, "status");
-        for (int bit = 1; bit < 16; bit++)
-            if (status & (1 << bit))
-                return fail(bit, status_text(bit));
+        for (size_t j = 0; j < m; j++)
+            for (int bit = 1; bit < 16; bit++)
+                if (host.status()[j] & (1 << bit))
+                    return fail(bit, status_text(bit));
     }
     return succeed();
 }

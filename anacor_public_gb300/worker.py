@@ -31,14 +31,16 @@ def python_2_c_3d(label_list: np.ndarray):
         raise ValueError("label_list must be a C-contiguous int8 array")
     Z, Y, X = label_list.shape
     base = label_list.ctypes.data
-    ptr_size = ct.sizeof(ct.c_void_p)
-    rows = (ct.c_void_p * (Z * Y))()
-    addr = base + np.arange(Z * Y, dtype=np.uint64) * np.uint64(X)
-    ct.memmove(rows, addr.astype(np.uint64).tobytes(), Z * Y * ptr_size)
-    planes = (ct.c_void_p * Z)()
-    paddr = np.uint64(ct.addressof(rows)) + np.arange(Z, dtype=np.uint64) * np.uint64(Y * ptr_size)
-    ct.memmove(planes, paddr.astype(np.uint64).tobytes(), Z * ptr_size)
-    return ct.cast(planes, ct.POINTER(ct.POINTER(ct.POINTER(ct.c_int8)))), (rows, planes, label_list)
+    rows = np.arange(Z * Y, dtype=np.uintp)   # one array written in place: the table of a large volume is megabytes
+    rows *= X
+    rows += base
+    planes = np.arange(Z, dtype=np.uintp)
+    planes *= Y * rows.itemsize
+    planes += rows.ctypes.data
+    return ct.cast(planes.ctypes.data, _ROW_TABLE), (rows, planes, label_list)
+
+
+_ROW_TABLE = ct.POINTER(ct.POINTER(ct.POINTER(ct.c_int8)))
 
 
 def kp_rotation(axis, theta):
