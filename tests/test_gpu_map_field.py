@@ -70,3 +70,42 @@ def test_bilinear_counts(n_vox, n_refl):
         assert abs(got[i] - want) <= 5e-7 * want
     g.close()
     plan.close()
+
+
+def test_map_ties_and_launch_groups():
+    """Whole-degree directions on the diagonals of a cube (exit-face ties), in
+    a map of enough directions for several uploads and launches: bit for bit,
+    around the lines between them too."""
+    lab = np.zeros((34, 34, 34), np.int8)
+    lab[3:31, 3:31, 3:31] = 3
+    lab[8:20, 10:25, 6:30] = 1
+    a = np.arange(4, 30, 2)
+    coords = np.concatenate([np.stack([a, a, a], 1), np.stack([a, a, 34 - a], 1), np.stack([a, 34 - a, a], 1),
+                             np.stack([a, a + 0 * a, 17 + 0 * a], 1)]).astype(np.int64)
+    vox, mu = np.array([0.3, 0.3, 0.3]), np.array([0.01, 0.007, 0.012, 0.0])
+    plan = tracer.Plan(lab, np.ascontiguousarray(coords), vox, mu)
+    g = gridding.GriddingMap(plan, 240, 120, 2).build()   # 28,800 directions, 1.5 degrees
+    m = g.map()
+    s1, _, _ = gridding.directions(240, 120)
+    o = Oracle()
+    ties = [ip * 240 + it for ip in (0, 30, 60, 90) for it in range(0, 240, 30)]
+    for d in ties + [4095, 4096, 4097, 20479, 20480, 28799]:
+        det = o.leg_detail(coords, s1[d], s1[d], vox, lab)
+        if (det["status"][:, 1] != 0).any():
+            continue
+        assert np.array_equal(m[d], go.map_value(det["L"][:, 1, :], mu, 0)), d
+    g.close()
+    plan.close()
+
+
+def test_lookups_in_chunks():
+    """A call with more lookups than the staging holds equals its parts."""
+    s = synth.small_sample(n_refl=61)
+    plan = tracer.Plan(s.label, s.coords[:40], s.voxel, s.mu)
+    g = gridding.GriddingMap(plan, 36, 18, 2).build()
+    s1, om = np.tile(s.s1, (960, 1)), np.tile(s.omega, 960)   # 58,560
+    whole = g.interpolate(s1, om, s.xray, s.omega_axis, s.F, method="linear")
+    part = g.interpolate(s.s1, s.omega, s.xray, s.omega_axis, s.F, method="linear")
+    assert np.array_equal(whole, np.tile(part, 960))
+    g.close()
+    plan.close()
