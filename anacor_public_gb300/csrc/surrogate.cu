@@ -951,7 +951,7 @@ cudaError_t train_init(int dev)
     std::call_once(g_train_once[dev], [dev] {
         cudaError_t e = cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
         if (!e)
-            e = cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwSmem);
+            e = cudaFuncSetAttribute(update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem);
         g_train_init_err[dev] = e;
     });
     return g_train_init_err[dev];
@@ -981,10 +981,10 @@ struct anacor_surrogate {
     // training workspace for `train_rows` rows per member (see surrogate_train.cuh)
     int train_rows = 0;
     uint4 *X0i = nullptr, *Ai[kDepth] = {}, *dHi[kDepth] = {};
-    float4 *Hi[2] = {}, *part = nullptr;
+    float4 *Hi[2] = {};
     float *ty = nullptr, *dy = nullptr;
     float *loss_acc = nullptr;              // zero between steps
-    unsigned *step = nullptr;
+    unsigned *step = nullptr, *ticket = nullptr;   // steps taken; blocks of a step that have read it
     float *loss_hist = nullptr;
     int hist_len = 0;
     int *err = nullptr;
@@ -1036,7 +1036,7 @@ void free_train(anacor_surrogate *s)
     for (int l = 0; l < kDepth; l++) {
         dfree(s->Ai[l]); dfree(s->dHi[l]);
     }
-    dfree(s->Hi[0]); dfree(s->Hi[1]); dfree(s->part); dfree(s->ty); dfree(s->dy);
+    dfree(s->Hi[0]); dfree(s->Hi[1]); dfree(s->ty); dfree(s->dy);
     s->train_rows = 0;
 }
 
@@ -1072,7 +1072,7 @@ int ensure_train(anacor_surrogate *s, int rows)
     free_train(s);
     const size_t E = s->E, R = rows;
     bool ok = !dalloc(&s->X0i, E * R * kFeat / 8) && !dalloc(&s->ty, E * R) && !dalloc(&s->dy, E * R) &&
-              !dalloc(&s->part, E * (size_t)kPartFloats / 4) && !dalloc(&s->Hi[0], E * R * kWidth / 4) &&
+              !dalloc(&s->Hi[0], E * R * kWidth / 4) &&
               !dalloc(&s->Hi[1], E * R * kWidth / 4);
     for (int l = 0; l < kDepth && ok; l++)
         ok = !dalloc(&s->Ai[l], E * R * kWidth / 8) && !dalloc(&s->dHi[l], E * R * kWidth / 8);
@@ -1177,27 +1177,13 @@ cudaError_t train_step(anacor_surrogate *s, const bf16 *feat, const float *targe
     c.loss_acc = s->loss_acc;
     c.err = s->err;
     const int units = s->train_rows / kTileRows * s->E;
-    chain_kernel<<<std::min(units, sms), kInferThreads, kChainSmem, st>>>(c);
-    DwArgs d{};
-    d.X0 = s->X0i;
+    chain_kernel<<<std::min(units, sms), kChainThreads, kChainSmem, st>>>(c);
     UpdateArgs u{};
+    u.X0 = s->X0i;
     for (int l = 0; l < kDepth; l++) {
-        d.A[l] = s->Ai[l];
-        d.dH[l] = s->dHi[l];
+        u.A[l] = s->Ai[l];
         u.dH[l] = s->dHi[l];
     }
-    d.batch = s->train_rows;
-    d.part = s->part;
-    d.step = s->step;
-    d.loss_acc = s->loss_acc;
-    d.loss_hist = s->loss_hist;
-    d.E = s->E;
-    d.hist_len = s->hist_len;
-    d.count_step = update;
-    d.err = s->err;
-    dw_kernel<<<dim3(2 * kSplitK * kDepth, s->E), kDwThreads, kDwSmem, st>>>(d);
-    u.part = s->part;
-    u.A3 = s->Ai[kDepth - 1];
     u.dy = s->dy;
     u.batch = s->train_rows;
     u.E = s->E;
@@ -1205,11 +1191,20 @@ cudaError_t train_step(anacor_surrogate *s, const bf16 *feat, const float *targe
     u.m = s->m;
     u.v = s->v;
     u.grad = s->grad;
-    u.step = s->step;
     u.adam = s->adam;
     u.update = update;
     u.copies = weight_copies(s);
-    update_kernel<<<dim3(kPatches + kVectors, s->E), 256, 0, st>>>(u);
+    u.step = s->step;
+    u.ticket = s->ticket;
+    u.loss_acc = s->loss_acc;
+    u.loss_hist = s->loss_hist;
+    u.hist_len = s->hist_len;
+    u.err = s->err;
+    // the column sums take the SMs that the tiles' last wave leaves, or a wave
+    // of their own where these are few (one block too many is a wave more: 6 us)
+    const int grad_tiles = s->E * kGradTiles, left = sms - grad_tiles % sms;
+    const int sums = std::min(s->E * kVectors, left < sms / 4 ? left + sms : left);
+    update_kernel<<<grad_tiles + sums, kGradThreads, kGradSmem, st>>>(u);
     return cudaGetLastError();
 }
 
@@ -1283,7 +1278,7 @@ anacor_surrogate *anacor_surrogate_create(int n_members, uint32_t seed, float fo
     const size_t np = (size_t)kParams * n_members;
     bool ok = !cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) && !dalloc(&s->params, np) &&
               !dalloc(&s->m, np) && !dalloc(&s->v, np) && !dalloc(&s->grad, np) && !dalloc(&s->Bf, 32 * kIn) &&
-              !dalloc(&s->loss_acc, 16) && !dalloc(&s->step, 1) && !dalloc(&s->err, 1) &&
+              !dalloc(&s->loss_acc, 16) && !dalloc(&s->step, 1) && !dalloc(&s->ticket, 1) && !dalloc(&s->err, 1) &&
               !dalloc(&s->wimg, (size_t)n_members * kChunksPerMember * kChunkBytes) &&
               !dalloc(&s->wtimg, (size_t)n_members * kChunksBack * kChunkBytes);
     for (int l = 0; l < kDepth && ok; l++) {
@@ -1302,6 +1297,7 @@ anacor_surrogate *anacor_surrogate_create(int n_members, uint32_t seed, float fo
     if (ok && ((e = cudaMemcpy(s->params, p.data(), np * sizeof(float), cudaMemcpyHostToDevice)) ||
                (e = cudaMemset(s->m, 0, np * sizeof(float))) || (e = cudaMemset(s->v, 0, np * sizeof(float))) ||
                (e = cudaMemset(s->grad, 0, np * sizeof(float))) || (e = cudaMemset(s->step, 0, sizeof(unsigned))) ||
+               (e = cudaMemset(s->ticket, 0, sizeof(unsigned))) ||
                (e = cudaMemset(s->err, 0, sizeof(int))) || (e = cudaMemset(s->loss_acc, 0, 16 * sizeof(float))) ||
                (e = cudaMemcpy(s->Bf, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice)) ||
                (e = convert_all(s, s->st)) || (e = cudaStreamSynchronize(s->st))))
@@ -1327,7 +1323,7 @@ void anacor_surrogate_destroy(anacor_surrogate *s)
     free_work(s);
     free_train(s);
     dfree(s->params); dfree(s->m); dfree(s->v); dfree(s->grad); dfree(s->Bf);
-    dfree(s->loss_acc); dfree(s->step); dfree(s->err); dfree(s->loss_hist); dfree(s->wimg); dfree(s->wtimg);
+    dfree(s->loss_acc); dfree(s->step); dfree(s->ticket); dfree(s->err); dfree(s->loss_hist); dfree(s->wimg); dfree(s->wtimg);
     dfree(s->target); dfree(s->feat);
     for (int l = 0; l < kDepth; l++) {
         dfree(s->W[l]);

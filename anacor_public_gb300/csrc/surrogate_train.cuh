@@ -1,18 +1,18 @@
-// One training step of the surrogate as three kernels.  Included by
+// One training step of the surrogate as two kernels.  Included by
 // surrogate.cu after the fused inference kernel, whose helpers it uses.
 //
 //   chain_kernel   a 128-row tile of one member's batch: gather, the four
 //                  forward layers, head and loss, and the three backward
 //                  products dH_{l-1} = (dH_l W_l) gelu'(H_{l-1}), all of which
 //                  need the tile's own rows only;
-//   dw_kernel      the weight gradients dH_l^T A_{l-1}, K-split over the rows;
-//   update_kernel  sums of the splits and of the biases, Adam, and the BF16
-//                  weights in the layouts the products read.
+//   update_kernel  the weight gradients dH_l^T A_{l-1} and the sums for the
+//                  biases, Adam, and the BF16 weights in the layouts the
+//                  products read.
 //
 // Step by step (a GEMM per layer and direction, transposed copies, sums,
 // Adam, conversions: 40 launches) it took 411 us for four members at a batch
 // of 4,096.  The numbers are the same: every product accumulates over the same
-// K order, the splits and column sums are added in the same order and the
+// K order, the K splits and column sums are added in the same order and the
 // BF16 roundings are the same.
 //
 // Activations and gradients leave the chain only as "row images" for the dW
@@ -58,8 +58,11 @@ struct ChainArgs {
 constexpr int kOffChainAct = 8 * kChunkBytes;                     // eight weight stages: a whole layer
 constexpr int kOffChainX0 = kOffChainAct + kActBytes;
 constexpr int kOffChainDy = kOffChainX0 + kActChunk;
-constexpr int kChainSmem = kOffChainDy + kTileRows * 4;
+constexpr int kOffChainVec = kOffChainDy + kTileRows * 4;          // a unit's biases and output weights, two units
+constexpr int kVecFloats = (kDepth + 1) * kWidth;
+constexpr int kChainSmem = kOffChainVec + 2 * kVecFloats * 4;
 constexpr int kChainStages = 8;
+constexpr int kActChunks = kWidth / umma::kBK;                    // 64-column chunks of an operand
 static_assert(kChainSmem + 512 <= 227 * 1024, "chain kernel shared memory");
 constexpr int kChainJobs = 2 * kDepth - 1;                        // four forward, three backward products
 
@@ -72,10 +75,21 @@ __device__ __forceinline__ long long drawn_row(const ChainArgs &a, unsigned step
     return (long long)(((uint64_t)h * (uint64_t)a.n_data) >> 32);
 }
 
-__global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
+// Bound by the epilogues, one after the other: a layer's 32,768 values a tile
+// take 8 to 12 thousand cycles (issue 55 % busy meanwhile, the pre-activations'
+// 128 KB a layer to L2 and back, values that the rounding test leaves open in
+// one warp or other), its product 2 to 4.5 thousand, of which the first
+// three quarters run beside the epilogue before it where the accumulator is
+// free.  Four members, a batch of 4,096 (128 tiles): 64.6 us with a product
+// waiting for its whole operand, biases from L2 for every 16 columns and the
+// pre-activations fetched where they are used; 58 us so.  (Two accumulator
+// pieces in flight a warp spill: 96 registers are all that 18 warps leave.)
+constexpr int kChainThreads = 32 * (kEpiWarps + 2);                // the epilogue's, MMA, copy
+
+__global__ void __launch_bounds__(kChainThreads, 1) chain_kernel(ChainArgs a)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t full[kChainStages], empty[kChainStages], acc_full, act_ready, x0_ready;
+    __shared__ uint64_t full[kChainStages], empty[kChainStages], acc_full, act_ready[kActChunks], x0_ready;
     __shared__ uint32_t tslot;
     __shared__ int s_abort;
     uint8_t *Ws = smem, *Act = smem + kOffChainAct, *X0s = smem + kOffChainX0;
@@ -91,7 +105,8 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
             umma::mbar_init(&empty[s], 1);
         }
         umma::mbar_init(&acc_full, 1);
-        umma::mbar_init(&act_ready, kEpiWarps);
+        for (int s = 0; s < kActChunks; s++)
+            umma::mbar_init(&act_ready[s], kEpiWarps);
         umma::mbar_init(&x0_ready, kEpiWarps);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -108,6 +123,9 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
     // first one until the first backward product is done)
     auto job_nk = [](int j) { return (j == 0 ? kFeat : kWidth) / kWChunkK; };
     auto job_acc = [](int j) { return j < 4 ? j & 1 : (j == 4 ? 1 : j & 1); };
+    // whether product j may start on the first columns of its operand while the
+    // epilogue writes the others: its accumulator is not being read by it
+    auto job_early = [](int j) { return (j >= 1 && j <= 3) || j == 6; };
 
     if (warp == kEpiWarps + 1) {
         if (lane == 0) {
@@ -145,8 +163,10 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
                 for (int j = 0; j < kChainJobs && ok; j++, jobs++) {
                     if (j == 0)
                         ok = wait_or_abort(&x0_ready, unit & 1u, abort);
-                    if (ok && jobs > 0)
-                        ok = wait_or_abort(&act_ready, (jobs - 1u) & 1u, abort);
+                    int ready = 0;   // column chunks of the operand known to be written
+                    const int at_least = job_early(j) ? 1 : kActChunks;
+                    for (; ok && jobs > 0 && ready < at_least; ready++)
+                        ok = wait_or_abort(&act_ready[ready], (jobs - 1u) & 1u, abort);
                     if (!ok)
                         break;
                     umma::tc_fence_after();
@@ -154,10 +174,13 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
                     const uint32_t d = tmem + (uint32_t)(job_acc(j) * kWidth);
                     for (int kc = 0; kc < job_nk(j); kc++, q++) {
                         const int st = (int)(q % kChainStages);
-                        if (!wait_or_abort(&full[st], (uint32_t)((q / kChainStages) & 1), abort)) {
+                        for (; ok && jobs > 0 && ready <= kc * kWChunkK / umma::kBK; ready++)
+                            ok = wait_or_abort(&act_ready[ready], (jobs - 1u) & 1u, abort);
+                        if (!ok || !wait_or_abort(&full[st], (uint32_t)((q / kChainStages) & 1), abort)) {
                             ok = false;
                             break;
                         }
+                        umma::tc_fence_after();
 #pragma unroll
                         for (int kk = 0; kk < kWChunkK / 16; kk++) {
                             const int k0 = kc * kWChunkK + kk * 16;
@@ -179,15 +202,24 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
     } else {
         // ---- epilogue warps (a warp whose wait runs out goes on through the
         // loops without waiting or writing, see infer_kernel)
-        const int quarter = warp & 3, rl = 32 * quarter + lane, cb = 64 * (warp >> 2);
+        // piece g of a warp: columns 64 g + cb .. + 15, so that all warps finish
+        // a 64-column chunk of the next operand together
+        const int quarter = warp & 3, rl = 32 * quarter + lane, cb = 16 * (warp >> 2);
         const uint32_t lane_base = (uint32_t)(32 * quarter) << 16;
         float *gs = reinterpret_cast<float *>(Act + quarter * kQuarterBytes) + 32 * lane;
         const unsigned step = *a.step;
         uint32_t jobs = 0;
         bool ok = true;
         // a unit's features: into the layer-0 operand and its row image
-        auto gather = [&](int u) {
+        // the unit after `unit` units of this CTA: also its biases and output
+        // weights, which from global memory cost each piece an L2 access
+        auto gather = [&](int u, uint32_t unit) {
             const int e = u / tiles, t = u - e * tiles;
+            float *vec = reinterpret_cast<float *>(smem + kOffChainVec) + (unit & 1u) * kVecFloats;
+            const float *P = a.params + (long long)e * kParams;
+            for (int i = tid; i < kVecFloats; i += 32 * kEpiWarps)
+                vec[i] = i < kDepth * kWidth ? __ldg(P + off_b(i / kWidth) + i % kWidth)
+                                             : __ldg(P + kOffW5 + i - kDepth * kWidth);
             const int r = tid >> 2, part = tid & 3;
             const int b = t * kTileRows + r;
             const uint4 *src = reinterpret_cast<const uint4 *>(a.feat + drawn_row(a, step, e, b) * kFeat) + 2 * part;
@@ -206,85 +238,88 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
             if (ok)
                 umma::tc_fence_after();
         };
-        auto done_job = [&]() {
+        auto done_chunk = [&](int g) {
             umma::tc_fence_before();
             umma::fence_async_smem();
             __syncwarp();
             if (lane == 0)
-                mbar_arrive(&act_ready);
+                mbar_arrive(&act_ready[g]);
+        };
+        // 16 values of a row to its image and into the next operand
+        auto keep = [&](uint4 *im, long long row, int c0, const uint32_t *w, bool operand) {
+            const uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
+            if (operand) {
+                uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
+                const int k = c0 % umma::kBK;
+                *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) = lo;
+                *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) = hi;
+            }
+            im[row_image(row, c0 / 8, kWidth)] = lo;
+            im[row_image(row, c0 / 8 + 1, kWidth)] = hi;
         };
         if ((int)blockIdx.x < units) {
-            gather(blockIdx.x);
+            gather(blockIdx.x, 0u);
             __syncwarp();
             if (lane == 0)
                 mbar_arrive(&x0_ready);
         }
-        for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        uint32_t unit = 0;
+        for (int u = blockIdx.x; u < units; u += gridDim.x, unit++) {
             const int e = u / tiles, t = u - e * tiles;
             const long long row = (long long)t * kTileRows + rl;     // of the member's batch
             const long long tile = (long long)e * tiles + t;
             const long long img = (long long)e * a.batch * (kWidth / 8);
             const float *P = a.params + (long long)e * kParams;
-            const float *w5 = P + kOffW5 + cb;
+            const float *vec = reinterpret_cast<const float *>(smem + kOffChainVec) + (unit & 1u) * kVecFloats + cb;
+            const float *w5 = vec + kDepth * kWidth;
+            asm volatile("bar.sync 5, 512;" ::: "memory");   // `vec` is written by all epilogue warps
             // ---- forward
             for (int l = 0; l < kDepth; l++) {
                 const uint32_t acc = tmem + (uint32_t)(job_acc(l) * kWidth + cb) + lane_base;
-                const float *bias = P + off_b(l) + cb;
+                const float *bias = vec + l * kWidth;
                 wait_job();
-                if (ok) {
-#pragma unroll 1
-                    for (int g = 0; g < 4; g++) {
-                        const int c0 = cb + 16 * g;
-                        float v[16], bs[16];
-                        umma::tmem_ld16_start(acc + 16 * g, v);
+                auto piece = [&](int g, float *v) {
+                    const int c0 = 64 * g + cb;
+                    uint32_t w[8];
+                    gelu::values_bf16<8>(v, bias + 64 * g, w);
+                    keep(a.A[l] + img, row, c0, w, l < kDepth - 1);
+                    if (l < 2) {
+                        float4 *h = a.H[l];
 #pragma unroll
                         for (int q = 0; q < 4; q++)
-                            *reinterpret_cast<float4 *>(bs + 4 * q) =
-                                __ldg(reinterpret_cast<const float4 *>(bias + 16 * g) + q);
-                        umma::tmem_ld16_wait(v);
-                        uint32_t w[8];
-                        gelu::values_bf16<8>(v, bs, w);
-                        if (l < 2) {
-                            float4 *h = a.H[l];
+                            h[pre_image(tile, c0 / 4 + q, rl)] =
+                                make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    }
+                    if (l == kDepth - 1) {
+                        // the head's per-8-column partial sums, as head_kernel's lanes form them
 #pragma unroll
-                            for (int q = 0; q < 4; q++)
-                                h[pre_image(tile, c0 / 4 + q, rl)] =
-                                    make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                        }
-                        const uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
-                        uint4 *im = a.A[l] + img;
-                        im[row_image(row, c0 / 8, kWidth)] = lo;
-                        im[row_image(row, c0 / 8 + 1, kWidth)] = hi;
-                        if (l < kDepth - 1) {
-                            uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
-                            const int k = c0 % umma::kBK;
-                            *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) = lo;
-                            *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) = hi;
-                        } else {
-                            // the head's per-8-column partial sums, as head_kernel's lanes form them
+                        for (int h = 0; h < 2; h++) {
+                            float sum = 0.0f;
 #pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                float sum = 0.0f;
-#pragma unroll
-                                for (int q = 0; q < 8; q++) {
-                                    const uint32_t b = w[4 * h + (q >> 1)];
-                                    sum += __uint_as_float(q & 1 ? b & 0xffff0000u : b << 16) *
-                                           __ldg(w5 + 16 * g + 8 * h + q);
-                                }
-                                gs[(c0 / 8 + h) ^ lane] = sum;
+                            for (int q = 0; q < 8; q++) {
+                                const uint32_t b = w[4 * h + (q >> 1)];
+                                sum += __uint_as_float(q & 1 ? b & 0xffff0000u : b << 16) * w5[64 * g + 8 * h + q];
                             }
+                            gs[(c0 / 8 + h) ^ lane] = sum;
                         }
                     }
-                }
-                if (l < kDepth - 1) {
-                    done_job();
-                    if (l == 0 && u + (int)gridDim.x < units) {   // the features have been read: the next unit's
-                        if (ok)
-                            gather(u + gridDim.x);
-                        __syncwarp();
-                        if (lane == 0)
-                            mbar_arrive(&x0_ready);
+                };
+#pragma unroll 1
+                for (int g = 0; g < 4; g++) {
+                    if (ok) {
+                        float v[16];
+                        umma::tmem_ld16(acc + 64 * g, v);
+                        piece(g, v);
                     }
+                    if (l < kDepth - 1)
+                        done_chunk(g);
+                }
+                if (l == 0 && u + (int)gridDim.x < units) {   // the features have been read: the next unit's
+                    if (ok)
+                        gather(u + gridDim.x, unit + 1u);
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(&x0_ready);
                 }
             }
             // ---- head, loss
@@ -314,78 +349,72 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
             }
             quarter_sync(quarter);
             // ---- dH_3 (the last hidden layer's), from its accumulator again
-            if (ok) {
-                const float gd = dys[rl];
-                const float *bias = P + off_b(kDepth - 1) + cb;
+            {
+                const float gd = ok ? dys[rl] : 0.0f;
+                const float *bias = vec + (kDepth - 1) * kWidth;
                 const uint32_t acc = tmem + (uint32_t)(job_acc(kDepth - 1) * kWidth + cb) + lane_base;
 #pragma unroll 1
                 for (int g = 0; g < 4; g++) {
-                    const int c0 = cb + 16 * g;
-                    float h[16], v[16];
-                    umma::tmem_ld16_start(acc + 16 * g, h);
+                    if (ok) {
+                        float h[16], v[16];
+                        umma::tmem_ld16_start(acc + 64 * g, h);
 #pragma unroll
-                    for (int q = 0; q < 16; q++)
-                        v[q] = gd * __ldg(w5 + 16 * g + q);
-                    umma::tmem_ld16_wait(h);
+                        for (int q = 0; q < 16; q++)
+                            v[q] = gd * w5[64 * g + q];
+                        umma::tmem_ld16_wait(h);
 #pragma unroll
-                    for (int q = 0; q < 16; q++)
-                        h[q] += __ldg(bias + 16 * g + q);
-                    uint32_t w[8];
-                    gelu::grads_bf16<8>(v, h, w);
-                    const uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
-                    uint4 *im = a.dH[kDepth - 1] + img;
-                    im[row_image(row, c0 / 8, kWidth)] = lo;
-                    im[row_image(row, c0 / 8 + 1, kWidth)] = hi;
-                    uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
-                    const int k = c0 % umma::kBK;
-                    *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) = lo;
-                    *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) = hi;
+                        for (int q = 0; q < 16; q++)
+                            h[q] += bias[64 * g + q];
+                        uint32_t w[8];
+                        gelu::grads_bf16<8>(v, h, w);
+                        keep(a.dH[kDepth - 1] + img, row, 64 * g + cb, w, true);
+                    }
+                    done_chunk(g);
                 }
             }
-            done_job();
             // ---- backward
             for (int l = kDepth - 2; l >= 0; l--) {
                 const int j = 2 * kDepth - 2 - l;   // product 4 gives layer 2's gradient, 6 layer 0's
                 const uint32_t acc = tmem + (uint32_t)(job_acc(j) * kWidth + cb) + lane_base;
                 const uint32_t hacc = tmem + (uint32_t)(job_acc(2) * kWidth + cb) + lane_base;
-                const float *bias = P + off_b(l) + cb;
+                const float *bias = vec + l * kWidth;
                 const float4 *hs = l < 2 ? a.H[l] : nullptr;
-                wait_job();
-                if (ok) {
-#pragma unroll 1
-                    for (int g = 0; g < 4; g++) {
-                        const int c0 = cb + 16 * g;
-                        float h[16], v[16];
-                        if (l == 2) {
-                            umma::tmem_ld16_start(hacc + 16 * g, h);
-                            umma::tmem_ld16_start(acc + 16 * g, v);
-                            umma::tmem_ld16_wait(h);
-                            umma::tmem_ld16_wait(v);
+                // layers 0 and 1: the pre-activations come from L2, a piece ahead
+                auto fetch = [&](int g, float *h) {
 #pragma unroll
-                            for (int q = 0; q < 16; q++)
-                                h[q] += __ldg(bias + 16 * g + q);
-                        } else {
-                            umma::tmem_ld16_start(acc + 16 * g, v);
+                    for (int q = 0; q < 4; q++)
+                        *reinterpret_cast<float4 *>(h + 4 * q) = hs[pre_image(tile, (64 * g + cb) / 4 + q, rl)];
+                };
+                auto piece = [&](int g, float *h, float *v) {
+                    if (l == 2) {
+                        umma::tmem_ld16_start(hacc + 64 * g, h);
+                        umma::tmem_ld16_start(acc + 64 * g, v);
+                        umma::tmem_ld16_wait(h);
+                        umma::tmem_ld16_wait(v);
 #pragma unroll
-                            for (int q = 0; q < 4; q++)
-                                *reinterpret_cast<float4 *>(h + 4 * q) = hs[pre_image(tile, c0 / 4 + q, rl)];
-                            umma::tmem_ld16_wait(v);
-                        }
-                        uint32_t w[8];
-                        gelu::grads_bf16<8>(v, h, w);
-                        const uint4 lo = make_uint4(w[0], w[1], w[2], w[3]), hi = make_uint4(w[4], w[5], w[6], w[7]);
-                        uint4 *im = a.dH[l] + img;
-                        im[row_image(row, c0 / 8, kWidth)] = lo;
-                        im[row_image(row, c0 / 8 + 1, kWidth)] = hi;
-                        if (l > 0) {
-                            uint8_t *dst = Act + (c0 / umma::kBK) * kActChunk;
-                            const int k = c0 % umma::kBK;
-                            *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k)) = lo;
-                            *reinterpret_cast<uint4 *>(dst + umma::tile_off(rl, k + 8)) = hi;
-                        }
+                        for (int q = 0; q < 16; q++)
+                            h[q] += bias[64 * g + q];
+                    } else {
+                        umma::tmem_ld16(acc + 64 * g, v);
                     }
+                    uint32_t w[8];
+                    gelu::grads_bf16<8>(v, h, w);
+                    keep(a.dH[l] + img, row, 64 * g + cb, w, l > 0);
+                };
+                float h[16];
+                if (ok && l < 2)
+                    fetch(0, h);
+                wait_job();
+#pragma unroll 1
+                for (int g = 0; g < 4; g++) {
+                    if (ok) {
+                        float v[16];
+                        piece(g, h, v);
+                        if (l < 2 && g + 1 < 4)
+                            fetch(g + 1, h);
+                    }
+                    done_chunk(g);
                 }
-                done_job();
             }
         }
     }
@@ -397,151 +426,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) chain_kernel(ChainArgs a)
         umma::tmem_dealloc(tmem, 2 * kWidth);
 }
 
-// ---------------------------------------------------------------- gradients
-//
-// dW_l = dH_l^T A_{l-1} for one (member, layer, K split, half of the 256
-// rows of dW_l): M = 128, N = 256 or 64, K = batch / 16 rows in blocks of 64,
-// both operands MN-major straight from the row images.  Partial sums go out
-// as [4-column group][128 rows][4], 512 contiguous bytes a warp and store.
-
-constexpr int kDwStages = 2;
-constexpr int kDwA = 16 * 1024;                     // 128 columns of a dH block
-constexpr int kDwStage = kDwA + 32 * 1024;          // and 256 of an activation block
-constexpr int kDwSmem = kDwStages * kDwStage;       // two CTAs an SM
-constexpr int kDwThreads = 192;                     // four epilogue warps, copy, MMA
-
-// floats of the partial sums before layer l of a member
-__host__ __device__ constexpr long long part_off(int l)
-{
-    return l == 0 ? 0 : (long long)kSplitK * kWidth * (kFeat + (l - 1) * kWidth);
-}
-constexpr long long kPartFloats = (long long)kSplitK * kWidth * (kFeat + (kDepth - 1) * kWidth);
-
-struct DwArgs {
-    const uint4 *X0, *A[kDepth], *dH[kDepth];
-    int batch;
-    float4 *part;             // [E][kPartFloats]
-    // the first block also closes the step's loss: its mean over the members
-    // into the history and the step count (when there is one to close)
-    unsigned *step;
-    float *loss_acc, *loss_hist;
-    int E, hist_len, count_step;
-    int *err;
-};
-
-__global__ void __launch_bounds__(kDwThreads, 2) dw_kernel(DwArgs a)
-{
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t full[kDwStages], empty[kDwStages], acc_full;
-    __shared__ uint32_t tslot;
-    __shared__ int s_abort;
-    volatile int *abort = &s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mh = blockIdx.x & 1, sp = (blockIdx.x >> 1) % kSplitK, l = (blockIdx.x >> 1) / kSplitK;
-    const int e = blockIdx.y;
-    const int K = l == 0 ? kFeat : kWidth;
-    const int rows = a.batch / kSplitK, blocks = rows / 64;
-    const long long block0 = (long long)sp * blocks;
-
-    if (tid == 0) {
-        for (int s = 0; s < kDwStages; s++) {
-            umma::mbar_init(&full[s], 1);
-            umma::mbar_init(&empty[s], 1);
-        }
-        umma::mbar_init(&acc_full, 1);
-        s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0)
-        umma::tmem_alloc(&tslot, kWidth);
-    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 64) {
-        float acc = 0.0f;
-        for (int m = 0; m < a.E; m++) {
-            acc += a.loss_acc[m];
-            a.loss_acc[m] = 0.0f;
-        }
-        if (a.count_step) {
-            const unsigned s = *a.step;
-            if ((int)s < a.hist_len)
-                a.loss_hist[s] = acc / (float)a.E;
-            *a.step = s + 1u;
-        }
-    }
-    umma::tc_fence_before();
-    __syncthreads();
-    umma::tc_fence_after();
-    const uint32_t tmem = tslot;
-    const uint32_t b_bytes = (uint32_t)K * 128u;    // 64 rows x K columns
-
-    if (warp == 4) {
-        if (lane == 0) {
-            const uint8_t *A = reinterpret_cast<const uint8_t *>(a.dH[l] + (long long)e * a.batch * (kWidth / 8));
-            const uint8_t *B =
-                reinterpret_cast<const uint8_t *>((l == 0 ? a.X0 : a.A[l - 1]) + (long long)e * a.batch * (K / 8));
-            int c = 0;
-            for (; c < blocks; c++) {
-                const int st = c % kDwStages;
-                if (c >= kDwStages && !wait_or_abort(&empty[st], (uint32_t)((c / kDwStages - 1) & 1), abort))
-                    break;
-                uint8_t *dst = smem + st * kDwStage;
-                mbar_expect_tx(&full[st], kDwA + b_bytes);
-                bulk_g2s(dst, A + (block0 + c) * (kWidth * 128) + mh * kDwA, kDwA, &full[st]);
-                bulk_g2s(dst + kDwA, B + (block0 + c) * b_bytes, b_bytes, &full[st]);
-            }
-            for (int p = c > kDwStages ? c - kDwStages : 0; p < c; p++)   // none in flight at the end
-                wait_or_abort(&full[p % kDwStages], (uint32_t)((p / kDwStages) & 1), abort);
-        }
-        __syncwarp();
-    } else if (warp == 5) {
-        if (lane == 0) {
-            // both operands MN-major (transpose bits of the instruction descriptor)
-            const uint32_t idesc = umma::idesc_bf16_f32(K) | (1u << 15) | (1u << 16);
-            bool ok = true;
-            for (int c = 0; c < blocks; c++) {
-                const int st = c % kDwStages;
-                if (!wait_or_abort(&full[st], (uint32_t)((c / kDwStages) & 1), abort)) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t a0 = umma::smem_u32(smem + st * kDwStage), b0 = a0 + kDwA;
-#pragma unroll
-                for (int kk = 0; kk < 4; kk++)   // 16 rows each
-                    umma::mma_bf16(tmem, umma::smem_desc(a0 + kk * 256, 128, 1024),
-                                   umma::smem_desc(b0 + kk * 256, 128, 1024), idesc, (c > 0 || kk > 0) ? 1u : 0u);
-                umma::mma_commit(&empty[st]);
-            }
-            umma::mma_commit(&acc_full);
-            if (!ok)
-                *abort = 1;
-        }
-        __syncwarp();
-    } else {
-        bool ok = wait_or_abort(&acc_full, 0u, abort);
-        ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-            umma::tc_fence_after();
-            float4 *out = a.part + ((long long)e * kPartFloats + part_off(l) +
-                                    (long long)(sp * 2 + mh) * (128 * K)) / 4;
-            const uint32_t acc = tmem + ((uint32_t)(32 * warp) << 16);
-            for (int c0 = 0; c0 < K; c0 += 16) {
-                float v[16];
-                umma::tmem_ld16(acc + c0, v);
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    out[(c0 / 4 + q) * 128 + 32 * warp + lane] =
-                        make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            }
-        }
-    }
-    umma::tc_fence_before();
-    __syncthreads();
-    if (tid == 0 && s_abort)
-        atomicOr(a.err, 1);
-    if (warp == 0)
-        umma::tmem_dealloc(tmem, kWidth);
-}
-
-// ------------------------------------------------------------------- update
+// --------------------------------------------------------- gradients, update
 
 struct AdamArgs {
     float lr_max, lr_min, b1, b2, eps;
@@ -595,102 +480,59 @@ __host__ __device__ constexpr long long back_image_off(int e, int l, int n, int 
     return ((long long)e * kChunksBack + (l - 1) * 8 + n / kWChunkK) * kChunkBytes + wchunk_off(k, n % kWChunkK);
 }
 
+// One launch for the weight gradients dW_l = dH_l^T A_{l-1}, the column sums
+// over the batch (bias gradients, the output weights' and bias's), Adam and
+// the weights' BF16 copies.
+//
+// Blocks 0 .. E * kGradTiles - 1: a tile of 128 x 64 weights of one matrix, the
+// whole batch.  Both operands come MN-major straight from the row images, 64
+// rows a stage; each K split (batch / kSplitK rows) has an accumulator of its
+// own, four of them in a ring, and the epilogue adds the splits in order while
+// the next are computed, so no partial sums are stored: a kernel with a CTA a
+// split and one that added them moved 110 MB between them.  Bound by the
+// operands' way from L2, 1.5 MB a tile (64 columns a tile are 104 tiles for
+// four members at a batch of 4,096, one an SM; 32 columns would be 2.5 MB an
+// SM), with eight stages of 24 KB in flight, and by Adam's quotients at the
+// end.  23 + 22 us as two kernels, 40 so.
+// The rest: column sums, a task (eight columns of an image) after the other,
+// on the SMs that the tiles leave; each thread's rows and the order of the
+// sums as in a block of 256 threads striding over the batch.
+
 struct UpdateArgs {
-    const float4 *part;
-    const uint4 *A3, *dH[kDepth];   // last activation, layer gradients (row images)
+    const uint4 *X0, *A[kDepth], *dH[kDepth];   // row images
     const float *dy;
     int batch, E;
     float *params, *m, *v, *grad;
-    const unsigned *step;           // already counted
     AdamArgs adam;
-    int update;                     // Adam and the copies, or (0) the gradients into `grad`
+    int update;                     // Adam, the copies and the step count, or (0) the gradients into `grad`
     WeightCopies copies;
+    // The last block to have read the step count closes the step: the loss, its
+    // mean over the members into the history, and the count.
+    unsigned *step, *ticket;
+    float *loss_acc, *loss_hist;
+    int hist_len;
+    int *err;
 };
 
-constexpr int kPatch = 32;          // weights in patches of 32 x 32
-constexpr int kPatches0 = (kWidth / kPatch) * (kFeat / kPatch), kPatchesL = (kWidth / kPatch) * (kWidth / kPatch);
-constexpr int kPatches = kPatches0 + (kDepth - 1) * kPatchesL;
-constexpr int kVectors = (kDepth + 1) * (kWidth / 8) + 1;   // column sums: four biases, w5 (8 columns each); b5
+constexpr int kGradCols = 64;
+constexpr int kGradTiles = 2 + (kDepth - 1) * 2 * (kWidth / kGradCols);   // per member
+constexpr int kGradStages = 8;
+constexpr int kGradA = 16 * 1024;                              // 128 columns of a dH block
+constexpr int kGradStage = kGradA + kGradCols * 128;           // and 64 of an activation block
+constexpr int kGradSmem = kGradStages * kGradStage;            // 192 KB: one CTA an SM
+constexpr int kGradAccs = 4;
+constexpr int kGradThreads = 320;                              // eight epilogue warps, copy, MMA
+constexpr int kGradPitch = kGradCols + 1;                      // floats a row of the gradient tile
+static_assert(128 * kGradPitch * 4 <= kGradSmem, "the gradient tile reuses the stages");
+constexpr int kVectors = (kDepth + 1) * (kWidth / 8) + 1;      // column sums: four biases, w5 (8 columns each); b5
 
-// Blocks 0 .. kPatches - 1 of a member: a 32 x 32 patch of a weight matrix.
-// The rest: column sums over the batch (bias gradients, the output weights'
-// and bias's), each thread's rows and the order of the sums as in a block of
-// 256 threads striding over the batch.
-__global__ void __launch_bounds__(256) update_kernel(UpdateArgs a)
+__device__ __forceinline__ void sync_256() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+// column sums of task b of member e (256 threads)
+__device__ __forceinline__ void column_sums(const UpdateArgs &a, const AdamStep &st, int e, int b, float (*red)[8])
 {
-    const int e = blockIdx.y, tid = threadIdx.x;
-    const AdamStep st = a.update ? adam_step(a.adam, *a.step - 1u) : AdamStep{0.0f, 1.0f, 1.0f};
-    float *P = a.params + (long long)e * kParams;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long pe = (long long)e * kParams;
-    __shared__ float g[kPatch][kPatch + 1];
-    if (blockIdx.x < kPatches) {
-        int b = blockIdx.x, l = 0;
-        if (b >= kPatches0) {
-            b -= kPatches0;
-            l = 1 + b / kPatchesL;
-            b %= kPatchesL;
-        }
-        const int K = in_dim(l), per_row = K / kPatch;
-        const int n0 = b / per_row * kPatch, k0 = b % per_row * kPatch;
-        {
-            // thread: row n0 + lane, columns k0 + 4 * warp ..; the splits in order
-            const int lane = tid & 31, c4 = k0 / 4 + (tid >> 5);
-            const float4 *p = a.part + (pe / kParams * kPartFloats + part_off(l)) / 4 +
-                              ((long long)(n0 / 128) * (K / 4) + c4) * 128 + n0 % 128 + lane;
-            const long long stride = (long long)2 * 32 * K;   // float4s of a split: 256 K / 4
-            float4 v[kSplitK];
-#pragma unroll
-            for (int s = 0; s < kSplitK; s++)
-                v[s] = __ldg(p + s * stride);
-            float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-            for (int s = 0; s < kSplitK; s++) {
-                t.x += v[s].x;
-                t.y += v[s].y;
-                t.z += v[s].z;
-                t.w += v[s].w;
-            }
-            float *row = &g[lane][4 * (tid >> 5)];
-            row[0] = t.x;
-            row[1] = t.y;
-            row[2] = t.z;
-            row[3] = t.w;
-        }
-        __syncthreads();
-        const int r = tid >> 3, c = 4 * (tid & 7);   // four weights along k
-        const long long o = pe + off_w(l) + (long long)(n0 + r) * K + k0 + c;
-        if (!a.update) {
-            *reinterpret_cast<float4 *>(a.grad + o) = make_float4(g[r][c], g[r][c + 1], g[r][c + 2], g[r][c + 3]);
-            return;
-        }
-        float4 p4 = *reinterpret_cast<float4 *>(a.params + o), m4 = *reinterpret_cast<float4 *>(a.m + o),
-               v4 = *reinterpret_cast<float4 *>(a.v + o);
-        float *pp = &p4.x, *mm = &m4.x, *vv = &v4.x;
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            pp[q] = adam(a.adam, st, g[r][c + q], mm[q], vv[q], pp[q]);
-        *reinterpret_cast<float4 *>(a.params + o) = p4;
-        *reinterpret_cast<float4 *>(a.m + o) = m4;
-        *reinterpret_cast<float4 *>(a.v + o) = v4;
-        const uint2 w = make_uint2(gelu::bf16x2(pp[0], pp[1]), gelu::bf16x2(pp[2], pp[3]));
-        *reinterpret_cast<uint2 *>(a.copies.w[l] + (long long)e * kWidth * K + (long long)(n0 + r) * K + k0 + c) = w;
-        *reinterpret_cast<uint2 *>(a.copies.wimg + image_off(e, l, n0 + r, k0 + c)) = w;
-        if (l > 0) {
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                g[r][c + q] = pp[q];
-            __syncthreads();
-            // four weights along n of column k0 + r
-            const uint2 wt = make_uint2(gelu::bf16x2(g[c][r], g[c + 1][r]), gelu::bf16x2(g[c + 2][r], g[c + 3][r]));
-            *reinterpret_cast<uint2 *>(a.copies.wtimg + back_image_off(e, l, n0 + c, k0 + r)) = wt;
-        }
-        return;
-    }
-    // ---- column sums
-    const int b = blockIdx.x - kPatches;
-    const int lane = tid & 31, warp = tid >> 5;
-    __shared__ float red[8][8];
     const bool last = b == kVectors - 1;             // b5
     const int l = b / (kWidth / 8), group = b % (kWidth / 8);
     float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -699,8 +541,8 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs a)
         for (int r = tid; r < a.batch; r += 256)
             acc[0] += dy[r];
     } else {
-        const uint4 *im = (l < kDepth ? a.dH[l] : a.A3) + (long long)e * a.batch * (kWidth / 8);
-#pragma unroll 4
+        const uint4 *im = (l < kDepth ? a.dH[l] : a.A[kDepth - 1]) + (long long)e * a.batch * (kWidth / 8);
+#pragma unroll 16
         for (int r = tid; r < a.batch; r += 256) {
             const uint4 x = __ldg(im + row_image(r, group, kWidth));
             const float w = l < kDepth ? 1.0f : dy[r];
@@ -710,6 +552,7 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs a)
                 acc[q] += __uint_as_float(q & 1 ? u[q >> 1] & 0xffff0000u : u[q >> 1] << 16) * w;
         }
     }
+    sync_256();   // the last task's sums have been read
 #pragma unroll
     for (int q = 0; q < 8; q++) {
 #pragma unroll
@@ -718,7 +561,7 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs a)
         if (lane == 0)
             red[q][warp] = acc[q];
     }
-    __syncthreads();
+    sync_256();
     if (tid < (last ? 1 : 8)) {
         float s[8];
 #pragma unroll
@@ -729,13 +572,230 @@ __global__ void __launch_bounds__(256) update_kernel(UpdateArgs a)
 #pragma unroll
             for (int w = 0; w < o; w++)
                 s[w] += s[w + o];
-        const long long o = last ? kOffB5 : (l < kDepth ? off_b(l) + 8 * group + tid : kOffW5 + 8 * group + tid);
-        if (!a.update) {
-            a.grad[pe + o] = s[0];
-        } else {
-            P[o] = adam(a.adam, st, s[0], a.m[pe + o], a.v[pe + o], P[o]);
+        const long long o = pe + (last ? kOffB5 : (l < kDepth ? off_b(l) : kOffW5) + 8 * group + tid);
+        if (!a.update)
+            a.grad[o] = s[0];
+        else
+            a.params[o] = adam(a.adam, st, s[0], a.m[o], a.v[o], a.params[o]);
+    }
+}
+
+// Adam and the copies of the tile g of gradients (256 threads): rows n0 ..,
+// columns k0 .. of W_l of member e
+__device__ __forceinline__ void update_tile(const UpdateArgs &a, const AdamStep &st, int e, int l, int n0, int k0,
+                                            float (*g)[kGradPitch])
+{
+    const int tid = threadIdx.x, K = in_dim(l);
+    const long long base = (long long)e * kParams + off_w(l);
+    // four weights along k a thread and pass; the loads of four passes together
+    constexpr int kPasses = 128 * (kGradCols / 4) / 256, kAhead = 4;
+    const int c = 4 * (tid % (kGradCols / 4)), r0 = tid / (kGradCols / 4);
+    constexpr int kRowStep = 256 / (kGradCols / 4);
+    for (int i0 = 0; i0 < kPasses; i0 += kAhead) {
+        float4 p4[kAhead], m4[kAhead], v4[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) {
+            const int r = r0 + (i0 + i) * kRowStep;
+            const long long o = base + (long long)(n0 + r) * K + k0 + c;
+            if (!a.update) {
+                *reinterpret_cast<float4 *>(a.grad + o) = make_float4(g[r][c], g[r][c + 1], g[r][c + 2], g[r][c + 3]);
+                continue;
+            }
+            p4[i] = *reinterpret_cast<const float4 *>(a.params + o);
+            m4[i] = *reinterpret_cast<const float4 *>(a.m + o);
+            v4[i] = *reinterpret_cast<const float4 *>(a.v + o);
+        }
+        if (!a.update)
+            continue;
+#pragma unroll
+        for (int i = 0; i < kAhead; i++) {
+            const int r = r0 + (i0 + i) * kRowStep;
+            const long long o = base + (long long)(n0 + r) * K + k0 + c;
+            float *pp = &p4[i].x, *mm = &m4[i].x, *vv = &v4[i].x;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                pp[q] = adam(a.adam, st, g[r][c + q], mm[q], vv[q], pp[q]);
+                g[r][c + q] = pp[q];
+            }
+            *reinterpret_cast<float4 *>(a.params + o) = p4[i];
+            *reinterpret_cast<float4 *>(a.m + o) = m4[i];
+            *reinterpret_cast<float4 *>(a.v + o) = v4[i];
+            const uint2 w = make_uint2(gelu::bf16x2(pp[0], pp[1]), gelu::bf16x2(pp[2], pp[3]));
+            *reinterpret_cast<uint2 *>(a.copies.w[l] + (long long)e * kWidth * K + (long long)(n0 + r) * K + k0 + c) =
+                w;
+            *reinterpret_cast<uint2 *>(a.copies.wimg + image_off(e, l, n0 + r, k0 + c)) = w;
         }
     }
+    if (!a.update || l == 0)
+        return;
+    sync_256();
+#pragma unroll 2
+    for (int i = tid; i < kGradCols * 32; i += 256) {
+        const int r = i / 32, n = 4 * (i % 32);   // four weights along n of column k0 + r
+        const uint2 w = make_uint2(gelu::bf16x2(g[n][r], g[n + 1][r]), gelu::bf16x2(g[n + 2][r], g[n + 3][r]));
+        *reinterpret_cast<uint2 *>(a.copies.wtimg + back_image_off(e, l, n0 + n, k0 + r)) = w;
+    }
+}
+
+__global__ void __launch_bounds__(kGradThreads, 1) update_kernel(UpdateArgs a)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t full[kGradStages], empty[kGradStages], acc_full[kGradAccs], acc_empty[kGradAccs];
+    __shared__ uint32_t tslot;
+    __shared__ int s_abort, s_bad;   // s_bad: of the epilogue warps, decided at a barrier
+    __shared__ float red[8][8];
+    volatile int *abort = &s_abort;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tiles = a.E * kGradTiles;
+    const bool is_tile = (int)blockIdx.x < tiles;
+    const AdamStep st = a.update ? adam_step(a.adam, *(volatile unsigned *)a.step) : AdamStep{0.0f, 1.0f, 1.0f};
+
+    if (tid == 0) {
+        for (int s = 0; s < kGradStages; s++) {
+            umma::mbar_init(&full[s], 1);
+            umma::mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < kGradAccs; s++) {
+            umma::mbar_init(&acc_full[s], 1);
+            umma::mbar_init(&acc_empty[s], 8);
+        }
+        s_abort = s_bad = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0 && is_tile)
+        umma::tmem_alloc(&tslot, kGradAccs * kGradCols);
+    umma::tc_fence_before();
+    __syncthreads();
+    umma::tc_fence_after();
+    if (tid == 0) {   // this block has read the step count
+        __threadfence();
+        if (atomicAdd(a.ticket, 1u) == gridDim.x - 1) {
+            *a.ticket = 0u;
+            float acc = 0.0f;
+            for (int m = 0; m < a.E; m++) {
+                acc += a.loss_acc[m];
+                a.loss_acc[m] = 0.0f;
+            }
+            if (a.update) {
+                const unsigned s = *(volatile unsigned *)a.step;
+                if ((int)s < a.hist_len)
+                    a.loss_hist[s] = acc / (float)a.E;
+                *a.step = s + 1u;
+            }
+        }
+    }
+    if (!is_tile) {
+        if (warp < 8)
+            for (int q = (int)blockIdx.x - tiles; q < a.E * kVectors; q += (int)gridDim.x - tiles)
+                column_sums(a, st, q / kVectors, q % kVectors, red);
+        return;
+    }
+
+    const uint32_t tmem = tslot;
+    const int e = blockIdx.x / kGradTiles, t = blockIdx.x % kGradTiles;
+    const int l = t < 2 ? 0 : 1 + (t - 2) / (2 * (kWidth / kGradCols));
+    const int mh = t & 1, nt = t < 2 ? 0 : (t - 2) / 2 % (kWidth / kGradCols);
+    const int per = a.batch / kSplitK / 64, blocks = kSplitK * per;   // 64-row blocks of a split, of the batch
+    if (warp == 8) {
+        if (lane == 0) {
+            const int K = in_dim(l);
+            const uint8_t *A =
+                reinterpret_cast<const uint8_t *>(a.dH[l] + (long long)e * a.batch * (kWidth / 8)) + mh * kGradA;
+            const uint8_t *B =
+                reinterpret_cast<const uint8_t *>((l == 0 ? a.X0 : a.A[l - 1]) + (long long)e * a.batch * (K / 8)) +
+                nt * (kGradCols * 128);
+            int c = 0;
+            for (; c < blocks; c++) {
+                const int s = c % kGradStages;
+                if (c >= kGradStages && !wait_or_abort(&empty[s], (uint32_t)((c / kGradStages - 1) & 1), abort))
+                    break;
+                uint8_t *dst = smem + s * kGradStage;
+                mbar_expect_tx(&full[s], kGradStage);
+                bulk_g2s(dst, A + (long long)c * (kWidth * 128), kGradA, &full[s]);
+                bulk_g2s(dst + kGradA, B + (long long)c * (K * 128), kGradCols * 128, &full[s]);
+            }
+            for (int p = c > kGradStages ? c - kGradStages : 0; p < c; p++)   // none in flight at the end
+                wait_or_abort(&full[p % kGradStages], (uint32_t)((p / kGradStages) & 1), abort);
+        }
+        __syncwarp();
+    } else if (warp == 9) {
+        if (lane == 0) {
+            // both operands MN-major (transpose bits of the instruction descriptor)
+            constexpr uint32_t idesc = umma::idesc_bf16_f32(kGradCols) | (1u << 15) | (1u << 16);
+            bool ok = true;
+            for (int sp = 0, c = 0; sp < kSplitK && ok; sp++) {
+                const int q = sp % kGradAccs;
+                if (sp >= kGradAccs)
+                    ok = wait_or_abort(&acc_empty[q], (uint32_t)((sp / kGradAccs - 1) & 1), abort);
+                umma::tc_fence_after();
+                for (int i = 0; i < per && ok; i++, c++) {
+                    const int s = c % kGradStages;
+                    ok = wait_or_abort(&full[s], (uint32_t)((c / kGradStages) & 1), abort);
+                    if (!ok)
+                        break;
+                    const uint32_t a0 = umma::smem_u32(smem + s * kGradStage), b0 = a0 + kGradA;
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)   // 16 rows each
+                        umma::mma_bf16(tmem + (uint32_t)(q * kGradCols), umma::smem_desc(a0 + kk * 256, 128, 1024),
+                                       umma::smem_desc(b0 + kk * 256, 128, 1024), idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                    umma::mma_commit(&empty[s]);
+                }
+                if (ok)
+                    umma::mma_commit(&acc_full[q]);
+            }
+            if (!ok)
+                *abort = 1;
+        }
+        __syncwarp();
+    } else {
+        const int quarter = warp & 3, c0 = 32 * (warp >> 2);
+        const uint32_t acc = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)c0;
+        float sum[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            sum[j] = 0.0f;
+        bool ok = true;
+        for (int sp = 0; sp < kSplitK; sp++) {
+            const int q = sp % kGradAccs;
+            ok = ok && wait_or_abort(&acc_full[q], (uint32_t)((sp / kGradAccs) & 1), abort);
+            ok = __all_sync(0xffffffffu, ok);
+            if (ok) {
+                float v[16], w[16];
+                umma::tc_fence_after();
+                umma::tmem_ld16_start(acc + q * kGradCols, v);
+                umma::tmem_ld16_start(acc + q * kGradCols + 16, w);
+                umma::tmem_ld16_wait(v);
+                umma::tmem_ld16_wait(w);
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    sum[j] += v[j];
+                    sum[16 + j] += w[j];
+                }
+                umma::tc_fence_before();
+            }
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&acc_empty[q]);
+        }
+        // all products are done: the stages hold the gradient tile now
+        float(*g)[kGradPitch] = reinterpret_cast<float(*)[kGradPitch]>(smem);
+        if (!ok)
+            s_bad = s_abort = 1;
+        sync_256();
+        if (!s_bad) {
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                g[32 * quarter + lane][c0 + j] = sum[j];
+            sync_256();
+            update_tile(a, st, e, l, 128 * mh, kGradCols * nt, g);
+        }
+    }
+    umma::tc_fence_before();
+    __syncthreads();
+    if (tid == 0 && s_abort)
+        atomicOr(a.err, 1);
+    if (warp == 0)
+        umma::tmem_dealloc(tmem, kGradAccs * kGradCols);
 }
 
 // BF16 copies of all weights from the FP32 masters
