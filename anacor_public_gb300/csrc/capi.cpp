@@ -124,11 +124,13 @@ int current_device(DeviceState **out)
             return fail(kErrCuda, "this library is built for sm_103a (Blackwell Ultra) only");
         if (rcp_table_init() != kOk)
             return fail(kErrCuda, "reciprocal table upload failed");
-        // 40 % of the unified storage as shared memory: room for 4 CTAs' 19 KB and
-        // the rest L1 for the label gathers (measured best of 0/25/40/60/100 %,
-        // by about 1 %); ANACOR_SMEM_CARVEOUT overrides
+        // Shared memory's share of the unified storage, the rest L1 for the label
+        // gathers.  Cooperative march: 40 %, room for 4 CTAs' 19 KB (30 .. 50 %
+        // are within 1 %).  Field march: 50 %, room for 5 CTAs' 20 KB; at 40 %
+        // only 4 fit (512x512x400, 4,000 reflections: 4.09 ms at 40 %, 3.80 at
+        // 45 .. 55, 3.89 at 60, 4.11 at 75).  ANACOR_SMEM_CARVEOUT overrides both.
         const char *cv = std::getenv("ANACOR_SMEM_CARVEOUT");
-        absorption_set_carveout(cv ? std::atoi(cv) : 40);
+        absorption_set_carveout(cv ? std::atoi(cv) : 40, cv ? std::atoi(cv) : 50);
         if (absorption_occupancy(&d.blocks_per_sm) != kOk || d.blocks_per_sm <= 0)
             return fail(kErrCuda, "kernel not loadable on this device");
         if ((e = cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking)) != cudaSuccess)

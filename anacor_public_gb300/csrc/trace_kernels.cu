@@ -2616,16 +2616,16 @@ int block_guard_selftest(int threads, int *status_out)
 
 // Preferred shared-memory carveout (percent of the unified L1/shared storage)
 // of every absorption kernel; a hint to the driver.
-int absorption_set_carveout(int pct)
+int absorption_set_carveout(int pct, int field_pct)
 {
     cudaError_t e = cudaSuccess;
-#define ANACOR_CARVE(K) \
+#define ANACOR_CARVE(K, P) \
     if (e == cudaSuccess) \
-        e = cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, pct)
-    ANACOR_CARVE(absorption_kernel<1>); ANACOR_CARVE(absorption_kernel<2>);
-    ANACOR_CARVE(absorption_kernel<3>); ANACOR_CARVE(absorption_kernel<4>);
+        e = cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, P)
+    ANACOR_CARVE(absorption_kernel<1>, pct); ANACOR_CARVE(absorption_kernel<2>, pct);
+    ANACOR_CARVE(absorption_kernel<3>, pct); ANACOR_CARVE(absorption_kernel<4>, pct);
 #define ANACOR_CARVE2(B) \
-    ANACOR_CARVE((field_kernel<B, false>)); ANACOR_CARVE((field_kernel<B, true>))
+    ANACOR_CARVE((field_kernel<B, false>), field_pct); ANACOR_CARVE((field_kernel<B, true>), field_pct)
     ANACOR_CARVE2(1); ANACOR_CARVE2(2); ANACOR_CARVE2(3); ANACOR_CARVE2(4);
 #undef ANACOR_CARVE2
 #undef ANACOR_CARVE

@@ -113,7 +113,7 @@ int absorption_block_threads();
 // status word it leaves (ANACOR_ERR_ARGS bit set when the block-shape guard
 // refused the launch).
 int block_guard_selftest(int threads, int *status_out);
-int absorption_set_carveout(int pct);
+int absorption_set_carveout(int pct, int field_pct);
 // Kernel variants: 1..4 the cooperative march with a register budget for
 // 1..4 CTAs per SM; 5..8 the same budgets with the distance-field march on
 // linear fields; 9..12 on 4^3-bricked fields (every sample needs its `field`

@@ -1,4 +1,4 @@
-"""The three-kernel training step at batches and ensemble sizes where its work
+"""The fused training step at batches and ensemble sizes where its work
 distribution changes (one to several 128-row tiles per CTA, one to several
 64-row blocks per K split), against the FP64 statement of the network with the
 same BF16 rounding points, and steps that do not depend on
