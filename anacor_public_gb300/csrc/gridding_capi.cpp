@@ -759,7 +759,7 @@ int anacor_gridding_interpolate(anacor_gridding *g, const double *s1, const doub
     // the host's lookups of one chunk beside the copy and the kernel of the
     // last (20,000 reflections bilinear, 1,658 voxels: 340 us of lookups, 37
     // of copy, 139 of kernel and 40 for a fresh array were 560 us in a row;
-    // a call is 530 us so, 625 before)
+    // a call is 360 us so)
     std::atomic<bool> ok{true};
     for (int64_t c = 0, k = 0; c < n && !e && ok; c += kStageRows, k++) {
         const int64_t m = std::min<int64_t>(kStageRows, n - c);
