@@ -237,7 +237,7 @@ constexpr size_t kStageBytes = kStageTables * sizeof(ReflTable);
 constexpr int kStageRows = (int)(kStageBytes / sizeof(InterpRow));
 // Launches of a map build: the first chunks at once, the rest when the device
 // is about to run out (512x512x400, 64,800 directions: the host needs 1.0 ms
-// for the tables, the device 4.9 ms for the map).
+// for the tables, the device 4.6 ms for the map).
 constexpr int kMapGroups = 3;
 constexpr long long kGroupEnd[kMapGroups - 1] = {kStageTables, 5 * kStageTables};
 

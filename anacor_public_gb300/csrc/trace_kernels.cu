@@ -900,15 +900,15 @@ __device__ __forceinline__ void trace_leg(const LegHead &h, const FaceRule *rule
 //    memory: 92 local loads a warp and leg then), what a march need not hold
 //    lies in shared memory at constant addresses (FieldShared; 10.2 -> 2.7
 //    local loads), and the kernel fits 48 registers, five CTAs an SM (six, at
-//    40 registers: 3 % slower);
+//    40 registers: 10 % slower, four 7 %);
 //  * everything rare (close exit-face calls, ratios beyond fixed point,
 //    full_iteration, legs that reach the wall limit, more than kMaxSegments
 //    class changes) is out of line in leg_slow, which reads the full rule
 //    from global memory.
-// 512x512x400, 13,266 voxels, 20,000 reflections: 30.0 -> 20.2 ms (1,430 ->
-// 915 warp instructions per 32 legs; L1 misses at 70 %, L2 at 59 % of their
-// peak rates, issue slots at 56 %).  1024x1024x800, all 11.7 million voxels,
-// 32 reflections: 22.9 -> 17.0 ms (18.6 with those 10.2 local loads).
+// 512x512x400, 13,266 voxels, 20,000 reflections: 30.0 -> 18.6 ms (1,430 ->
+// 852 warp instructions per 32 legs; L1 misses at 69 %, L2 at 60 % of their
+// peak rates, issue slots at 53 %).  1024x1024x800, every crystal voxel (6.8 million),
+// 32 reflections: 22.9 -> 16.9 ms (18.6 with those 10.2 local loads).
 
 // One leg's rule for one exit axis.  q: the 32.32 ratios of the two other
 // axes a and b (lo, hi words).  off: their initial low words -- the rounding
@@ -2261,8 +2261,9 @@ __global__ void __launch_bounds__(kBlock, 2) gridding_map_kernel(const MapDesc *
 // rounding to float open (a few in 10^5) map_slow evaluates the FP64
 // expressions.  On GB300 those bound the kernel before (a square root, the
 // quotients and the sums of every leg on an FP64 pipe of two lanes a cycle).
-// 64,800 directions x 1,657 voxels of a 512x512x400 volume: 14.8 -> 4.9 ms,
-// 3.9 with exit-face ties on the march (exact_axis).
+// 64,800 directions x 1,657 voxels of a 512x512x400 volume: 14.8 -> 4.9 ms
+// in one launch; in the launches of a build 4.6, exit-face ties on the march
+// (exact_axis), which left each of them a tail of 1 to 2 ms.
 __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *__restrict__ dp, long long total_items,
                                                               unsigned long long *__restrict__ work_counter,
                                                               float *__restrict__ out, long long ld,
