@@ -1170,11 +1170,12 @@ bool tune_lookup(const anacor_plan *p, TuneVal &v)
 // the octant-field march where it saves more than building the fields costs,
 // and the cooperative march for the rest.  Measured on whole drop-in calls:
 // the field march saves about 0.16 ps per leg and voxel of the longest axis
-// (0.13 at 512, 0.19 at 96, 0.3 at 160), the fields cost 110 us (launches, a
-// synchronisation) and 9 ps per voxel, 19 where rows are not whole 4-byte
-// words.  E.g. 96^3 voxels, 9,346 of them sampled: 300 reflections 590 us
-// cooperative, 655 on fields; 1,200: 1,420 and 1,125.  512 x 509 x 505 with
-// 26,685 sampled: 10 reflections 2.0 and 4.5 ms, 400: 4.4 and 5.5 ms.
+// (0.24 at 96), the fields cost 60 us (launches, a synchronisation) and 14 ps
+// per voxel, 20 where rows are not whole 4-byte words.  Cooperative and on
+// fields: 96^3 voxels, 11,740 of them sampled: 300 reflections 741 and 601 us,
+// 600 1,081 and 776; 160^3 with 6,787: 300 630 and 677; 160x150x170 with 5,595:
+// 600 838 and 747; 256x256x255 with 3,426: 1,000 1,115 and 1,279; 400^3 with
+// 13,266: 300 1.80 and 2.24 ms; 512x509x505 with 26,685: 300 3.4 and 4.9 ms.
 int plan_default_config(anacor_plan *p)
 {
     TuneVal v{0, 0, 1, 0.0f};
@@ -1184,7 +1185,7 @@ int plan_default_config(anacor_plan *p)
     const int big = std::max(p->dims[0], std::max(p->dims[1], p->dims[2]));
     const double nvol = (double)p->dims[0] * p->dims[1] * p->dims[2];
     const double saved_us = 0.16e-6 * 2.0 * (double)p->n_vox * (double)p->n_refl * big;
-    const double built_us = 110.0 + (p->dims[2] % 4 ? 19e-6 : 9e-6) * nvol;
+    const double built_us = 60.0 + (p->dims[2] % 4 ? 20e-6 : 14e-6) * nvol;
     if (!std::getenv("ANACOR_CTAS_PER_SM") && saved_us > built_us) {
         if (plan_ensure_field(p, 2) == kOk)
             variant = 12;
