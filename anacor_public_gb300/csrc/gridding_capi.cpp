@@ -237,7 +237,7 @@ constexpr size_t kStageBytes = kStageTables * sizeof(ReflTable);
 constexpr int kStageRows = (int)(kStageBytes / sizeof(InterpRow));
 // Launches of a map build: the first chunks at once, the rest when the device
 // is about to run out (512x512x400, 64,800 directions: the host needs 1.0 ms
-// for the tables, the device 4.6 ms for the map).
+// for the tables, the device 4.2 ms for the map).
 constexpr int kMapGroups = 3;
 constexpr long long kGroupEnd[kMapGroups - 1] = {kStageTables, 5 * kStageTables};
 
@@ -436,8 +436,9 @@ int run_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int i
 
 // The same on the view's octant fields, left on the stream: h_sample (page-
 // locked) and d_sample are this launch's until the stream has passed it.
-// Items of 512 voxels: a direction is a few of them, thousands of directions
-// fill the device.
+// Items of 256 voxels: a direction is a few of them, thousands of directions
+// fill the device, and a slow item's tail is short (64,800 directions x 1,657
+// voxels, whole call: 5.16 ms, of 128 5.17, of 512 5.52, of 1,024 6.3).
 cudaError_t enqueue_field_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int is_exp, float *out,
                               long long ld, SampleDesc *h_sample, SampleDesc *d_sample, unsigned long long *d_counter,
                               int *d_status, int grid, cudaStream_t st)
@@ -458,7 +459,7 @@ cudaError_t enqueue_field_map(const PlanView &pv, const ReflTable *d_dirs, long 
     d.coords = pv.coords;
     d.refl = d_dirs;
     d.n_refl = n_dirs;
-    d.tile = 512;
+    d.tile = 256;
     d.tiles = (pv.n_vox + d.tile - 1) / d.tile;
     d.full_iteration = pv.full_iteration;
     d.is_exp = is_exp;

@@ -916,7 +916,9 @@ __device__ __forceinline__ void trace_leg(const LegHead &h, const FaceRule *rule
 // below twice the margin (adding it changes the integer
 // part only there, where the exact expression is used).  A whole-numbered
 // ratio gets 2^31: its fraction stays one half, which is never ambiguous and
-// rounds to the exact integer in both modes.
+// rounds to the exact integer in both modes.  So does a ratio from 0 to 2^-33
+// (Q = 0; a map's directions along an axis): i * q is below 2^-19, so c + i * q
+// rounds to c either way.
 struct alignas(16) HotRule {
     uint32_t qa_lo, qa_hi, qb_lo, qb_hi;
     uint32_t off_a, off_b;
@@ -984,8 +986,8 @@ __device__ __forceinline__ void fill_warp_tab(WarpTab &w, const ReflTable *__res
         h.qb_lo = (uint32_t)Qb;
         h.qb_hi = (uint32_t)(Qb >> 32);
         const uint32_t off = (R.use_round ? 0x80000000u : 0u) + kFieldMargin;
-        h.off_a = (R.exact_mask >> ia) & 1 ? 0x80000000u : off;
-        h.off_b = (R.exact_mask >> ib) & 1 ? 0x80000000u : off;
+        h.off_a = (R.exact_mask >> ia) & 1 || (Qa == 0 && R.q[ia] >= 0.0) ? 0x80000000u : off;
+        h.off_b = (R.exact_mask >> ib) & 1 || (Qb == 0 && R.q[ib] >= 0.0) ? 0x80000000u : off;
         h.ds = R.Q[a] > 0 ? 1 : -1;
         const int sz = D.dim[1] * D.dim[2], sy = D.dim[2];
         h.dS = h.ds * pick3(a, sz, sy, 1);
