@@ -76,6 +76,14 @@ __device__ __forceinline__ FloatPair pair_mul(FloatPair a, FloatPair b)
     return pair_norm(p, __fmaf_rn(a.h, b.l, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.h, -p))));
 }
 
+// x * x, exact: a whole number of more than 12 bits has a square that a float
+// does not hold
+__device__ __forceinline__ FloatPair pair_square(float x)
+{
+    const float h = __fmul_rn(x, x);
+    return {h, __fmaf_rn(x, x, -h)};
+}
+
 // square root: one Newton step on the FP32 root
 __device__ __forceinline__ FloatPair pair_sqrt(FloatPair a)
 {

@@ -2259,7 +2259,8 @@ __global__ void __launch_bounds__(kBlock, 2) gridding_map_kernel(const MapDesc *
 
 // The absorption map on the octant fields, bit for bit the FP64 values rounded
 // to float: the reference's sum mu_m L_m = total / (len - 1) * sum mu_m span_m
-// is formed on pairs of floats (within 2^-43 of it), and where that leaves the
+// is formed on pairs of floats (within 2^-43 of it, the squared displacements
+// exact: those of an axis beyond 4,096 need 26 bits), and where that leaves the
 // rounding to float open (a few in 10^5) map_slow evaluates the FP64
 // expressions.  On GB300 those bound the kernel before (a square root, the
 // quotients and the sums of every leg on an FP64 pipe of two lanes a cycle).
@@ -2301,8 +2302,9 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
                 1, vi, [&] { return W.is_exp ? 1.0f : 0.0f; },
                 [&](int i, int nseg, int d0, int d1, int d2) {
                     const FloatPair tot = pair_sqrt(
-                        pair_add(pair_add(pair_mul(consts[0], (float)(d0 * d0)), pair_mul(consts[1], (float)(d1 * d1))),
-                                 pair_mul(consts[2], (float)(d2 * d2))));
+                        pair_add(pair_add(pair_mul(consts[0], pair_square((float)d0)),
+                                          pair_mul(consts[1], pair_square((float)d1))),
+                                 pair_mul(consts[2], pair_square((float)d2))));
                     FloatPair sum = {0.0f, 0.0f};
                     int cur = 3 << 13;
                     for (int j = 1; j <= nseg; j++) {
