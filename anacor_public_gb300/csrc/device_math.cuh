@@ -6,6 +6,13 @@
 
 namespace anacor {
 
+// Exponents beyond this are answered by exp_neg directly (exp(-4096) < 2^-5900
+// is 0 in FP32, exp(4096) infinite).  Their range reduction would go wrong:
+// where k ln2 no longer holds x's last bits (from about 1e17 in FP64, 1e9 on
+// pairs of floats) r lies far outside [-ln2/2, ln2/2], its expf overflows and
+// stays infinite under any scaling.
+constexpr float kExpBeyond = 4096.0f;
+
 // exp(-x) = 2^-k exp(-r) with the additive range reduction of exp by
 // multiples of ln 2 (Cody and Waite, "Software Manual for the Elementary
 // Functions", 1980, the exp chapter): k = rint(x / ln2), r = x - k ln2 in FP64
@@ -14,6 +21,8 @@ namespace anacor {
 // |r| <= ln2/2, and an exact scaling by 2^-k.
 __device__ __forceinline__ float exp_neg(double x)
 {
+    if (fabs(x) > (double)kExpBeyond && fabs(x) <= 1.7976931348623157e308)
+        return x > 0.0 ? 0.0f : __int_as_float(0x7f800000);
     const double kd = rint(__dmul_rn(x, 1.4426950408889634));
     const double r = __fma_rn(-kd, 0.6931471805599453, x);
     const float e = expf(-(float)r);
@@ -100,6 +109,8 @@ __device__ __forceinline__ FloatPair pair_sqrt(FloatPair a)
 // its product with k is exact.
 __device__ __forceinline__ float exp_neg(FloatPair x)
 {
+    if (fabsf(x.h) > kExpBeyond && fabsf(x.h) <= 3.402823466e38f)
+        return x.h > 0.0f ? 0.0f : __int_as_float(0x7f800000);
     const float k = rintf(__fmul_rn(x.h, 1.44269504f));
     const float c1 = 2839.0f / 4096.0f;
     const float c2 = 0x1.0bfbe80000000p-15f;
