@@ -2283,8 +2283,14 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
     else if (tid < 7)
         consts[tid] = pair_of(D.mu[tid - 3]);
     __syncthreads();
-    // the error bound is relative to the sum: no cancellation between terms
-    const bool positive = D.mu[0] >= 0.0 && D.mu[1] >= 0.0 && D.mu[2] >= 0.0 && D.mu[3] >= 0.0;
+    // The error bound is relative to the sum: no cancellation between terms,
+    // and squares that a float's range holds.  Every class counts, an absent
+    // one with length zero: infinite or undefined coefficients give NaN for it.
+    bool plain = true;
+    for (int a = 0; a < 4; a++)
+        plain = plain && D.mu[a] >= 0.0 && D.mu[a] < 1e300;
+    for (int a = 0; a < 3; a++)
+        plain = plain && fabs(D.voxel[a]) > 0x1p-40 && fabs(D.voxel[a]) < 0x1p40;
     for (;;) {
         unsigned long long it = 0;
         if (lane == 0)
@@ -2299,7 +2305,10 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
         __syncwarp();
         for (int vi = lane; vi < W.n; vi += 32) {
             const float val = field_march<false, true>(
-                1, vi, [&] { return W.is_exp ? 1.0f : 0.0f; },
+                1, vi,
+                [&] {
+                    return !plain ? map_slow(vi, kFromStart, 0, 0, 1, 0, 0, -1, 0, 0) : (W.is_exp ? 1.0f : 0.0f);
+                },
                 [&](int i, int nseg, int d0, int d1, int d2) {
                     const FloatPair tot = pair_sqrt(
                         pair_add(pair_add(pair_mul(consts[0], pair_square((float)d0)),
@@ -2331,7 +2340,7 @@ __global__ void __launch_bounds__(kBlock, 5) field_map_kernel(const SampleDesc *
                         v = r.h;
                         sure = __fadd_rn(r.h, r.l + err) == r.h && __fadd_rn(r.h, r.l - err) == r.h && r.h > 0x1p-80f;
                     }
-                    return positive && sure ? v
+                    return plain && sure ? v
                                             : map_slow(vi, kFromStop, 0, i, nseg, 0, 0, d0, d1, d2);
                 },
                 [&](int from, int axis, int i, int nseg, int prev, int lim) {
