@@ -970,7 +970,13 @@ int plan_launch_bisection(anacor_plan *p, cudaStream_t st, int num_cls)
     const long long items = (long long)p->n_refl * p->tiles;
     if (items == 0)
         return kOk;
-    const bool fixed = std::max(p->dims[0], std::max(p->dims[1], p->dims[2])) <= kBisectFixedDim;
+    // the fixed-point searches' lengths and exponents run on pairs of floats:
+    // edges whose squares, and coefficients that, a float's range holds
+    bool fixed = std::max(p->dims[0], std::max(p->dims[1], p->dims[2])) <= kBisectFixedDim;
+    for (int a = 0; a < 3; a++)
+        fixed = fixed && std::fabs(p->voxel[a]) > 0x1p-40 && std::fabs(p->voxel[a]) < 0x1p40;
+    for (int a = 0; a < 4; a++)
+        fixed = fixed && std::fabs(p->mu[a]) < 0x1p60;
     int bps = 0;
     if (bisection_occupancy(&bps, fixed) != kOk || bps <= 0)
         bps = 1;

@@ -177,7 +177,8 @@ cudaError_t launch_leg_detail(const ReflTable *d_tab, const int8_t *d_vol, const
 // The reference's iterative-bisection variant (ib_test) over the same work
 // items as launch_absorption; num_cls > 3 also searches bubble boundaries.
 // `fixed`: the fixed-point searches, for volumes with axes of at most
-// kBisectFixedDim voxels; else the FP64 ones.
+// kBisectFixedDim voxels whose edges and coefficients lie well inside FP32's
+// range; else the FP64 ones.
 constexpr int kBisectFixedDim = 1023;
 cudaError_t launch_bisection(const SampleDesc *d_descs, int n_desc, long long total_items,
                              unsigned long long *d_counter, int grid, int num_cls, bool fixed, cudaStream_t st);
