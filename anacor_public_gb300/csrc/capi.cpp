@@ -292,7 +292,9 @@ struct anacor_plan {
     int field8_state = 0;
     uint8_t *d_field8b = nullptr;  // the same in 4^3 bricks, built on first use by variants 13..16
     int field8b_state = 0;
-    int *d_walls = nullptr;        // [6] room between the non-vacuum labels and the walls, built with a field
+    // [6] room between the non-vacuum labels and the walls, made with the first
+    // field and never written again: launches in flight, on any stream, read it
+    int *d_walls = nullptr;
     // One allocation each: status, counter, descriptor and squared lengths;
     // and what is sized by the reflections (tables, results, arrivals, order).
     uint8_t *d_fixed = nullptr, *d_per_refl = nullptr;
@@ -767,21 +769,25 @@ int plan_ensure_field(anacor_plan *p, int kind = 1)
     const size_t nvol = (size_t)p->dims[0] * p->dims[1] * p->dims[2];
     const size_t copies = kind == 2 ? 8 : 1, tmp_copies = kind == 2 ? 6 : 1;
     uint8_t *tmp = nullptr;
-    int *d_bad = nullptr;
+    int *d_bad = nullptr, *walls = nullptr;   // published once they have been written
     int bad = 0;
     cudaError_t e;
     if ((e = dev_alloc(&field, nvol * copies, st)) || (e = dev_alloc(&tmp, nvol * tmp_copies, st)) ||
-        (e = dev_alloc(&d_bad, 1, st)) || (!p->d_walls && (e = dev_alloc(&p->d_walls, 6, st))) ||
-        (e = launch_wall_room(p->d_vol, p->dims, p->d_walls, st)) ||
+        (e = dev_alloc(&d_bad, 1, st)) ||
+        (!p->d_walls &&
+         ((e = dev_alloc(&walls, 6, st)) || (e = launch_wall_room(p->d_vol, p->dims, walls, st)))) ||
         (e = kind == 2 ? launch_octant_fields(p->d_vol, p->dims, field, tmp, d_bad, st)
                        : launch_distance_field(p->d_vol, p->dims, field, tmp, d_bad, st)) ||
         (e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
         (e = cudaStreamSynchronize(st))) {
         dev_free(tmp, st);
         dev_free(d_bad, st);
+        dev_free(walls, st);
         dev_free(field, st);
         return cuda_fail(e, "distance field");
     }
+    if (walls)
+        p->d_walls = walls;
     dev_free(tmp, st);
     dev_free(d_bad, st);
     if (bad) {
