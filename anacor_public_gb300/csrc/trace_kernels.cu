@@ -1410,59 +1410,6 @@ __device__ __forceinline__ int find_sample(const SampleDesc *d, int n, long long
     return s;
 }
 
-// End of a work item: block reduction of the per-thread compensated sums
-// (warp-shuffle TwoSum, then across warps), the item's FP64 partial, and --
-// for the last tile of the reflection to arrive -- the fixed-order
-// combination of the partials into A_h.
-__device__ __forceinline__ void finish_item(float s, float c, const SampleDesc &D, long long r, int t, float *red_s,
-                                            float *red_c, int &last_s)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float so = __shfl_down_sync(kAll, s, o);
-        const float co = __shfl_down_sync(kAll, c, o);
-        float ns, e;
-        two_sum(s, so, ns, e);
-        s = ns;
-        c = c + co + e;
-    }
-    if (lane == 0) {
-        red_s[warp] = s;
-        red_c[warp] = c;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        float bs = red_s[0], bc = red_c[0];
-        for (int w = 1; w < kWarps; w++) {
-            float ns, e;
-            two_sum(bs, red_s[w], ns, e);
-            bs = ns;
-            bc = bc + red_c[w] + e;
-        }
-        D.partial[r * D.tiles + t] = (double)bs + (double)bc;
-        __threadfence();
-        const unsigned prev = atomicAdd(D.arrive + r, 1u);
-        last_s = prev == (unsigned)(D.tiles - 1);
-    }
-    __syncthreads();
-    if (last_s && warp == 0) {
-        // the last tile of this reflection combines all partials in a fixed order
-        __threadfence();
-        const volatile double *pp = D.partial + r * D.tiles;
-        double acc = 0.0;
-        for (int k = lane; k < D.tiles; k += 32)
-            acc += pp[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            acc += __shfl_down_sync(kAll, acc, o);
-        if (lane == 0) {
-            D.out[r] = acc / (double)D.n_vox;
-            D.arrive[r] = 0u;   // ready for the next launch
-        }
-    }
-}
-
 // The end of an absorption work item: the warp's compensated sum, the item's
 // FP64 partial and, for the last tile of the reflection to arrive, the
 // fixed-order combination of the partials into A_h.
@@ -1851,23 +1798,24 @@ __global__ void __launch_bounds__(kBlock) ib_direction_kernel(const ReflTable *_
 }
 
 // ib_test over every work item: as absorption_kernel, with bisection paths.
+// An item a warp, as plan_split cuts them (down to one voxel a lane): with an
+// item a block, 20 reflections of 20,000 voxels (1100x220x210) left seven
+// warps of eight idle.
 __global__ void __launch_bounds__(kBlock, 2) bisection_kernel(const SampleDesc *__restrict__ descs, int n_desc,
                                                               long long total_items,
                                                               unsigned long long *__restrict__ work_counter,
                                                               int num_cls)
 {
-    __shared__ ReflTable tab;
-    __shared__ float red_s[kWarps], red_c[kWarps];
-    __shared__ long long item_s;
-    __shared__ int last_s;
+    __shared__ ReflTable tabs[kWarps];
     if (!block_shape_ok(n_desc > 0 ? descs[0].status : nullptr))
         return;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
+    ReflTable &tab = tabs[tid >> 5];
     for (;;) {
-        if (tid == 0)
-            item_s = (long long)atomicAdd(work_counter, 1ull);
-        __syncthreads();
-        const long long item = item_s;
+        unsigned long long it = 0;
+        if (lane == 0)
+            it = atomicAdd(work_counter, 1ull);
+        const long long item = (long long)__shfl_sync(kAll, it, 0);
         if (item >= total_items)
             break;
         const int si = find_sample(descs, n_desc, item);
@@ -1876,25 +1824,25 @@ __global__ void __launch_bounds__(kBlock, 2) bisection_kernel(const SampleDesc *
         const long long k = local / D.tiles;
         const long long r = D.order ? (long long)__ldg(D.order + k) : k;
         const int t = (int)(local - k * D.tiles);
+        __syncwarp();   // the previous item's reads of the table are done
         {
             const int4 *src = reinterpret_cast<const int4 *>(D.refl + r);
             int4 *dst = reinterpret_cast<int4 *>(&tab);
-            for (int k = tid; k < (int)(sizeof(ReflTable) / 16); k += kBlock)
+            for (int k = lane; k < (int)(sizeof(ReflTable) / 16); k += 32)
                 dst[k] = __ldg(src + k);
         }
-        __syncthreads();
+        __syncwarp();
         const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
         float s = 0.0f, c = 0.0f;
-        int bad = kOk;
         const int v1 = min(D.n_vox, (t + 1) * D.tile);
-        for (int vi = t * D.tile + tid; vi < v1; vi += kBlock) {
+        for (int vi = t * D.tile + lane; vi < v1; vi += 32) {
             const short4 cv = __ldg(D.coords + vi);
             double a[4], b[4];
             int st = ib_leg(tab.head[0], tab.rule[0], cv.x, cv.y, cv.z, v, num_cls, D.voxel, a);
             if (!st)
                 st = ib_leg(tab.head[1], tab.rule[1], cv.x, cv.y, cv.z, v, num_cls, D.voxel, b);
             if (st) {
-                bad |= st;
+                atomicOr(D.status, 1 << st);
                 continue;
             }
             // cal_rate, operand order of AnACor/src/ray_tracing_basic.c:1573-1576
@@ -1908,9 +1856,8 @@ __global__ void __launch_bounds__(kBlock, 2) bisection_kernel(const SampleDesc *
             s = ns;
             c += e;
         }
-        if (bad)
-            atomicOr(D.status, 1 << bad);
-        finish_item(s, c, D, r, t, red_s, red_c, last_s);
+        __syncwarp();
+        finish_warp_item(s, c, D, r, t, lane);
     }
 }
 
