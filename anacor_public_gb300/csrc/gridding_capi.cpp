@@ -633,6 +633,7 @@ int anacor_gridding_build(anacor_gridding *g, const double *rotated_s1, const do
         if ((e = stage_upload(g, b, 0, d_dirs + c, (size_t)n * sizeof(ReflTable), launch || done == G, st)))
             break;
         if (launch) {
+            g->built = false;   // the map is being written to
             e = enqueue_field_map(g->pv, d_dirs + launched, done - launched, g->method == 1,
                                   g->d_map + launched * g->ld, g->ld, h_sample + group, g->d_sample + group,
                                   g->d_counter, g->d_status, g->map_grid, st);
@@ -641,12 +642,18 @@ int anacor_gridding_build(anacor_gridding *g, const double *rotated_s1, const do
         }
     }
     int r = e ? cuda_err(e) : bad ? report_status(bad, "gridding: non-finite or zero grid direction") : kOk;
-    if (!r)
+    if (!r) {
+        g->built = false;
         r = g->pv.field ? check_map_status(g->d_status, st)
                         : run_map(g->pv, d_dirs, G, g->method == 1, g->pv.mu, g->d_map, nullptr, g->ld, nullptr,
                                   g->d_desc, g->d_counter, g->d_status, g->map_grid, st);
-    if (r)
-        cudaStreamSynchronize(g->copy);   // nothing may still be writing the tables
+    }
+    if (r) {
+        // nothing may still be writing the tables, or reading the staged
+        // descriptors that the next build writes
+        cudaStreamSynchronize(g->copy);
+        cudaStreamSynchronize(st);
+    }
     cudaFreeAsync(d_dirs, st);
     if (r)
         return r;
