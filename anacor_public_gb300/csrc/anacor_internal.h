@@ -66,6 +66,23 @@ struct alignas(16) FaceRule {
 };
 static_assert(sizeof(FaceRule) == 64, "FaceRule layout");
 
+#ifdef __CUDACC__
+#define ANACOR_BOTH __host__ __device__ __forceinline__
+#else
+#define ANACOR_BOTH inline
+#endif
+
+// A leg on the fields needs no wall limit ("free") when the volume's
+// non-vacuum labels keep free_leg_room voxels from every wall it moves toward:
+// the increment examined after a non-vacuum one lies at most ceil(|q|) voxels
+// further on each axis, so it meets vacuum before an increment can clamp, with
+// one voxel to spare for a fixed-point position near a rounding boundary.
+// qmax: the larger |Q| of the two axes besides the step axis.
+ANACOR_BOTH int free_leg_room(long long qmax) { return (int)(qmax >> 32) + 2; }
+// The wall ahead on an axis as an index into a sample's six rooms (0..2 the
+// walls at coordinate 0 of z, y, x; 3..5 the far ones); octant as FaceRule's.
+ANACOR_BOTH int wall_ahead(int octant, int axis) { return (octant >> (2 - axis)) & 1 ? axis : 3 + axis; }
+
 // Direction data for the exit-face test of one leg (AnACor/src/ray_tracing_basic.c:69-186).
 // e is the my-frame direction (z, y, x components), negated for the incident leg
 // so that every candidate distance is fl(n / |e_a|).

@@ -1000,20 +1000,13 @@ __device__ __forceinline__ void fill_warp_tab(WarpTab &w, const ReflTable *__res
         uint32_t f = 0u;
         if (R.fast && !R.status && !D.full_iteration && !zero) {
             f |= kHotSimple;
-            // The examined increment after a non-vacuum one lies at most
-            // ceil(|q|) voxels further on each axis: when the non-vacuum
-            // labels keep that distance (and one more) from the walls the leg
-            // moves toward, it meets vacuum before a clamped increment, and
-            // before the last one of its face.
+            // see free_leg_room; such a leg also stops before its face's last increment
             if (D.walls) {
-                const long long qm = max(Qa < 0 ? -Qa : Qa, Qb < 0 ? -Qb : Qb);
-                const int need = (int)(qm >> 32) + 2;
+                const int need = free_leg_room(max(Qa < 0 ? -Qa : Qa, Qb < 0 ? -Qb : Qb));
                 bool free_leg = true;
 #pragma unroll
-                for (int x = 0; x < 3; x++) {
-                    const bool back = (R.octant >> (2 - x)) & 1;   // toward coordinate 0
-                    free_leg = free_leg && __ldg(D.walls + (back ? x : 3 + x)) >= need;
-                }
+                for (int x = 0; x < 3; x++)
+                    free_leg = free_leg && __ldg(D.walls + wall_ahead(R.octant, x)) >= need;
                 if (free_leg)
                     f |= kHotFree;
             }
