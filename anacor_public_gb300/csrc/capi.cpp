@@ -265,7 +265,7 @@ struct anacor_plan {
     short4 *d_coords = nullptr;
     ReflTable *d_refl = nullptr;
     double *d_out = nullptr;
-    double *d_partial = nullptr;
+    float2 *d_partial = nullptr;
     unsigned *d_arrive = nullptr;
     int *d_status = nullptr;
     unsigned long long *d_counter = nullptr;
@@ -279,7 +279,7 @@ struct anacor_plan {
     int *d_order = nullptr;        // processing order of the reflections (grouped by direction octants)
     std::vector<int> h_order;
     int64_t n_refl = 0, refl_cap = 0;
-    size_t partial_cap = 0;        // entries of d_partial (refl_cap * tiles)
+    size_t partial_cap = 0;        // entries of d_partial (refl_cap * tiles); their third floats follow
     int tiles = 0;
     int tile = kTile;              // most voxels of a work item (the configured tile)
     int work_tile = kTile;         // voxels per work item (plan_split)
@@ -516,7 +516,7 @@ int effective_tile(int n_vox, int tile)
 // reflections still fills the device (3,001 reflections of 1,150 voxels: 926
 // us at one item a warp, 810 at four, 840 at nine; six samples in one batch,
 // whose items are many already: 3.98 ms, 4.01, 4.26).  The per-voxel terms are
-// summed with compensation, so the split changes A_h by less than 1e-12.
+// summed exactly (FloatSum, finish_warp_item), so the split does not show in A_h.
 int plan_ensure_partial(anacor_plan *p);
 long long wanted_items(const anacor_plan *p) { return (long long)p->dev->sms * 40 * kItemsPerWarp; }
 int plan_split(anacor_plan *p)
@@ -693,7 +693,7 @@ int plan_ensure_partial(anacor_plan *p)
     cudaStream_t st = p->stream;
     dev_free(p->d_partial, st);
     p->partial_cap = 0;
-    if (cudaError_t e = dev_alloc(&p->d_partial, need, st))
+    if (cudaError_t e = dev_alloc(&p->d_partial, need + (need + 1) / 2, st))
         return cuda_fail(e, "device allocation");
     p->partial_cap = need;
     return kOk;
@@ -846,6 +846,7 @@ SampleDesc plan_desc(const anacor_plan *p, long long work_begin, int fk = -1, bo
     d.is_exp = p->is_exp;
     d.out = p->d_out;
     d.partial = p->d_partial;
+    d.partial_low = reinterpret_cast<float *>(p->d_partial + p->partial_cap);
     d.arrive = p->d_arrive;
     d.status = p->d_status;
     d.sq = p->d_sq;

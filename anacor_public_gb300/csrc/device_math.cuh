@@ -38,6 +38,40 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
     e = (a - (s - bp)) + (b - bp);
 }
 
+// A sum of floats as three: each holds what the ones before it round away
+// (72 bits), so it is exact while the terms lie within about 2^40 of each other
+// and the order of the terms does not matter.
+struct FloatSum {
+    float s, c, d;
+};
+
+__device__ __forceinline__ void sum_add(FloatSum &a, float x)
+{
+    float s, c, e, f;
+    two_sum(a.s, x, s, e);
+    two_sum(a.c, e, c, f);
+    a.s = s;
+    a.c = c;
+    a.d += f;
+}
+
+__device__ __forceinline__ void sum_merge(FloatSum &a, float s, float c, float d)
+{
+    sum_add(a, s);
+    float h, f;
+    two_sum(a.c, c, h, f);
+    a.c = h;
+    a.d += d + f;
+}
+
+// the same in FP64, s + e exactly a + b
+__device__ __forceinline__ void two_sum(double a, double b, double &s, double &e)
+{
+    s = __dadd_rn(a, b);
+    const double bp = __dadd_rn(s, -a);
+    e = __dadd_rn(__dadd_rn(a, -__dadd_rn(s, -bp)), __dadd_rn(b, -bp));
+}
+
 // ---- pairs of floats (h + l, |l| <= ulp(h) / 2) ----------------------------
 //
 // About 46 significant bits from FP32 instructions (Dekker, "A floating-point

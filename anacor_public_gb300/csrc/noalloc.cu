@@ -131,7 +131,7 @@ extern "C" int anacor_absorption_noalloc(const int8_t *d_label, const int64_t *s
     const size_t off_coords = align256(off_status + sizeof(int));
     const size_t off_tables = align256(off_coords + (size_t)n_coords * sizeof(short4));
     const size_t off_partial = align256(off_tables + (size_t)n_refl * sizeof(ReflTable));
-    const size_t off_arrive = align256(off_partial + (size_t)n_refl * (size_t)tiles * sizeof(double));
+    const size_t off_arrive = align256(off_partial + (size_t)n_refl * (size_t)tiles * sizeof(float2));
     const size_t need = align256(off_arrive + (size_t)n_refl * sizeof(unsigned));
     if (need > kScratchBytes) {
         char msg[256];
@@ -151,7 +151,7 @@ extern "C" int anacor_absorption_noalloc(const int8_t *d_label, const int64_t *s
     int *d_status = reinterpret_cast<int *>(base + off_status);
     short4 *d_pack = reinterpret_cast<short4 *>(base + off_coords);
     ReflTable *d_tables = reinterpret_cast<ReflTable *>(base + off_tables);
-    double *d_partial = reinterpret_cast<double *>(base + off_partial);
+    float2 *d_partial = reinterpret_cast<float2 *>(base + off_partial);
     unsigned *d_arrive = reinterpret_cast<unsigned *>(base + off_arrive);
     SampleDesc *d_desc = reinterpret_cast<SampleDesc *>(base + off_desc);
     unsigned long long *d_counter = reinterpret_cast<unsigned long long *>(base + off_counter);

@@ -1078,7 +1078,8 @@ struct FieldShared {
     WarpTab tabs[kWarps];
     uint16_t seg[kSegRows * kBlock];
     float4 incident[kBlock];     // the incident leg's lengths while the diffracted leg marches
-    float2 total[kBlock];        // compensated sums
+    float2 total[kBlock];        // the lanes' sums (FloatSum)
+    float total_low[kBlock];
     unsigned steps[kBlock];
     FloatPair consts[7];         // map kernel: squared voxel edges (z, y, x), mu
 };
@@ -1403,37 +1404,44 @@ __device__ __forceinline__ int find_sample(const SampleDesc *d, int n, long long
     return s;
 }
 
-// The end of an absorption work item: the warp's compensated sum, the item's
-// FP64 partial and, for the last tile of the reflection to arrive, the
-// fixed-order combination of the partials into A_h.
-__device__ __forceinline__ void finish_warp_item(float s, float c, const SampleDesc &D, long long r, int t, int lane)
+// The end of an absorption work item: the warp's sum, the item's partial sum
+// and, for the last tile of the reflection to arrive, the combination of the
+// partials into A_h.  The sums stay three floats (FloatSum) to the end, exact as
+// far as those go, so A_h has the same bits however the voxels are cut into
+// items: for a full set of reflections, a part of it and in a batch.  (A launch
+// without room for the third floats folds them in.)
+__device__ __forceinline__ void finish_warp_item(FloatSum a, const SampleDesc &D, long long r, int t, int lane)
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float so = __shfl_down_sync(kAll, s, o);
-        const float co = __shfl_down_sync(kAll, c, o);
-        float ns, e;
-        two_sum(s, so, ns, e);
-        s = ns;
-        c = c + co + e;
-    }
+    for (int o = 16; o > 0; o >>= 1)
+        sum_merge(a, __shfl_down_sync(kAll, a.s, o), __shfl_down_sync(kAll, a.c, o), __shfl_down_sync(kAll, a.d, o));
     int last = 0;
     if (lane == 0) {
-        D.partial[r * D.tiles + t] = (double)s + (double)c;
+        const long long at = r * D.tiles + t;
+        if (D.partial_low)
+            D.partial_low[at] = a.d;
+        else
+            a.c += a.d;
+        D.partial[at] = make_float2(a.s, a.c);
         __threadfence();
         last = atomicAdd(D.arrive + r, 1u) == (unsigned)(D.tiles - 1);
     }
     if (__shfl_sync(kAll, last, 0)) {
         __threadfence();
-        const volatile double *pp = D.partial + r * D.tiles;
-        double acc = 0.0;
-        for (int k = lane; k < D.tiles; k += 32)
-            acc += pp[k];
+        const float2 *sc = D.partial + r * D.tiles;
+        const float *low = D.partial_low ? D.partial_low + r * D.tiles : nullptr;
+        a = {0.0f, 0.0f, 0.0f};
+        for (int k = lane; k < D.tiles; k += 32) {
+            const float2 p = __ldcg(sc + k);
+            sum_merge(a, p.x, p.y, low ? __ldcg(low + k) : 0.0f);
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
-            acc += __shfl_down_sync(kAll, acc, o);
+            sum_merge(a, __shfl_down_sync(kAll, a.s, o), __shfl_down_sync(kAll, a.c, o), __shfl_down_sync(kAll, a.d, o));
         if (lane == 0) {
-            D.out[r] = acc / (double)D.n_vox;
+            double h, l;
+            two_sum((double)a.s, (double)a.c, h, l);
+            D.out[r] = (h + (l + (double)a.d)) / (double)D.n_vox;
             D.arrive[r] = 0u;   // ready for the next launch
         }
     }
@@ -1476,7 +1484,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
         __syncwarp();
 
         const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
-        float s = 0.0f, c = 0.0f;
+        FloatSum sum = {0.0f, 0.0f, 0.0f};
         int bad = kOk;
         unsigned nsteps = 0;
         const int v0 = t * D.tile;
@@ -1506,10 +1514,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
                 const float ex = D.muf[0] * lsum[0][tid] + D.muf[1] * lsum[1][tid] + D.muf[2] * lsum[2][tid] +
                                  D.muf[3] * lsum[3][tid];
                 const float term = D.is_exp ? expf(-ex) : ex;
-                float ns, e;
-                two_sum(s, term, ns, e);
-                s = ns;
-                c += e;
+                sum_add(sum, term);
             }
         }
         if (bad)
@@ -1522,7 +1527,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) absorption_kernel(const Sa
             if (lane == 0)
                 atomicAdd(D.steps, w);
         }
-        finish_warp_item(s, c, D, r, t, lane);
+        finish_warp_item(sum, D, r, t, lane);
     }
 }
 
@@ -1560,6 +1565,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks + 1) field_kernel(const Sam
         __syncwarp();
 
         S.total[thread_now()] = make_float2(0.0f, 0.0f);
+        S.total_low[thread_now()] = 0.0f;
         S.steps[thread_now()] = 0u;
         for (int vi = lane; vi < warp_tab().n; vi += 32) {
             float4 L;
@@ -1582,9 +1588,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks + 1) field_kernel(const Sam
                              W.mu[3] * (I.w + L.w);
             const float term = W.is_exp ? expf(-ex) : ex;
             const float2 sc = S.total[tid];
-            float ns, e;
-            two_sum(sc.x, term, ns, e);
-            S.total[tid] = make_float2(ns, sc.y + e);
+            FloatSum sum = {sc.x, sc.y, S.total_low[tid]};
+            sum_add(sum, term);
+            S.total[tid] = make_float2(sum.s, sum.c);
+            S.total_low[tid] = sum.d;
         }
         __syncwarp();
         if (D.steps) {
@@ -1597,7 +1604,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks + 1) field_kernel(const Sam
         }
         {
             const float2 sc = S.total[thread_now()];
-            finish_warp_item(sc.x, sc.y, D, r, t, lane);
+            finish_warp_item({sc.x, sc.y, S.total_low[thread_now()]}, D, r, t, lane);
         }
     }
 }
@@ -1826,7 +1833,7 @@ __global__ void __launch_bounds__(kBlock, 2) bisection_kernel(const SampleDesc *
         }
         __syncwarp();
         const Vol v{D.vol, D.dim[0], D.dim[1], D.dim[2]};
-        float s = 0.0f, c = 0.0f;
+        FloatSum sum = {0.0f, 0.0f, 0.0f};
         const int v1 = min(D.n_vox, (t + 1) * D.tile);
         for (int vi = t * D.tile + lane; vi < v1; vi += 32) {
             const short4 cv = __ldg(D.coords + vi);
@@ -1844,13 +1851,10 @@ __global__ void __launch_bounds__(kBlock, 2) bisection_kernel(const SampleDesc *
             const double t2 = __dmul_rn(D.mu[2], __dadd_rn(a[2], b[2]));
             const double t3 = __dmul_rn(D.mu[3], __dadd_rn(a[3], b[3]));
             const double ex = __dadd_rn(__dadd_rn(__dadd_rn(t0, t1), t2), t3);
-            float ns, e;
-            two_sum(s, exp_neg(ex), ns, e);
-            s = ns;
-            c += e;
+            sum_add(sum, exp_neg(ex));
         }
         __syncwarp();
-        finish_warp_item(s, c, D, r, t, lane);
+        finish_warp_item(sum, D, r, t, lane);
     }
 }
 
@@ -2027,6 +2031,7 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
 {
     __shared__ WarpTab tabs[kWarps];
     __shared__ FloatPair consts[kWarps][7];   // squared voxel edges (z, y, x), mu
+    __shared__ FloatSum sums[kBlock];         // the lanes' sums: in registers they spill what a search needs
     if (!block_shape_ok(n_desc > 0 ? descs[0].status : nullptr))
         return;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -2051,7 +2056,7 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
         else if (lane < 7)
             K[lane] = pair_of(D.mu[lane - 3]);
         __syncwarp();
-        float s = 0.0f, c = 0.0f;
+        sums[tid] = {0.0f, 0.0f, 0.0f};
         const int n = min(D.tile, D.n_vox - t * D.tile);
         const short4 *coords = D.coords + (long long)t * D.tile;
         for (int vi = lane; vi < n; vi += 32) {
@@ -2120,13 +2125,10 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
 #pragma unroll
             for (int m = 0; m < 4; m++)
                 ex = pair_add(ex, pair_mul(pair_add(L[0][m], L[1][m]), K[3 + m]));
-            float ns, e;
-            two_sum(s, exp_neg(ex), ns, e);
-            s = ns;
-            c += e;
+            sum_add(sums[tid], exp_neg(ex));
         }
         __syncwarp();
-        finish_warp_item(s, c, D, refl, t, lane);
+        finish_warp_item(sums[tid], D, refl, t, lane);
     }
 }
 

@@ -11,7 +11,7 @@ namespace anacor {
 
 // Voxels per work item unless a sample sets its own: a sample with N voxels
 // and R reflections is R * ceil(N / tile) work items (taken per warp by the
-// absorption kernel, per CTA by the map and bisection kernels).
+// absorption and bisection kernels, per CTA by the map kernel).
 constexpr int kTile = 2048;
 constexpr int kMinTile = 128;
 // A plan's tile is raised where needed so that a reflection has at most this
@@ -36,7 +36,8 @@ struct SampleDesc {
     float voxelf[3];        // (float) voxel, for the FP32 lengths of A_h
     float muf[4];           // (float) mu, for the FP32 exponent of A_h
     double *out;            // [n_refl]
-    double *partial;        // [n_refl * tiles] scratch
+    float2 *partial;        // [n_refl * tiles] scratch: the items' sums (FloatSum's first two floats)
+    float *partial_low;     // their third floats, or null
     unsigned int *arrive;   // [n_refl] scratch, zero before the first launch
     int *status;            // bit (1 << code) set for every failing voxel's status
     unsigned long long *steps;  // optional: += sum of len_path_2 over all rays
@@ -115,8 +116,8 @@ int absorption_block_threads();
 int block_guard_selftest(int threads, int *status_out);
 int absorption_set_carveout(int pct, int field_pct);
 // Kernel variants: 1..4 the cooperative march with a register budget for
-// 1..4 CTAs per SM; 5..8 the same budgets with the distance-field march on
-// linear fields; 9..12 on 4^3-bricked fields (every sample needs its `field`
+// 1..4 CTAs per SM; 5..8 the distance-field march on linear fields, for 2..5;
+// 9..12 on 4^3-bricked fields (every sample needs its `field`
 // in the variant's layout).
 constexpr int kVariants = 12;
 // CTAs per SM of a variant (0 = the process default)

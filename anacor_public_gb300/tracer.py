@@ -139,10 +139,13 @@ class Plan:
     def configure(self, variant: int = 0, tile: int = 0, order: int = -1):
         """Execution parameters.  variant: 1..4 the warp-cooperative march
         compiled for 1..4 CTAs per SM, 5..8 the march on the chessboard distance
-        field, 9..12 on the 8 octant fields, 13..16 on the octant fields stored
-        in 4x4x4 bricks (fields need labels in 0..7), 0 the process default; tile: voxels per work item (0 unchanged); order: voxel
-        order (0 the caller's, 1 Morton, 2..7 blocked, -1 unchanged).  Results
-        do not depend on them beyond the FP32 summation order of A_h."""
+        field compiled for 2..5, 9..12 on the 8 octant fields, 13..16 on the
+        octant fields stored in 4x4x4 bricks (fields need labels in 0..7), 0 the
+        process default; tile: most voxels of a work item (0 unchanged; launches
+        that would have few items halve it, down to 32); order: voxel order (0
+        the caller's, 1 Morton, 2..7 blocked, -1 unchanged).  Results do not
+        depend on them, nor A_h's bits while its terms lie within about 2^40 of
+        each other (beyond that, its last ones)."""
         _lib.check(self._L.anacor_plan_configure(self._h, int(variant), int(tile), int(order)), self._L)
 
     def config(self) -> dict:

@@ -140,18 +140,20 @@ int anacor_bisection(const int8_t *label, const int64_t *shape, const int64_t *c
                      double *out);
 
 /* Execution parameters of a plan (no counterpart in the reference; they do
- * not change the per-ray results, only the FP32 summation order of A_h):
+ * not change the per-ray results; the per-voxel terms are summed exactly while
+ * they lie within about 2^40 of each other, so A_h has the same bits too):
  * variant = kernel variant: 1..4 the warp-cooperative march compiled for
- * 1..4 CTAs per SM, 5..8 the same register budgets with the distance-field
- * march (steps over increments that a chessboard distance field proves to
- * keep the label; needs labels in 0..7, else kErrUnsupported), 9..12 the
- * same on the 8 octant fields (each leg reads the field of its direction's
- * octant), 13..16 the same on a copy of the octant fields stored in 4x4x4
- * bricks of 64 bytes (a ray's next step along any axis mostly stays in the
- * 32-byte sector of its last load), 0 = process default; tile = voxels per
- * work item
- * (>= 128, 0 = unchanged); order = voxel order of the packed list: 0 the
- * caller's, 1 Morton (Z-order) of (z, y, x), 2..7 blocked (Morton order of
+ * 1..4 CTAs per SM, 5..8 the distance-field march compiled for 2..5 (steps
+ * over increments that a chessboard distance field proves to keep the label;
+ * needs labels in 0..7, else kErrUnsupported), 9..12 the same on the 8 octant
+ * fields (each leg reads the field of its direction's octant), 13..16 the same
+ * on a copy of the octant fields stored in 4x4x4 bricks of 64 bytes (a ray's
+ * next step along any axis mostly stays in the 32-byte sector of its last
+ * load), 0 = process default; a plan with full_iteration builds the field and
+ * runs 5..16 as 1..4; tile = most voxels of a work item (>= 128, 0 =
+ * unchanged; launches that would have few items halve it, down to 32); order =
+ * voxel order of the packed list: 0 the caller's, 1 Morton (Z-order) of (z, y,
+ * x), 2..7 blocked (Morton order of
  * blocks of 1x2x16, 1x4x8, 2x4x32, 4x8x64, 4x16x32 or 8x16x128 voxels, row
  * order inside a block), -1 unchanged. */
 int anacor_plan_configure(anacor_plan *p, int variant, int tile, int order);
