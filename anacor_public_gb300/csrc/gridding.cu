@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kInterpBlock) gridding_interp_kernel(const T *
 // (about 46 bits, so the FP32 argument of expf is the FP64 evaluation's but
 // for near ties): in FP64 the 16 multiply-adds per voxel bound the kernel, at
 // 1.04 ms for 20,000 reflections of 960 voxels; now 614 MB of map rows take
-// 0.15 ms in one launch.  One warp per reflection when there are enough of
+// 0.14 ms in one launch.  One warp per reflection when there are enough of
 // them to fill the device (no block barrier), else a whole block.
 template <int kGroup>
 __global__ void __launch_bounds__(kInterpBlock) gridding_bilinear_kernel(const float *__restrict__ map, long long sR,
@@ -244,8 +244,8 @@ cudaError_t launch_interp(const T *map, long long sK, long long sR, int n_vox, c
     if constexpr (sizeof(T) == 4) {
         if (linear && sK == 1 && sR % 4 == 0 && ((uintptr_t)map & 15) == 0) {
             // Warps of a device at eight blocks an SM: one reflection each once
-            // there are that many (9,728 of 960 voxels: 81 us, a block each 116;
-            // of 1,658: 120 and 168).  Prepared and asynchronous lookups launch
+            // there are that many (9,728 of 960 voxels: 76 us, a block each 100;
+            // of 1,658: 113 and 144).  Prepared and asynchronous lookups launch
             // all their rows at once; a synchronous call launches 2,048 at a time,
             // blocks, which its host lookups hide.
             if (n_refl >= (long long)sms * 64)
