@@ -2031,7 +2031,10 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
 {
     __shared__ WarpTab tabs[kWarps];
     __shared__ FloatPair consts[kWarps][7];   // squared voxel edges (z, y, x), mu
-    __shared__ FloatSum sums[kBlock];         // the lanes' sums: in registers they spill what a search needs
+    // third floats of the lanes' sums: a third register spills what a search
+    // needs (701 reflections of 6,800 voxels: 1.0 % slower), all three here are
+    // 2 KB more a block out of L1 (0.6 %)
+    __shared__ float low[kBlock];
     if (!block_shape_ok(n_desc > 0 ? descs[0].status : nullptr))
         return;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -2056,7 +2059,8 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
         else if (lane < 7)
             K[lane] = pair_of(D.mu[lane - 3]);
         __syncwarp();
-        sums[tid] = {0.0f, 0.0f, 0.0f};
+        float s = 0.0f, c = 0.0f;
+        low[tid] = 0.0f;
         const int n = min(D.tile, D.n_vox - t * D.tile);
         const short4 *coords = D.coords + (long long)t * D.tile;
         for (int vi = lane; vi < n; vi += 32) {
@@ -2125,10 +2129,14 @@ __global__ void __launch_bounds__(kBlock, 4) bisection_fixed_kernel(const Sample
 #pragma unroll
             for (int m = 0; m < 4; m++)
                 ex = pair_add(ex, pair_mul(pair_add(L[0][m], L[1][m]), K[3 + m]));
-            sum_add(sums[tid], exp_neg(ex));
+            FloatSum sum = {s, c, low[tid]};
+            sum_add(sum, exp_neg(ex));
+            s = sum.s;
+            c = sum.c;
+            low[tid] = sum.d;
         }
         __syncwarp();
-        finish_warp_item(sums[tid], D, refl, t, lane);
+        finish_warp_item({s, c, low[tid]}, D, refl, t, lane);
     }
 }
 
