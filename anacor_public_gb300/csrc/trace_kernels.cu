@@ -1412,7 +1412,7 @@ __device__ __forceinline__ int find_sample(const SampleDesc *d, int n, long long
 // without room for the third floats folds them in.)
 __device__ __forceinline__ void finish_warp_item(FloatSum a, const SampleDesc &D, long long r, int t, int lane)
 {
-#pragma unroll
+#pragma unroll 1   // inlined everywhere: unrolled, it costs the bisection 0.8 % in instruction fetches
     for (int o = 16; o > 0; o >>= 1)
         sum_merge(a, __shfl_down_sync(kAll, a.s, o), __shfl_down_sync(kAll, a.c, o), __shfl_down_sync(kAll, a.d, o));
     int last = 0;
@@ -1431,11 +1431,24 @@ __device__ __forceinline__ void finish_warp_item(FloatSum a, const SampleDesc &D
         const float2 *sc = D.partial + r * D.tiles;
         const float *low = D.partial_low ? D.partial_low + r * D.tiles : nullptr;
         a = {0.0f, 0.0f, 0.0f};
-        for (int k = lane; k < D.tiles; k += 32) {
-            const float2 p = __ldcg(sc + k);
-            sum_merge(a, p.x, p.y, low ? __ldcg(low + k) : 0.0f);
-        }
+        // eight entries' loads together: a few reflections of many items wait for
+        // this loop (6 of 64,000 voxels: 53 us a launch, 69 one after the other)
+        constexpr int kAhead = 8;
+        for (int k0 = lane; k0 < D.tiles; k0 += 32 * kAhead) {
+            float2 p[kAhead];
+            float d[kAhead];
 #pragma unroll
+            for (int j = 0; j < kAhead; j++) {
+                const int k = k0 + 32 * j;
+                const bool in = k < D.tiles;
+                p[j] = in ? __ldcg(sc + k) : make_float2(0.0f, 0.0f);
+                d[j] = in && low ? __ldcg(low + k) : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < kAhead; j++)
+                sum_merge(a, p[j].x, p[j].y, d[j]);
+        }
+#pragma unroll 1
         for (int o = 16; o > 0; o >>= 1)
             sum_merge(a, __shfl_down_sync(kAll, a.s, o), __shfl_down_sync(kAll, a.c, o), __shfl_down_sync(kAll, a.d, o));
         if (lane == 0) {
