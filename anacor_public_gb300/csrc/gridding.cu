@@ -12,7 +12,7 @@
 // load.  For nearest lookups exp runs in FP32 on the FP32 sum of the two map
 // values (within 1e-7 relative of the reference's FP64 sum and exp); bilinear
 // lookups carry the FP64 weights and the range reduction on pairs of floats.  The mean is a
-// compensated FP32 sum, as in the absorption kernel.
+// compensated FP32 sum.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -438,7 +438,8 @@ int run_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int i
 // locked) and d_sample are this launch's until the stream has passed it.
 // Items of 256 voxels: a direction is a few of them, thousands of directions
 // fill the device, and a slow item's tail is short (64,800 directions x 1,657
-// voxels, whole call: 5.16 ms, of 128 5.17, of 512 5.52, of 1,024 6.3).
+// voxels, whole call: 5.16 ms, of 128 5.17, of 512 5.52, of 1,024 6.3; between
+// boxes 5.2 to 5.4).
 cudaError_t enqueue_field_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int is_exp, float *out,
                               long long ld, SampleDesc *h_sample, SampleDesc *d_sample, unsigned long long *d_counter,
                               int *d_status, int grid, cudaStream_t st)

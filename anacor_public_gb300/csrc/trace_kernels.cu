@@ -33,10 +33,9 @@
 //              fl(span / (len-1)) from a table of correctly rounded quotients,
 //              or a correctly rounded reciprocal and one FMA correction.  A
 //              leg that stopped at vacuum takes its last point from the march.
-//   rate       (cal_rate, :1554-1583): FP32 exponent and exp; per-thread
-//              Neumaier sums, warp-shuffle TwoSum reduction, tile partials
-//              combined in FP64 in a fixed order (deterministic for any
-//              schedule).
+//   rate       (cal_rate, :1554-1583): FP32 exponent and exp; sums of three
+//              floats (FloatSum) a lane, warp, tile and reflection, rounded
+//              once (the same bits for any schedule and cut into tiles).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -908,7 +907,8 @@ __device__ __forceinline__ void trace_leg(const LegHead &h, const FaceRule *rule
 // 512x512x400, 13,266 voxels, 20,000 reflections: 30.0 -> 18.6 ms (1,430 ->
 // 852 warp instructions per 32 legs; L1 misses at 69 %, L2 at 60 % of their
 // peak rates, issue slots at 53 %).  1024x1024x800, every crystal voxel (6.8 million),
-// 32 reflections: 22.9 -> 16.9 ms (18.6 with those 10.2 local loads).
+// 32 reflections: 23.0 -> 17.7 ms on one box, 24.3 -> 19.9 on another (10 %
+// more with those 10.2 local loads).
 
 // One leg's rule for one exit axis.  q: the 32.32 ratios of the two other
 // axes a and b (lo, hi words).  off: their initial low words -- the rounding

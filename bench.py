@@ -479,7 +479,7 @@ def run_ours(args):
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": args.scaling,
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "arith": "u8 labels, int32/32.32 fixed-point march (FP64 where a step is near a rounding boundary), "
-                     "FP32 lengths and exp, FP64 reflection set-up and partial sums",
+                     "FP32 lengths and exp, FP64 reflection set-up, three-float sums",
             "config": {"workload": WORKLOADS[args.workload], "n_samples": len(samples), "n_voxels": n_vox,
                        "n_reflections": sum(job_n), "reflections_per_rank": n_refl,
                        "sharding": ("shard.reflection_slice over the job's reflections, results gathered to "
