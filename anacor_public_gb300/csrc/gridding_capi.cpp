@@ -759,25 +759,29 @@ int anacor_gridding_interpolate(anacor_gridding *g, const double *s1, const doub
     }
     cudaStream_t st = g->pv.stream;
     cudaError_t e;
-    InterpRow *d_rows = nullptr;   // this call's; the results follow
-    if ((e = cudaEventSynchronize(g->landed[0])) || (e = cudaEventSynchronize(g->landed[1])) ||
-        (e = lib_malloc_async(reinterpret_cast<void **>(&d_rows), (size_t)n * (sizeof(InterpRow) + sizeof(double)), st)))
-        return cuda_err(e);
-    double *d_out = reinterpret_cast<double *>(d_rows + n);
-    e = stage_begin(g, st);
     // the host's lookups of one chunk beside the copy and the kernel of the
     // last (20,000 reflections bilinear, 1,658 voxels: 340 us of lookups, 37
     // of copy, 139 of kernel and 40 for a fresh array were 560 us in a row;
-    // a call is 360 us so)
+    // a call is 360 us so).  One chunk alone needs no second stream, whose
+    // events cost it 8 us (100 nearest lookups of 40 voxels: 66 us, 52 so).
+    constexpr int64_t kChunk = 2048;
+    const bool beside = n > kChunk;
+    InterpRow *d_rows = nullptr;   // this call's; the results follow
+    if ((beside && ((e = cudaEventSynchronize(g->landed[0])) || (e = cudaEventSynchronize(g->landed[1])))) ||
+        (e = lib_malloc_async(reinterpret_cast<void **>(&d_rows), (size_t)n * (sizeof(InterpRow) + sizeof(double)), st)))
+        return cuda_err(e);
+    double *d_out = reinterpret_cast<double *>(d_rows + n);
+    double *got = beside ? out : reinterpret_cast<double *>(g->h_stage + kStageBytes);
+    e = beside ? stage_begin(g, st) : cudaSuccess;
     std::atomic<bool> ok{true};
     for (int64_t c = 0, k = 0; c < n && !e && ok; c += kStageRows, k++) {
         const int64_t m = std::min<int64_t>(kStageRows, n - c);
         const int b = (int)(k & 1);
-        if ((e = cudaEventSynchronize(g->landed[b])))
+        if (beside && (e = cudaEventSynchronize(g->landed[b])))
             break;
         InterpRow *rows = reinterpret_cast<InterpRow *>(g->h_stage + b * kStageBytes);
         produce(
-            m, 2048,
+            m, kChunk,
             [&](int64_t i0, int64_t i1) {
                 if (!interp_row_block(g, s1, omega, c + i0, c + i1, xray, omega_axis, F, method == 2, rows + i0))
                     ok = false;
@@ -785,16 +789,18 @@ int anacor_gridding_interpolate(anacor_gridding *g, const double *s1, const doub
             [&](int64_t i0, int64_t i1) {
                 if (e || !ok)
                     return;
-                if (!(e = stage_upload(g, b, (size_t)i0 * sizeof(InterpRow), d_rows + c + i0,
-                                       (size_t)(i1 - i0) * sizeof(InterpRow), true, st)))
+                const size_t bytes = (size_t)(i1 - i0) * sizeof(InterpRow);
+                e = beside ? stage_upload(g, b, (size_t)i0 * sizeof(InterpRow), d_rows + c + i0, bytes, true, st)
+                           : cudaMemcpyAsync(d_rows, rows, bytes, cudaMemcpyHostToDevice, st);
+                if (!e)
                     e = launch_gridding_interp_f32(g->d_map, 1, g->ld, g->pv.n_vox, d_rows + c + i0, i1 - i0,
                                                    method == 2, d_out + c + i0, st);
             });
     }
     const int bad = ok ? kOk : rows_refused();
     if (!e && !bad)
-        e = cudaMemcpyAsync(out, d_out, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
-    else
+        e = cudaMemcpyAsync(got, d_out, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
+    else if (beside)
         cudaStreamSynchronize(g->copy);   // nothing may still be writing the rows
     cudaFreeAsync(d_rows, st);
     const cudaError_t e2 = cudaStreamSynchronize(st);
@@ -802,6 +808,8 @@ int anacor_gridding_interpolate(anacor_gridding *g, const double *s1, const doub
         return bad;   // reported
     if (e || e2)
         return cuda_err(e ? e : e2);
+    if (!beside)
+        std::memcpy(out, got, (size_t)n * sizeof(double));
     return report_status(kOk, "");
 }
 
