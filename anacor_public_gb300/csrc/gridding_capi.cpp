@@ -439,7 +439,11 @@ int run_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int i
 // Items of 256 voxels: a direction is a few of them, thousands of directions
 // fill the device, and a slow item's tail is short (64,800 directions x 1,657
 // voxels, whole call: 5.16 ms, of 128 5.17, of 512 5.52, of 1,024 6.3; between
-// boxes 5.2 to 5.4).
+// boxes 5.2 to 5.4).  Fewer directions or voxels: halved, down to one voxel a
+// lane, until there are sixteen items for each of the forty warps an SM runs:
+// legs that touch walls or change class often take many times the others'.
+// 342 directions x 1,500 voxels of a 60^3 volume 218 -> 89 us, 4,277 of a
+// 9x164x13 one of stripes 5.99 -> 2.70 ms (four items a warp: 4.78).
 cudaError_t enqueue_field_map(const PlanView &pv, const ReflTable *d_dirs, long long n_dirs, int is_exp, float *out,
                               long long ld, SampleDesc *h_sample, SampleDesc *d_sample, unsigned long long *d_counter,
                               int *d_status, int grid, cudaStream_t st)
@@ -461,6 +465,8 @@ cudaError_t enqueue_field_map(const PlanView &pv, const ReflTable *d_dirs, long 
     d.refl = d_dirs;
     d.n_refl = n_dirs;
     d.tile = 256;
+    while (d.tile > 32 && n_dirs * ((pv.n_vox + d.tile - 1) / d.tile) < (long long)pv.sms * 40 * 16)
+        d.tile /= 2;
     d.tiles = (pv.n_vox + d.tile - 1) / d.tile;
     d.full_iteration = pv.full_iteration;
     d.is_exp = is_exp;
