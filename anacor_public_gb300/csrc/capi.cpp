@@ -126,7 +126,7 @@ int current_device(DeviceState **out)
             return fail(kErrCuda, "reciprocal table upload failed");
         // Shared memory's share of the unified storage, the rest L1 for the label
         // gathers.  Cooperative march: 40 %, room for 4 CTAs' 19 KB (30 .. 50 %
-        // are within 1 %).  Field march: 50 %, room for 5 CTAs' 20 KB; at 40 %
+        // are within 1 %).  Field march: 50 %, room for 5 CTAs' 21 KB; at 40 %
         // only 4 fit (512x512x400, 4,000 reflections: 4.09 ms at 40 %, 3.80 at
         // 45 .. 55, 3.89 at 60, 4.11 at 75).  ANACOR_SMEM_CARVEOUT overrides both.
         const char *cv = std::getenv("ANACOR_SMEM_CARVEOUT");
